@@ -89,6 +89,24 @@ def load():
     return lib
 
 
+_native = None
+
+
+def native():
+    """The CPython extension that is the library's host path (csrc/torch_host.cpp), loaded once; raises
+    if it or the library is missing."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise RuntimeError(f"naju_b200/_native.so is missing or does not load ({e}): build it with "
+                               "`python -m naju_b200.build` (there is no CPU or PyTorch fallback for the scan)") from e
+        _native = mod
+    return _native
+
+
 def strerror(code):
     return load().naju_b200_strerror(int(code)).decode()
 

@@ -83,6 +83,29 @@ __device__ __forceinline__ int wait_flag(const int* flag) {
   return v;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// A kernel started with launch_pdl() may begin while the kernel before it in the stream is still
+// running: pdl_wait() returns once that one has completed and its writes are visible, and nothing that
+// touches global memory may come before it.  pdl_launch_dependents() lets the next such kernel's
+// blocks start as soon as every block of this one has called it (or ended).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // ---------------------------------------------------------------- async tile movement
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));

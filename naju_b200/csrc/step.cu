@@ -3,90 +3,170 @@
 //
 //   state[b,d,n] <- f state[b,d,n] + (i u) B[b,n];   y[b,d] = sum_n C[b,n] state[b,d,n] + D_skip u
 //
-// Pure HBM streaming of the fp32 state (read once, written once).  Each thread owns four
-// consecutive states (one 16-byte load/store); the N/4 lanes that share a channel are
-// adjacent, so a warp touches one contiguous 512-byte span per access and the readout is a
-// short shuffle reduction.
+// HBM streaming of the fp32 state (read once, written once): 8 N bytes per channel against 8 to 16 of
+// everything else.  A thread owns four consecutive states of kIter channels, so all of its state loads
+// (16 bytes each) are in flight at once and the row's B and C are read once for all of them, as one
+// vector each; the N/4 lanes that share a channel are adjacent, so a warp touches contiguous
+// 512-byte spans and the readout is a short shuffle reduction.  Decode calls follow one another layer by
+// layer, each too short to hide a launch: the kernel lets its successor's blocks launch early and waits
+// for its predecessor itself (programmatic dependent launch).
 #include "common.cuh"
 #include "params.h"
 
 namespace naju {
 
-constexpr int kStepBlock = 128;  // (measured: 128 threads 20.2 us per launch, 256: 20.8, 512: 22.2)
+constexpr int kStepBlock = 128;
 
-template <typename TA, typename TG>
+// four consecutive elements of a row of B or C as floats (`vec`: one 8- or 16-byte load)
+template <typename TB>
+__device__ __forceinline__ void load_row4(const TB* __restrict__ p, int n0, int N, bool vec, float (&v)[4]) {
+  if (vec) {
+    if constexpr (sizeof(TB) == 4) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(p + n0));
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+      const uint2 t = __ldg(reinterpret_cast<const uint2*>(p + n0));
+      TB e[4];
+      *reinterpret_cast<uint2*>(e) = t;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = to_f32(e[k]);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = n0 + k < N ? to_f32(p[n0 + k]) : 0.f;
+  }
+}
+
+// Block = kStepBlock threads of one batch row (blockIdx.y); lpc lanes per channel (a power of two, at
+// least N/4); kIter channels per thread, kStepBlock / lpc apart.
+template <typename TA, typename TG, typename TB, int kIter>
 __global__ void __launch_bounds__(kStepBlock) step_kernel(float* __restrict__ state, const TA* __restrict__ u,
                                                    const TG* __restrict__ fl, const TG* __restrict__ il,
-                                                   const void* __restrict__ Bm, const void* __restrict__ Cm,
-                                                   const float* __restrict__ Dskip, TA* __restrict__ y,
-                                                   int B, int D, int N, int lpc /* lanes per channel, pow2 */,
-                                                   int bc_dtype, int64_t u_sb, int64_t fl_sb, int64_t il_sb,
+                                                   const TB* __restrict__ Bm, const TB* __restrict__ Cm,
+                                                   const float* __restrict__ Dskip, TA* __restrict__ y, int D, int N,
+                                                   int lpc_log2, bool vec, int64_t u_sb, int64_t fl_sb, int64_t il_sb,
                                                    int64_t bm_sb, int64_t cm_sb) {
-  const int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t chan = gid / lpc;           // flat (b, d)
-  const int q = static_cast<int>(gid % lpc);  // which group of four states
-  const bool ok = chan < static_cast<int64_t>(B) * D;
-  float part = 0.f;
-  float ut = 0.f;
-  int b = 0, d = 0;
-  if (ok) {
-    b = static_cast<int>(chan / D);
-    d = static_cast<int>(chan % D);
-    ut = to_f32(u[b * u_sb + d]);
-    const float f = sigmoid_f(to_f32(fl[b * fl_sb + d]));
-    const float w = sigmoid_f(to_f32(il[b * il_sb + d])) * ut;
-    const int n0 = 4 * q;
-    float* sp = state + chan * N + n0;
-    if (n0 + 4 <= N && (N & 3) == 0) {
-      // the state is touched once per token: streaming (evict-first) accesses keep it from pushing
-      // the token's small inputs out of L2
-      float4 s = __ldcs(reinterpret_cast<const float4*>(sp));
-      s.x = fmaf(f, s.x, w * load_dyn(Bm, bc_dtype, b * bm_sb + n0 + 0));
-      s.y = fmaf(f, s.y, w * load_dyn(Bm, bc_dtype, b * bm_sb + n0 + 1));
-      s.z = fmaf(f, s.z, w * load_dyn(Bm, bc_dtype, b * bm_sb + n0 + 2));
-      s.w = fmaf(f, s.w, w * load_dyn(Bm, bc_dtype, b * bm_sb + n0 + 3));
-      __stcs(reinterpret_cast<float4*>(sp), s);
-      part = s.x * load_dyn(Cm, bc_dtype, b * cm_sb + n0 + 0);
-      part = fmaf(s.y, load_dyn(Cm, bc_dtype, b * cm_sb + n0 + 1), part);
-      part = fmaf(s.z, load_dyn(Cm, bc_dtype, b * cm_sb + n0 + 2), part);
-      part = fmaf(s.w, load_dyn(Cm, bc_dtype, b * cm_sb + n0 + 3), part);
-    } else {
-      for (int n = n0; n < min(n0 + 4, N); ++n) {
-        const float s = fmaf(f, sp[n - n0], w * load_dyn(Bm, bc_dtype, b * bm_sb + n));
-        sp[n - n0] = s;
-        part = fmaf(s, load_dyn(Cm, bc_dtype, b * cm_sb + n), part);
+  pdl_launch_dependents();
+  const int b = blockIdx.y, q = threadIdx.x & ((1 << lpc_log2) - 1), n0 = 4 * q;
+  const int per_pass = kStepBlock >> lpc_log2;
+  const int d0 = blockIdx.x * per_pass * kIter + (static_cast<int>(threadIdx.x) >> lpc_log2);
+  const bool whole = (N & 3) == 0;   // states of a channel come in 16-byte pieces
+  const bool mine = n0 < N;
+  pdl_wait();
+  float4 s[kIter];
+  float ut[kIter], xf[kIter], xi[kIter];
+#pragma unroll
+  for (int k = 0; k < kIter; ++k) {
+    const int d = d0 + k * per_pass;
+    s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ut[k] = xf[k] = xi[k] = 0.f;
+    if (d < D) {
+      const float* sp = state + (static_cast<int64_t>(b) * D + d) * N + n0;
+      if (whole) {
+        // the state is touched once per token: streaming (evict-first) accesses keep it from pushing
+        // the token's small inputs out of L2
+        if (mine) s[k] = __ldcs(reinterpret_cast<const float4*>(sp));
+      } else {
+        if (n0 + 0 < N) s[k].x = sp[0];
+        if (n0 + 1 < N) s[k].y = sp[1];
+        if (n0 + 2 < N) s[k].z = sp[2];
+        if (n0 + 3 < N) s[k].w = sp[3];
       }
+      ut[k] = to_f32(u[b * u_sb + d]);
+      xf[k] = to_f32(fl[b * fl_sb + d]);
+      xi[k] = to_f32(il[b * il_sb + d]);
     }
   }
-  // lanes sharing a channel are adjacent and lpc divides 32
-  for (int m = lpc >> 1; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
-  if (ok && q == 0) y[static_cast<int64_t>(b) * D + d] = from_f32<TA>(fmaf(Dskip[d], ut, part));
+  float bv[4] = {0.f, 0.f, 0.f, 0.f}, cv[4] = {0.f, 0.f, 0.f, 0.f};
+  if (mine) {
+    load_row4(Bm + b * bm_sb, n0, N, vec, bv);
+    load_row4(Cm + b * cm_sb, n0, N, vec, cv);
+  }
+#pragma unroll
+  for (int k = 0; k < kIter; ++k) {
+    const int d = d0 + k * per_pass;
+    const float f = sigmoid_f(xf[k]);
+    const float w = sigmoid_f(xi[k]) * ut[k];
+    s[k].x = fmaf(f, s[k].x, w * bv[0]);
+    s[k].y = fmaf(f, s[k].y, w * bv[1]);
+    s[k].z = fmaf(f, s[k].z, w * bv[2]);
+    s[k].w = fmaf(f, s[k].w, w * bv[3]);
+    float part = s[k].x * cv[0];
+    part = fmaf(s[k].y, cv[1], part);
+    part = fmaf(s[k].z, cv[2], part);
+    part = fmaf(s[k].w, cv[3], part);
+    if (d < D) {
+      float* sp = state + (static_cast<int64_t>(b) * D + d) * N + n0;
+      if (whole) {
+        if (mine) __stcs(reinterpret_cast<float4*>(sp), s[k]);
+      } else {
+        if (n0 + 0 < N) sp[0] = s[k].x;
+        if (n0 + 1 < N) sp[1] = s[k].y;
+        if (n0 + 2 < N) sp[2] = s[k].z;
+        if (n0 + 3 < N) sp[3] = s[k].w;
+      }
+    }
+    // lanes sharing a channel are adjacent and their number divides 32
+    for (int m = (1 << lpc_log2) >> 1; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
+    if (d < D && q == 0) y[static_cast<int64_t>(b) * D + d] = from_f32<TA>(fmaf(Dskip[d], ut[k], part));
+  }
+}
+
+template <typename TA, typename TG, typename TB, int kIter>
+static int launch_iter(const naju_scan_desc& d, float* state, const void* u, const void* fl, const void* il, const void* Bm,
+                       const void* Cm, const float* Dskip, void* y, int lpc_log2, cudaStream_t st) {
+  const int span = (kStepBlock >> lpc_log2) * kIter;
+  auto aligned4 = [](const void* p, int64_t sb) {
+    return reinterpret_cast<uintptr_t>(p) % (4 * sizeof(TB)) == 0 && sb % 4 == 0;
+  };
+  const bool vec = d.N % 4 == 0 && aligned4(Bm, d.bm_sb) && aligned4(Cm, d.cm_sb);
+  for (int b0 = 0; b0 < d.B; b0 += 65535) {   // (grid.y limit)
+    const int nb = d.B - b0 < 65535 ? d.B - b0 : 65535;
+    const dim3 grid(static_cast<unsigned>((d.D + span - 1) / span), static_cast<unsigned>(nb));
+    const int rc = launch_pdl(step_kernel<TA, TG, TB, kIter>, grid, dim3(kStepBlock), 0, st,
+                              state + static_cast<int64_t>(b0) * d.D * d.N, static_cast<const TA*>(u) + b0 * d.u_sb,
+                              static_cast<const TG*>(fl) + b0 * d.fl_sb, static_cast<const TG*>(il) + b0 * d.il_sb,
+                              static_cast<const TB*>(Bm) + b0 * d.bm_sb, static_cast<const TB*>(Cm) + b0 * d.cm_sb, Dskip,
+                              static_cast<TA*>(y) + static_cast<int64_t>(b0) * d.D, d.D, d.N, lpc_log2, vec, d.u_sb, d.fl_sb,
+                              d.il_sb, d.bm_sb, d.cm_sb);
+    if (rc != 0) return rc;
+  }
+  return 0;
+}
+
+template <typename TA, typename TG, typename TB>
+static int launch_t(const naju_scan_desc& d, float* state, const void* u, const void* fl, const void* il, const void* Bm,
+                    const void* Cm, const float* Dskip, void* y, cudaStream_t st) {
+  int lpc_log2 = 0;
+  while ((4 << lpc_log2) < d.N) ++lpc_log2;  // 1..32 lanes
+#ifndef NAJU_STEP_ITER
+#define NAJU_STEP_ITER 4
+#endif
+  // One channel per thread until that gives the GPU two blocks per warp scheduler (148 SMs x 8): below it
+  // the call is bound by latency and more blocks are all there is; above it by memory bandwidth.
+  const int64_t blocks1 = static_cast<int64_t>(d.B) * ((static_cast<int64_t>(d.D) << lpc_log2) / kStepBlock);
+  if (blocks1 <= 148 * 8 * NAJU_STEP_ITER)
+    return launch_iter<TA, TG, TB, 1>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+  return launch_iter<TA, TG, TB, NAJU_STEP_ITER>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
 }
 
 template <typename TA, typename TG>
-static int launch_t(const naju_scan_desc& d, float* state, const void* u, const void* fl,
-                    const void* il, const void* Bm, const void* Cm, const float* Dskip, void* y,
-                    cudaStream_t st) {
-  int lpc = 1;
-  while (lpc * 4 < d.N) lpc <<= 1;  // 1..32
-  const int64_t threads = static_cast<int64_t>(d.B) * d.D * lpc;
-  const unsigned blocks = static_cast<unsigned>((threads + kStepBlock - 1) / kStepBlock);
-  step_kernel<TA, TG><<<blocks, kStepBlock, 0, st>>>(
-      state, static_cast<const TA*>(u), static_cast<const TG*>(fl), static_cast<const TG*>(il), Bm,
-      Cm, Dskip, static_cast<TA*>(y), d.B, d.D, d.N, lpc, d.bc_dtype, d.u_sb, d.fl_sb, d.il_sb,
-      d.bm_sb, d.cm_sb);
-  return static_cast<int>(cudaGetLastError());
+static int launch_bc(const naju_scan_desc& d, float* state, const void* u, const void* fl, const void* il, const void* Bm,
+                     const void* Cm, const float* Dskip, void* y, cudaStream_t st) {
+  if (d.bc_dtype == NAJU_F32) return launch_t<TA, TG, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (d.bc_dtype == NAJU_BF16) return launch_t<TA, TG, __nv_bfloat16>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  return launch_t<TA, TG, __half>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
 }
 
 int launch_step(const naju_scan_desc& d, float* state, const void* u, const void* fl, const void* il,
                 const void* Bm, const void* Cm, const float* Dskip, void* y, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int a = d.act_dtype, g = d.gate_dtype;
-  if (a == NAJU_F32 && g == NAJU_F32) return launch_t<float, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
-  if (a == NAJU_BF16 && g == NAJU_BF16) return launch_t<__nv_bfloat16, __nv_bfloat16>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
-  if (a == NAJU_BF16 && g == NAJU_F32) return launch_t<__nv_bfloat16, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
-  if (a == NAJU_F16 && g == NAJU_F16) return launch_t<__half, __half>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
-  if (a == NAJU_F16 && g == NAJU_F32) return launch_t<__half, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (a == NAJU_F32 && g == NAJU_F32) return launch_bc<float, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (a == NAJU_BF16 && g == NAJU_BF16) return launch_bc<__nv_bfloat16, __nv_bfloat16>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (a == NAJU_BF16 && g == NAJU_F32) return launch_bc<__nv_bfloat16, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (a == NAJU_F16 && g == NAJU_F16) return launch_bc<__half, __half>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
+  if (a == NAJU_F16 && g == NAJU_F32) return launch_bc<__half, float>(d, state, u, fl, il, Bm, Cm, Dskip, y, st);
   return NAJU_E_DTYPE;
 }
 
