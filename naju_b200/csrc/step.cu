@@ -38,50 +38,50 @@ __device__ __forceinline__ void load_row4(const TB* __restrict__ p, int n0, int 
 }
 
 // Block = kStepBlock threads of one batch row (blockIdx.y); lpc lanes per channel (a power of two, at
-// least N/4); kIter channels per thread, kStepBlock / lpc apart.
-template <typename TA, typename TG, typename TB, int kIter>
+// least N/4); kIter channels per thread, kStepBlock / lpc apart.  kWhole: a channel's states come in
+// 16-byte pieces (N % 4 == 0).  kN: N at compile time, or 0.  Lanes beyond the last channel or state read in-bounds duplicates and
+// write nothing, so that no load of the batch sits behind a branch (with branches around them the
+// loads were issued one iteration at a time: 18.9 us against 13 us at 256 sequences x 2048 channels).
+template <typename TA, typename TG, typename TB, int kIter, bool kWhole, int kN>
 __global__ void __launch_bounds__(kStepBlock) step_kernel(float* __restrict__ state, const TA* __restrict__ u,
                                                    const TG* __restrict__ fl, const TG* __restrict__ il,
                                                    const TB* __restrict__ Bm, const TB* __restrict__ Cm,
-                                                   const float* __restrict__ Dskip, TA* __restrict__ y, int D, int N,
-                                                   int lpc_log2, bool vec, int64_t u_sb, int64_t fl_sb, int64_t il_sb,
+                                                   const float* __restrict__ Dskip, TA* __restrict__ y, int D, int N_,
+                                                   int lpc_log2_, bool vec, int64_t u_sb, int64_t fl_sb, int64_t il_sb,
                                                    int64_t bm_sb, int64_t cm_sb) {
   pdl_launch_dependents();
-  const int b = blockIdx.y, q = threadIdx.x & ((1 << lpc_log2) - 1), n0 = 4 * q;
+  const int N = kN > 0 ? kN : N_;
+  const int lpc_log2 = kN == 0 ? lpc_log2_ : kN <= 4 ? 0 : kN <= 8 ? 1 : kN <= 16 ? 2 : kN <= 32 ? 3 : kN <= 64 ? 4 : 5;
+  const int b = blockIdx.y, q = threadIdx.x & ((1 << lpc_log2) - 1);
   const int per_pass = kStepBlock >> lpc_log2;
   const int d0 = blockIdx.x * per_pass * kIter + (static_cast<int>(threadIdx.x) >> lpc_log2);
-  const bool whole = (N & 3) == 0;   // states of a channel come in 16-byte pieces
-  const bool mine = n0 < N;
+  const bool mine = 4 * q < N;
+  const int n0 = mine ? 4 * q : 0;
+  float* srow = state + static_cast<int64_t>(b) * D * N + n0;
+  u += b * u_sb;
+  fl += b * fl_sb;
+  il += b * il_sb;
   pdl_wait();
   float4 s[kIter];
-  float ut[kIter], xf[kIter], xi[kIter];
+  float ut[kIter], xf[kIter], xi[kIter], bv[4], cv[4];
 #pragma unroll
   for (int k = 0; k < kIter; ++k) {
-    const int d = d0 + k * per_pass;
-    s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    ut[k] = xf[k] = xi[k] = 0.f;
-    if (d < D) {
-      const float* sp = state + (static_cast<int64_t>(b) * D + d) * N + n0;
-      if (whole) {
-        // the state is touched once per token: streaming (evict-first) accesses keep it from pushing
-        // the token's small inputs out of L2
-        if (mine) s[k] = __ldcs(reinterpret_cast<const float4*>(sp));
-      } else {
-        if (n0 + 0 < N) s[k].x = sp[0];
-        if (n0 + 1 < N) s[k].y = sp[1];
-        if (n0 + 2 < N) s[k].z = sp[2];
-        if (n0 + 3 < N) s[k].w = sp[3];
-      }
-      ut[k] = to_f32(u[b * u_sb + d]);
-      xf[k] = to_f32(fl[b * fl_sb + d]);
-      xi[k] = to_f32(il[b * il_sb + d]);
+    const int d = min(d0 + k * per_pass, D - 1);
+    const float* sp = srow + static_cast<int64_t>(d) * N;
+    if constexpr (kWhole) {
+      s[k] = *reinterpret_cast<const float4*>(sp);
+    } else {
+      s[k].x = sp[0];
+      s[k].y = sp[min(1, N - 1 - n0)];
+      s[k].z = sp[min(2, N - 1 - n0)];
+      s[k].w = sp[min(3, N - 1 - n0)];
     }
+    ut[k] = to_f32(u[d]);
+    xf[k] = to_f32(fl[d]);
+    xi[k] = to_f32(il[d]);
   }
-  float bv[4] = {0.f, 0.f, 0.f, 0.f}, cv[4] = {0.f, 0.f, 0.f, 0.f};
-  if (mine) {
-    load_row4(Bm + b * bm_sb, n0, N, vec, bv);
-    load_row4(Cm + b * cm_sb, n0, N, vec, cv);
-  }
+  load_row4(Bm + b * bm_sb, n0, N, vec, bv);
+  load_row4(Cm + b * cm_sb, n0, N, vec, cv);
 #pragma unroll
   for (int k = 0; k < kIter; ++k) {
     const int d = d0 + k * per_pass;
@@ -95,24 +95,26 @@ __global__ void __launch_bounds__(kStepBlock) step_kernel(float* __restrict__ st
     part = fmaf(s[k].y, cv[1], part);
     part = fmaf(s[k].z, cv[2], part);
     part = fmaf(s[k].w, cv[3], part);
-    if (d < D) {
-      float* sp = state + (static_cast<int64_t>(b) * D + d) * N + n0;
-      if (whole) {
-        if (mine) __stcs(reinterpret_cast<float4*>(sp), s[k]);
+    if (!mine) part = 0.f;
+    if (d < D && mine) {
+      float* sp = srow + static_cast<int64_t>(d) * N;
+      if constexpr (kWhole) {
+        *reinterpret_cast<float4*>(sp) = s[k];
       } else {
-        if (n0 + 0 < N) sp[0] = s[k].x;
+        sp[0] = s[k].x;
         if (n0 + 1 < N) sp[1] = s[k].y;
         if (n0 + 2 < N) sp[2] = s[k].z;
         if (n0 + 3 < N) sp[3] = s[k].w;
       }
     }
     // lanes sharing a channel are adjacent and their number divides 32
+#pragma unroll
     for (int m = (1 << lpc_log2) >> 1; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
     if (d < D && q == 0) y[static_cast<int64_t>(b) * D + d] = from_f32<TA>(fmaf(Dskip[d], ut[k], part));
   }
 }
 
-template <typename TA, typename TG, typename TB, int kIter>
+template <typename TA, typename TG, typename TB, int kIter, bool kWhole, int kN>
 static int launch_iter(const naju_scan_desc& d, float* state, const void* u, const void* fl, const void* il, const void* Bm,
                        const void* Cm, const float* Dskip, void* y, int lpc_log2, cudaStream_t st) {
   const int span = (kStepBlock >> lpc_log2) * kIter;
@@ -123,7 +125,7 @@ static int launch_iter(const naju_scan_desc& d, float* state, const void* u, con
   for (int b0 = 0; b0 < d.B; b0 += 65535) {   // (grid.y limit)
     const int nb = d.B - b0 < 65535 ? d.B - b0 : 65535;
     const dim3 grid(static_cast<unsigned>((d.D + span - 1) / span), static_cast<unsigned>(nb));
-    const int rc = launch_pdl(step_kernel<TA, TG, TB, kIter>, grid, dim3(kStepBlock), 0, st,
+    const int rc = launch_pdl(step_kernel<TA, TG, TB, kIter, kWhole, kN>, grid, dim3(kStepBlock), 0, st,
                               state + static_cast<int64_t>(b0) * d.D * d.N, static_cast<const TA*>(u) + b0 * d.u_sb,
                               static_cast<const TG*>(fl) + b0 * d.fl_sb, static_cast<const TG*>(il) + b0 * d.il_sb,
                               static_cast<const TB*>(Bm) + b0 * d.bm_sb, static_cast<const TB*>(Cm) + b0 * d.cm_sb, Dskip,
@@ -139,15 +141,23 @@ static int launch_t(const naju_scan_desc& d, float* state, const void* u, const 
                     const void* Cm, const float* Dskip, void* y, cudaStream_t st) {
   int lpc_log2 = 0;
   while ((4 << lpc_log2) < d.N) ++lpc_log2;  // 1..32 lanes
-#ifndef NAJU_STEP_ITER
-#define NAJU_STEP_ITER 4
-#endif
-  // One channel per thread until that gives the GPU two blocks per warp scheduler (148 SMs x 8): below it
-  // the call is bound by latency and more blocks are all there is; above it by memory bandwidth.
+  // Two channels per thread once the grid stays at several blocks per SM with them: below that the call is
+  // bound by latency and more blocks are all there is.  (256 sequences x 2048 channels x 16 states: one
+  // channel per thread 14.9 us, two 13.2, four 13.7, eight 14.7; reading and writing the state in place
+  // and nothing else takes 14.4.)
   const int64_t blocks1 = static_cast<int64_t>(d.B) * ((static_cast<int64_t>(d.D) << lpc_log2) / kStepBlock);
-  if (blocks1 <= 148 * 8 * NAJU_STEP_ITER)
-    return launch_iter<TA, TG, TB, 1>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
-  return launch_iter<TA, TG, TB, NAJU_STEP_ITER>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+  // The usual widths have N, and with it every address and the readout's shuffles, at compile time
+  // (16.7 us with run-time ones at that size).
+  if (d.N % 4 != 0) return launch_iter<TA, TG, TB, 1, false, 0>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+  if (blocks1 <= 148 * 16) return launch_iter<TA, TG, TB, 1, true, 0>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+  switch (d.N) {
+    case 8: return launch_iter<TA, TG, TB, 2, true, 8>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+    case 16: return launch_iter<TA, TG, TB, 2, true, 16>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+    case 32: return launch_iter<TA, TG, TB, 2, true, 32>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+    case 64: return launch_iter<TA, TG, TB, 2, true, 64>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+    case 128: return launch_iter<TA, TG, TB, 2, true, 128>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+    default: return launch_iter<TA, TG, TB, 2, true, 0>(d, state, u, fl, il, Bm, Cm, Dskip, y, lpc_log2, st);
+  }
 }
 
 template <typename TA, typename TG>
