@@ -2,14 +2,13 @@
 // kernel dispatch.  No allocation, no host synchronisation except naju_b200_read_status().
 #include <cuda_runtime.h>
 
+#include "common.cuh"
 #include "naju_b200.h"
 #include "params.h"
 
 using namespace naju;
 
 namespace {
-
-size_t dtype_size(int dt) { return dt == NAJU_F32 ? 4 : 2; }
 
 bool dtype_ok(int dt) { return dt == NAJU_F32 || dt == NAJU_BF16 || dt == NAJU_F16; }
 
@@ -54,53 +53,6 @@ __global__ void copy_state_kernel(const float* __restrict__ src, float* __restri
   if (i < n) dst[i] = src ? src[i] : fill;
 }
 
-// Makes a device-side failure loud without a host round trip.  Runs after the kernels of a call,
-// on the same stream: when the call's status word is non-zero (a bounded wait ran out), or the
-// forward that wrote these checkpoints failed that way, every output of the call is overwritten
-// with all-ones bytes (NaN in fp32, bf16 and fp16 alike).  In the normal case it reads two words
-// and returns.
-struct PoisonList {
-  void* ptr[8];
-  unsigned long long bytes[8];
-  int n;
-};
-
-__global__ void poison_on_failure_kernel(ScratchHeader* hdr, int* fwd_form, int mark_trailer, int inject,
-                                         PoisonList list) {
-  __shared__ int s_bad;
-  if (threadIdx.x == 0) {
-    if (inject && blockIdx.x == 0) atomicOr(&hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
-    int st = *reinterpret_cast<volatile int*>(&hdr->status);
-    if (inject) st |= NAJU_ST_LOOKBACK_TIMEOUT;
-    const int failed_before = (!mark_trailer && fwd_form != nullptr) ? (*fwd_form & 4) : 0;
-    s_bad = (st != 0 || failed_before != 0) ? 1 : 0;
-    if (s_bad && mark_trailer && fwd_form != nullptr && blockIdx.x == 0) atomicOr(fwd_form, 4);
-  }
-  __syncthreads();
-  if (!s_bad) return;
-  for (int k = 0; k < list.n; ++k) {
-    unsigned char* p = static_cast<unsigned char*>(list.ptr[k]);
-    const unsigned long long nb = list.bytes[k];
-    for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nb;
-         i += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
-      p[i] = 0xFF;
-  }
-}
-
-void poison_add(PoisonList& l, void* p, size_t bytes) {
-  if (p != nullptr && bytes > 0 && l.n < 8) {
-    l.ptr[l.n] = p;
-    l.bytes[l.n] = bytes;
-    ++l.n;
-  }
-}
-
-int launch_poison(ScratchHeader* hdr, int* fwd_form, bool mark_trailer, bool inject, const PoisonList& l,
-                  cudaStream_t st) {
-  poison_on_failure_kernel<<<64, 256, 0, st>>>(hdr, fwd_form, mark_trailer ? 1 : 0, inject ? 1 : 0, l);
-  return static_cast<int>(cudaGetLastError());
-}
-
 int read_header_word(const void* scratch, size_t offset, void* stream) {
   if (!scratch) return NAJU_E_NULL;
   int word = 0;
@@ -112,7 +64,23 @@ int read_header_word(const void* scratch, size_t offset, void* stream) {
   return word;
 }
 
+// (16-byte stores: the scratch is 256-byte aligned and `words` counts 256-byte rounded regions)
+__global__ void init_kernel(uint4* __restrict__ scratch, int64_t n16, int* __restrict__ trailer) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x, i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int64_t i = i0; i < n16; i += step) scratch[i] = make_uint4(0, 0, 0, 0);
+  if (trailer != nullptr && i0 < 64) trailer[i0] = 0;
+}
+
 }  // namespace
+
+int naju::launch_init(ScratchHeader* hdr, size_t bytes, int* trailer, cudaStream_t stream) {
+  const int64_t n16 = static_cast<int64_t>((bytes + 15) / 16);
+  const int64_t blocks = (n16 + 255) / 256;
+  return launch_pdl(init_kernel, dim3(static_cast<unsigned>(blocks < 148 ? blocks : 148)), dim3(256), 0, stream,
+                    reinterpret_cast<uint4*>(hdr), n16, trailer);
+}
 
 extern "C" {
 
@@ -139,7 +107,7 @@ const char* naju_b200_strerror(int code) {
 
 int naju_b200_chunk_len(const naju_scan_desc* desc) {
   if (check_desc(desc, false) != NAJU_OK) return 0;
-  return chunk_len_for(padded_states(desc->N));
+  return chunk_len_for(*desc);
 }
 
 size_t naju_b200_ckpt_bytes(const naju_scan_desc* desc) {
@@ -190,13 +158,10 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
   const FwdScratchLayout sl = fwd_scratch_layout(g);
   char* ck = static_cast<char*>(ckpt);
   char* sc = static_cast<char*>(scratch);
-  cudaError_t e = cudaMemsetAsync(sc, 0, sl.zero_bytes, st);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  e = cudaMemsetAsync(ck + cl.off_trailer, 0, 256, st);
-  if (e != cudaSuccess) return static_cast<int>(e);
 
   FwdParams p;
   fill_common(p, desc, g);
+  p.inject = (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0;
   p.u = u; p.fl = f_logit; p.il = i_logit; p.Bm = Bm; p.Cm = Cm; p.Dskip = D_skip; p.h0 = h0;
   p.y = y; p.hT = hT; p.pT = pT;
   p.ckS = reinterpret_cast<float*>(ck + cl.off_S);
@@ -216,12 +181,7 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;
   }
   if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
-  if (rck != 0) return rck;
-  PoisonList pl = {};
-  poison_add(pl, y, static_cast<size_t>(desc->B) * desc->T * desc->D * dtype_size(desc->act_dtype));
-  poison_add(pl, hT, static_cast<size_t>(nstate) * 4);
-  poison_add(pl, pT, static_cast<size_t>(nchan) * 4);
-  return launch_poison(p.hdr, p.fwd_form, true, (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0, pl, st);
+  return rck;
 }
 
 int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit,
@@ -250,8 +210,8 @@ int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit
   const BwdScratchLayout sl = bwd_scratch_layout(g);
   const char* ck = static_cast<const char*>(ckpt);
   char* sc = static_cast<char*>(scratch);
-  cudaError_t e = cudaMemsetAsync(sc, 0, sl.zero_bytes, st);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  rc = launch_init(reinterpret_cast<ScratchHeader*>(sc), sl.zero_bytes, nullptr, st);
+  if (rc != 0) return rc;
 
   BwdParams p;
   fill_common(p, desc, g);
@@ -277,19 +237,10 @@ int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     if (rc2 == 0) p.tc_launched = 1;
     else if (rc2 != -1000) return rc2;
   }
-  const int rcs = launch_bwd_simt(p, g, desc->act_dtype, desc->gate_dtype, dB, dC, dD, stream);
-  if (rcs != 0) return rcs;
-  PoisonList pl = {};
-  const size_t ntd = static_cast<size_t>(desc->B) * desc->T * desc->D;
-  const size_t ntn = static_cast<size_t>(desc->B) * desc->T * desc->N;
-  poison_add(pl, du, ntd * dtype_size(desc->act_dtype));
-  poison_add(pl, dfl, ntd * dtype_size(desc->gate_dtype));
-  poison_add(pl, dil, ntd * dtype_size(desc->gate_dtype));
-  poison_add(pl, dB, ntn * dtype_size(desc->bc_dtype));
-  poison_add(pl, dC, ntn * dtype_size(desc->bc_dtype));
-  poison_add(pl, dD, static_cast<size_t>(desc->D) * 4);
-  poison_add(pl, dh0, static_cast<size_t>(desc->B) * desc->D * desc->N * 4);
-  return launch_poison(p.hdr, const_cast<int*>(p.fwd_form), false, (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0, pl, st);
+  rc = launch_bwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
+  if (rc != 0) return rc;
+  return launch_bwd_finalize(p, g, desc->act_dtype, desc->gate_dtype, dB, dC, dD,
+                             (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0, stream);
 }
 
 int naju_b200_step(const naju_scan_desc* desc, float* state, const void* u, const void* f_logit,

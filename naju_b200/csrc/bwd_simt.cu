@@ -10,427 +10,469 @@
 //
 // r_t obeys a scalar recurrence, r_t = r_{t+1} + dy_t <C_t, x_t> - w_t g_t, seeded at the
 // chunk end by r = <carry_in, x_end>.  That removes the need to hold x_t and xbar_t at the
-// same time: a tile (TC steps x 128 channels, thread = channel) is walked once forward from
-// the chunk-start state the forward saved (states, dC, dy*cx, the adjoint aggregate) and once
-// in reverse (adjoint, dB, du, d f_logit, d i_logit).  The adjoint carry crosses chunks by the
-// same bounded decoupled look-back as the forward, run towards later chunks.
-// dB/dC are reduced over the tile's channels by a fixed-order warp reduce-scatter and written
-// as per-channel-tile partials; small finalize kernels add the partials (deterministic).
-#include "common.cuh"
-#include "params.h"
-
+// same time: a tile (TC steps x 128 channels; a thread owns four channels x K states, simt_common.cuh) is
+// walked once forward from the chunk-start state the forward saved (states, dC, dy*cx, the adjoint
+// aggregate) and once in reverse (adjoint, dB, g, r); the elementwise gradients follow from g and r in a
+// pass over the tile that reads the logits again (they are still in L2).  The adjoint carry crosses chunks
+// by the same bounded decoupled look-back as the forward, run towards later chunks.
+// Shared memory holds the gates of kSB = 32 steps; the 64-step chunks of the tensor-core kernels, whose
+// checkpoints this kernel takes over when their backward stands down, go through it in two pieces.
+// dB/dC are reduced over the tile's channels in registers, by a fixed-order warp reduce-scatter and across
+// the warps, and written as per-channel-tile partials; a finalize kernel adds those (deterministic).
 #include <algorithm>
+
+#include "simt_common.cuh"
+#include "tma_host.h"
 
 namespace naju {
 
-constexpr int kG = 8;  // time steps between two cross-warp partial-sum flushes
+using namespace simt;
+
 // Below this retention the difference form of d f_logit loses more than ~3e-5 relative
 // accuracy (it matches the f_logit >= -5 envelope of naju/chunk_triton.py:200).
 constexpr float kDeepGate = 0.0078125f;
 
-template <typename TA, typename TG, int NS, int TC>
-__global__ void __launch_bounds__(kThreads) bwd_simt_kernel(const BwdParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TA* s_u = reinterpret_cast<TA*>(smem_raw);             // [TC][128]; reused for du
-  TA* s_dy = s_u + TC * kDT;                             // [TC][128]
-  TG* s_fl = reinterpret_cast<TG*>(s_dy + TC * kDT);     // [TC][128]; reused for dfl
-  TG* s_il = s_fl + TC * kDT;                            // [TC][128]; reused for dil
-  float* s_B = reinterpret_cast<float*>(s_il + TC * kDT);   // [TC][NS]
-  float* s_C = s_B + TC * NS;                               // [TC][NS]
-  float* s_a = s_C + TC * NS;                               // [TC][128]  dy_t * <C_t, x_t>
-  float* s_part = s_a + TC * kDT;                           // [kWarps][kG][NS]
+template <int NS>
+struct BwdShape : Shape<NS> {
+  // steps between two cross-warp flushes of the dB / dC partial sums
+  static constexpr int G = NS == 16 ? 16 : NS == 32 ? 8 : 8;
+  static constexpr int part_floats = Shape<NS>::W * G * NS;
+};
+
+template <typename TA, typename TG, int NS, int NH>
+__global__ void __launch_bounds__(Shape<NS>::NT, NS == 128 ? 1 : NS == 64 ? 2 : NH == 2 ? 2 : 3)
+bwd_simt_kernel(const BwdParams p) {
+  using S = BwdShape<NS>;
+  constexpr int K = S::K, L = S::L, GW = S::GW, W = S::W, NT = S::NT, G = S::G, TC = NH * kSB;
+  using RG = ReduceGroups<K, L, GW>;
+  extern __shared__ __align__(16) float sm[];
+  float* s_f = sm;                       // [kSB][128] retention; du on its way out of a time-contiguous layout
+  float* s_w = s_f + kSB * kDT;          // [kSB][128] i u
+  float* s_dy = s_w + kSB * kDT;         // [kSB][128] dy; g replaces it in the reverse walk
+  float* s_a = s_dy + kSB * kDT;         // [TC][128] dy_t <C_t, x_t>; r replaces it in the reverse walk
+  float* s_B = s_a + TC * kDT;           // [TC][NS]
+  float* s_C = s_B + TC * NS;            // [TC][NS]
+  float* s_part = s_C + TC * NS;         // [W][G][NS]; also the dD partials [W][128]
   __shared__ unsigned int s_ticket;
 
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
   // the tensor-core backward was launched for this call and is doing the work
   if (p.tc_launched && (*p.fwd_form & 3) == 1) return;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (blockIdx.x == 0 && tid == 0) p.hdr->form = NAJU_FORM_RECURRENT;
+
+  const int q = lane % L, g = lane / L, chan0 = (warp * GW + g) * kC, my_ch = chan0 + chan_of<L>(q);
+  const bool ch_writer = L == 4 || (q % (L / 4)) == 0;
+  const int part_n = q * K + RG::base(g);
+  const bool part_writer = !RG::dup || (g & 1) == 0;
+  const int per_chunk = p.B * p.ndt;
+
   // Persistent CTAs: each takes tile tickets (reverse-time-major, so the chunk a tile waits on is
   // always held by a running CTA or done) until they run out.  The grid is a few CTAs per SM, which
   // also makes the stand-down above cost a few microseconds instead of one CTA launch per tile.
   for (;;) {
-  __syncthreads();  // the previous tile is done with shared memory (and with s_ticket)
-  if (tid == 0) s_ticket = atomicAdd(&p.hdr->ticket, 1u);
-  __syncthreads();
-  const int per_chunk = p.B * p.ndt;
-  const int order = static_cast<int>(s_ticket / per_chunk);  // 0 = last chunk in time
-  const int rem = static_cast<int>(s_ticket % per_chunk);
-  if (order >= p.nchunks) return;
-  const int c = p.nchunks - 1 - order;
-  const int b = rem / p.ndt, dt = rem % p.ndt;
-  const int64_t tile = static_cast<int64_t>(c) * per_chunk + rem;
-  const int t0 = c * TC;
-  const int len = min(TC, p.T - t0);
-  const int d0 = dt * kDT;
-  const int cols = min(kDT, p.D - d0);
-  const int d = d0 + tid;
-  const bool d_ok = d < p.D;
+    __syncthreads();  // the previous tile is done with shared memory (and with s_ticket)
+    if (tid == 0) s_ticket = atomicAdd(&p.hdr->ticket, 1u);
+    __syncthreads();
+    const int order = static_cast<int>(s_ticket / per_chunk);  // 0 = last chunk in time
+    const int rem = static_cast<int>(s_ticket % per_chunk);
+    if (order >= p.nchunks) return;
+    const int c = p.nchunks - 1 - order;
+    const int b = rem / p.ndt, dt = rem % p.ndt;
+    const int64_t tile = static_cast<int64_t>(c) * per_chunk + rem;
+    const int t0 = c * TC, len = min(TC, p.T - t0), d0 = dt * kDT, cols = min(kDT, p.D - d0), d = d0 + chan0;
+    const int64_t slot0 = tile * kDT + chan0, bd0 = static_cast<int64_t>(b) * p.D + d;
+    const int64_t part_row0 = (static_cast<int64_t>(b) * p.T + t0) * p.ndt + dt;  // + t*ndt
+    float4 dd = make_float4(0.f, 0.f, 0.f, 0.f);
 
-  if (p.u_sd > 1)
-    load_tile_tmajor(s_u, reinterpret_cast<const TA*>(p.u) + b * p.u_sb + t0 + d0 * p.u_sd, p.u_sd, len, cols, tid);
-  else
-    load_tile_async(s_u, reinterpret_cast<const TA*>(p.u) + b * p.u_sb + t0 * p.u_st + d0, p.u_st,
-                    len, cols, tid);
-  load_tile_async(s_dy, reinterpret_cast<const TA*>(p.dy) + (static_cast<int64_t>(b) * p.T + t0) * p.D + d0,
-                  static_cast<int64_t>(p.D), len, cols, tid);
-  load_tile_async(s_fl, reinterpret_cast<const TG*>(p.fl) + b * p.fl_sb + t0 * p.fl_st + d0,
-                  p.fl_st, len, cols, tid);
-  load_tile_async(s_il, reinterpret_cast<const TG*>(p.il) + b * p.il_sb + t0 * p.il_st + d0,
-                  p.il_st, len, cols, tid);
-  cp_async_commit();
-  load_bc_tile<NS>(s_B, p.Bm, p.bc_dtype, b * p.bm_sb + t0 * p.bm_st, p.bm_st, len, p.N, tid);
-  load_bc_tile<NS>(s_C, p.Cm, p.bc_dtype, b * p.cm_sb + t0 * p.cm_st, p.cm_st, len, p.N, tid);
-
-  // chunk-start state: the forward's inclusive state of the previous chunk (or h0)
-  float x[NS];
-  if (c == 0) {
+    auto stage = [&](int h, float4& dd) {
+      if (p.u_sd > 1) {
+        load_tmajor<TA, NT>(s_w, reinterpret_cast<const TA*>(p.u) + b * p.u_sb + t0 + h * kSB + static_cast<int64_t>(d0) * p.u_sd,
+                            p.u_sd, len - h * kSB, cols, tid);
+        __syncthreads();
+      }
+      stage_gates<TA, TG, NT, true>(p, s_f, s_w, s_dy, b, t0 + h * kSB, len - h * kSB, d0, tid, dd);
+    };
+    // the partial sums of steps [h kSB + tg, + G) over the tile's channels, summed over the warps
+    auto flush = [&](float* part, int t_first) {
+      __syncthreads();
+      for (int e = tid; e < G * NS; e += NT) {
+        const int gg = e / NS, n = e % NS;
+        if (t_first + gg < len) {
+          float s = 0.f;
 #pragma unroll
-    for (int n = 0; n < NS; ++n)
-      x[n] = (p.h0 != nullptr && d_ok && n < p.N) ? p.h0[(static_cast<int64_t>(b) * p.D + d) * p.N + n] : 0.f;
-  } else {
-    const float4* src =
-        reinterpret_cast<const float4*>(p.ckS + ((tile - per_chunk) * kDT + tid) * NS);
-#pragma unroll
-    for (int q = 0; q < NS / 4; ++q) {
-      const float4 v = __ldg(src + q);
-      x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-
-  const int nbase = WarpRS<NS>::out_base(lane);
-  constexpr int OC = WarpRS<NS>::out_count;
-  // For NS == 16 lanes 2k and 2k+1 end up with the same total; only even lanes write it.
-  const bool writer = (NS >= 32) || ((lane & 1) == 0);
-  const int64_t part_row0 = (static_cast<int64_t>(b) * p.T + t0) * p.ndt + dt;  // + t*ndt
-
-  // ---------------- forward walk: states, dC partials, a_t, adjoint aggregate
-  float lam[NS];
-#pragma unroll
-  for (int n = 0; n < NS; ++n) lam[n] = 0.f;
-  float P = 1.f, dDsum = 0.f;
-  for (int tg = 0; tg < len; tg += kG) {
-#pragma unroll 1
-    for (int g = 0; g < kG; ++g) {
-      const int t = tg + g;
-      if (t < len) {
-        const float ut = to_f32(s_u[t * kDT + tid]);
-        const float dyt = to_f32(s_dy[t * kDT + tid]);
-        const float f = sigmoid_f(to_f32(s_fl[t * kDT + tid]));
-        const float w = sigmoid_f(to_f32(s_il[t * kDT + tid])) * ut;
-        P *= f;
-        dDsum = fmaf(dyt, ut, dDsum);
-        const float pdy = P * dyt;
-        const float4* Bt = reinterpret_cast<const float4*>(s_B + t * NS);
-        const float4* Ct = reinterpret_cast<const float4*>(s_C + t * NS);
-        float cx = 0.f;
-        float dc[NS];
-#pragma unroll
-        for (int q = 0; q < NS / 4; ++q) {
-          const float4 bv = Bt[q];
-          const float4 cv = Ct[q];
-          x[4 * q + 0] = fmaf(f, x[4 * q + 0], w * bv.x);
-          x[4 * q + 1] = fmaf(f, x[4 * q + 1], w * bv.y);
-          x[4 * q + 2] = fmaf(f, x[4 * q + 2], w * bv.z);
-          x[4 * q + 3] = fmaf(f, x[4 * q + 3], w * bv.w);
-          cx = fmaf(cv.x, x[4 * q + 0], cx);
-          cx = fmaf(cv.y, x[4 * q + 1], cx);
-          cx = fmaf(cv.z, x[4 * q + 2], cx);
-          cx = fmaf(cv.w, x[4 * q + 3], cx);
-          lam[4 * q + 0] = fmaf(pdy, cv.x, lam[4 * q + 0]);
-          lam[4 * q + 1] = fmaf(pdy, cv.y, lam[4 * q + 1]);
-          lam[4 * q + 2] = fmaf(pdy, cv.z, lam[4 * q + 2]);
-          lam[4 * q + 3] = fmaf(pdy, cv.w, lam[4 * q + 3]);
-          dc[4 * q + 0] = dyt * x[4 * q + 0];
-          dc[4 * q + 1] = dyt * x[4 * q + 1];
-          dc[4 * q + 2] = dyt * x[4 * q + 2];
-          dc[4 * q + 3] = dyt * x[4 * q + 3];
-        }
-        s_a[t * kDT + tid] = dyt * cx;
-        WarpRS<NS>::run(dc, lane);
-        if (writer) {
-#pragma unroll
-          for (int j = 0; j < OC; ++j) s_part[(warp * kG + g) * NS + nbase + j] = dc[j];
+          for (int wq = 0; wq < W; ++wq) s += s_part[(wq * G + gg) * NS + n];
+          part[(part_row0 + static_cast<int64_t>(t_first + gg) * p.ndt) * NS + n] = s;
         }
       }
+      __syncthreads();
+    };
+    auto chunk_start_state = [&](float (&v)[kC][K]) {   // the forward's inclusive state of the previous chunk, or h0
+      if (c == 0) get_user_state<K>(p.h0, bd0, d, p.D, p.N, q, v);
+      else get_state<NS, K>(p.ckS, slot0 - static_cast<int64_t>(per_chunk) * kDT, q, v);
+    };
+
+    float x[kC][K];
+    {
+      StageBC<NS, NT, TC> bc;
+      bc.load(p, b, t0, len, tid);
+      chunk_start_state(x);
+      stage(0, dd);
+      bc.store(p, s_B, s_C, b, t0, len, tid);
     }
     __syncthreads();
-    for (int e = tid; e < kG * NS; e += kThreads) {
-      const int g = e / NS, n = e % NS;
-      if (tg + g < len) {
+
+    // ---------------- forward walk: states, dC partials, a_t, adjoint aggregate
+    float lam[kC][K], P[kC];
+    [[maybe_unused]] float xh[NH == 2 ? kC : 1][NH == 2 ? K : 1];   // state between the two pieces
+#pragma unroll
+    for (int k = 0; k < kC; ++k) {
+      P[k] = 1.f;
+#pragma unroll
+      for (int n = 0; n < K; ++n) lam[k][n] = 0.f;
+    }
+#pragma unroll 1
+    for (int h = 0; h < NH; ++h) {
+      if (h > 0) {
+        if constexpr (NH == 2)
+#pragma unroll
+          for (int k = 0; k < kC; ++k)
+#pragma unroll
+            for (int n = 0; n < K; ++n) xh[k][n] = x[k][n];
+        stage(h, dd);
+        __syncthreads();
+      }
+#pragma unroll 1
+      for (int tg = 0; tg < kSB; tg += G) {
+#pragma unroll 2
+        for (int gg = 0; gg < G; ++gg) {
+          const int tl = tg + gg, t = h * kSB + tl;
+          float f[kC], w[kC], y[kC], Bv[K], Cv[K], cx[kC], dc[K];
+          lds_row<kC>(s_f + tl * kDT + chan0, f);
+          lds_row<kC>(s_w + tl * kDT + chan0, w);
+          lds_row<kC>(s_dy + tl * kDT + chan0, y);
+          lds_row<K>(s_B + t * NS + q * K, Bv);
+          lds_row<K>(s_C + t * NS + q * K, Cv);
+#pragma unroll
+          for (int k = 0; k < kC; ++k) {
+            P[k] *= f[k];
+            const float pdy = P[k] * y[k];
+            cx[k] = 0.f;
+#pragma unroll
+            for (int n = 0; n < K; ++n) {
+              x[k][n] = fmaf(f[k], x[k][n], w[k] * Bv[n]);
+              cx[k] = fmaf(Cv[n], x[k][n], cx[k]);
+              lam[k][n] = fmaf(pdy, Cv[n], lam[k][n]);
+              dc[n] = k == 0 ? y[0] * x[0][n] : fmaf(y[k], x[k][n], dc[n]);
+            }
+            cx[k] *= y[k];
+          }
+          const float a = reduce_states<L>(cx, q);
+          if (ch_writer) s_a[t * kDT + my_ch] = a;
+          RG::run(dc, g);
+          if (part_writer)
+#pragma unroll
+            for (int j = 0; j < RG::count; ++j) s_part[(warp * G + gg) * NS + part_n + j] = dc[j];
+        }
+        flush(p.dCpart, h * kSB + tg);
+      }
+    }
+    {
+      // dD partials: a thread holds the sums of four channels over its rows
+      *reinterpret_cast<float4*>(s_part + warp * kDT + 4 * lane) = dd;
+      __syncthreads();
+      for (int e = tid; e < kDT; e += NT) {
         float s = 0.f;
 #pragma unroll
-        for (int wq = 0; wq < kWarps; ++wq) s += s_part[(wq * kG + g) * NS + n];
-        p.dCpart[(part_row0 + static_cast<int64_t>(tg + g) * p.ndt) * NS + n] = s;
+        for (int wq = 0; wq < W; ++wq) s += s_part[wq * kDT + e];
+        p.dDpart[(static_cast<int64_t>(c) * p.B + b) * (p.ndt * kDT) + d0 + e] = s;
       }
     }
-    __syncthreads();
-  }
-  p.dDpart[(static_cast<int64_t>(c) * p.B + b) * (p.ndt * kDT) + d0 + tid] = dDsum;
 
-  // ---------------- adjoint carry-in by decoupled look-back towards later chunks
-  const int64_t slot = tile * kDT + tid;
-  float carry[NS];
-  if (c == p.nchunks - 1) {
-#pragma unroll
-    for (int n = 0; n < NS; ++n)
-      carry[n] = (p.dhT != nullptr && d_ok && n < p.N) ? p.dhT[(static_cast<int64_t>(b) * p.D + d) * p.N + n] : 0.f;
-  } else {
-    p.aggP[slot] = P;
-    float4* dstL = reinterpret_cast<float4*>(p.aggL + slot * NS);
-#pragma unroll
-    for (int q = 0; q < NS / 4; ++q)
-      dstL[q] = make_float4(lam[4 * q], lam[4 * q + 1], lam[4 * q + 2], lam[4 * q + 3]);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(p.flags + tile, 1);
-
-    float accP = 1.f;
-#pragma unroll
-    for (int n = 0; n < NS; ++n) carry[n] = 0.f;
-    for (int j = c + 1; j < p.nchunks; ++j) {
-      const int64_t jt = static_cast<int64_t>(j) * per_chunk + rem;
-      const int64_t js = jt * kDT + tid;
-      const int st = wait_flag(p.flags + jt);
-      if (st == 0) {
-        atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
-        break;
+    // ---------------- adjoint carry-in by decoupled look-back towards later chunks
+    float carry[kC][K];
+    if (c == p.nchunks - 1) {
+      get_user_state<K>(p.dhT, bd0, d, p.D, p.N, q, carry);
+    } else {
+      if (c > 0) {   // (nobody looks back to chunk 0)
+        put_state<NS, K>(p.aggL, slot0, q, lam);
+        if (q == 0) *reinterpret_cast<float4*>(p.aggP + slot0) = make_float4(P[0], P[1], P[2], P[3]);
+        __syncthreads();
+        if (tid == 0) {
+          __threadfence();
+          st_release(p.flags + tile, 1);
+        }
       }
-      const float4* src = reinterpret_cast<const float4*>((st == 2 ? p.inclL : p.aggL) + js * NS);
+      float accP[kC];
+      const int64_t src = look_back<NS, K>(p.flags, p.aggP, p.aggL, p.inclL, tile + per_chunk, per_chunk, p.nchunks - 1 - c, chan0,
+                                           q, lane, carry, accP);
+      if (src < 0) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
+    }
+    // inclusive adjoint leaving this chunk towards earlier time: lam + P * carry_in
+    {
 #pragma unroll
-      for (int q = 0; q < NS / 4; ++q) {
-        const float4 v = __ldcg(src + q);
-        carry[4 * q + 0] = fmaf(accP, v.x, carry[4 * q + 0]);
-        carry[4 * q + 1] = fmaf(accP, v.y, carry[4 * q + 1]);
-        carry[4 * q + 2] = fmaf(accP, v.z, carry[4 * q + 2]);
-        carry[4 * q + 3] = fmaf(accP, v.w, carry[4 * q + 3]);
+      for (int k = 0; k < kC; ++k)
+#pragma unroll
+        for (int n = 0; n < K; ++n) lam[k][n] = fmaf(P[k], carry[k][n], lam[k][n]);
+      if (c > 0) {
+        put_state<NS, K>(p.inclL, slot0, q, lam);
+        __syncthreads();
+        if (tid == 0) {
+          __threadfence();
+          st_release(p.flags + tile, 2);
+        }
+      } else {
+        __syncthreads();
+        if (p.dh0 != nullptr) put_user_state<K>(p.dh0, bd0, d, p.D, p.N, q, lam);
       }
-      if (st == 2) break;
-      accP *= __ldcg(p.aggP + js);
     }
-  }
-  // inclusive adjoint leaving this chunk towards earlier time: lam + P * carry_in
-  {
-    float4* dstL = reinterpret_cast<float4*>(p.inclL + slot * NS);
-#pragma unroll
-    for (int q = 0; q < NS / 4; ++q)
-      dstL[q] = make_float4(fmaf(P, carry[4 * q + 0], lam[4 * q + 0]), fmaf(P, carry[4 * q + 1], lam[4 * q + 1]),
-                            fmaf(P, carry[4 * q + 2], lam[4 * q + 2]), fmaf(P, carry[4 * q + 3], lam[4 * q + 3]));
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(p.flags + tile, 2);
-    if (c == 0 && p.dh0 != nullptr && d_ok) {
-      float* o = p.dh0 + (static_cast<int64_t>(b) * p.D + d) * p.N;
-#pragma unroll
-      for (int n = 0; n < NS; ++n)
-        if (n < p.N) o[n] = fmaf(P, carry[n], lam[n]);
-    }
-  }
 
-  // ---------------- reverse walk
-  float r = 0.f;
+    // ---------------- reverse walk
+    float r;   // of channel my_ch
+    {
+      float v[kC];
 #pragma unroll
-  for (int n = 0; n < NS; ++n) r = fmaf(carry[n], x[n], r);
-  const float Dv = d_ok ? p.Dskip[d] : 0.f;
-  const int last_group = ((len - 1) / kG) * kG;
-  for (int tg = last_group; tg >= 0; tg -= kG) {
+      for (int k = 0; k < kC; ++k) {
+        v[k] = 0.f;
+#pragma unroll
+        for (int n = 0; n < K; ++n) v[k] = fmaf(carry[k][n], x[k][n], v[k]);
+      }
+      r = reduce_states<L>(v, q);
+    }
 #pragma unroll 1
-    for (int g = kG - 1; g >= 0; --g) {
-      const int t = tg + g;
-      if (t < len) {
-        const float ut = to_f32(s_u[t * kDT + tid]);
-        const float dyt = to_f32(s_dy[t * kDT + tid]);
-        const Gate fg = gate(to_f32(s_fl[t * kDT + tid]));
-        const Gate ig = gate(to_f32(s_il[t * kDT + tid]));
-        const float f = fg.s, w = ig.s * ut;
-        const float4* Bt = reinterpret_cast<const float4*>(s_B + t * NS);
-        const float4* Ct = reinterpret_cast<const float4*>(s_C + t * NS);
-        // Deep retention gate: r_t = f_t <xbar_t, x_{t-1}> is then far smaller than the two
-        // terms whose difference the recurrence forms, so it is computed directly instead,
-        // from x_{t-1} re-walked from the chunk-start state (rare; cost O(t) for this thread).
-        const bool deep = f < kDeepGate;
-        float r_exact = 0.f;
-        if (deep) {
-          float xp[NS];
-          if (c == 0) {
+    for (int h = NH - 1; h >= 0; --h) {
+      if (h < NH - 1) {
+        float4 again = make_float4(0.f, 0.f, 0.f, 0.f);
+        stage(h, again);
+        __syncthreads();
+      }
+#pragma unroll 1
+      for (int tg = kSB - G; tg >= 0; tg -= G) {
+#pragma unroll 2
+        for (int gg = G - 1; gg >= 0; --gg) {
+          const int tl = tg + gg, t = h * kSB + tl;
+          float f[kC], w[kC], y[kC], Bv[K], Cv[K], gs[kC], db[K];
+          lds_row<kC>(s_f + tl * kDT + chan0, f);
+          lds_row<kC>(s_w + tl * kDT + chan0, w);
+          lds_row<kC>(s_dy + tl * kDT + chan0, y);
+          lds_row<K>(s_B + t * NS + q * K, Bv);
+          lds_row<K>(s_C + t * NS + q * K, Cv);
+          const float a = s_a[t * kDT + my_ch], wm = s_w[tl * kDT + my_ch];
+          // Deep retention gate: r_t = f_t <xbar_t, x_{t-1}> is then far smaller than the two
+          // terms whose difference the recurrence forms, so it is computed directly instead,
+          // from x_{t-1} re-walked from the start of the piece (rare; cost O(t) for this warp).
+          float r_exact = 0.f;
+          bool deep_m = false;
+          if (__any_sync(0xffffffffu, fminf(fminf(f[0], f[1]), fminf(f[2], f[3])) < kDeepGate)) {
+            float xp[kC][K], v[kC];
+            if (h == 0) chunk_start_state(xp);
+            else if constexpr (NH == 2)
 #pragma unroll
-            for (int n = 0; n < NS; ++n)
-              xp[n] = (p.h0 != nullptr && d_ok && n < p.N) ? p.h0[(static_cast<int64_t>(b) * p.D + d) * p.N + n] : 0.f;
-          } else {
-            const float4* src =
-                reinterpret_cast<const float4*>(p.ckS + ((tile - per_chunk) * kDT + tid) * NS);
+              for (int k = 0; k < kC; ++k)
 #pragma unroll
-            for (int q = 0; q < NS / 4; ++q) {
-              const float4 v = __ldg(src + q);
-              xp[4 * q] = v.x; xp[4 * q + 1] = v.y; xp[4 * q + 2] = v.z; xp[4 * q + 3] = v.w;
+                for (int n = 0; n < K; ++n) xp[k][n] = xh[k][n];
+#pragma unroll 1
+            for (int tt = 0; tt < tl; ++tt) {
+              float f2[kC], w2[kC], B2[K];
+              lds_row<kC>(s_f + tt * kDT + chan0, f2);
+              lds_row<kC>(s_w + tt * kDT + chan0, w2);
+              lds_row<K>(s_B + (h * kSB + tt) * NS + q * K, B2);
+#pragma unroll
+              for (int k = 0; k < kC; ++k)
+#pragma unroll
+                for (int n = 0; n < K; ++n) xp[k][n] = fmaf(f2[k], xp[k][n], w2[k] * B2[n]);
+            }
+#pragma unroll
+            for (int k = 0; k < kC; ++k) {
+              v[k] = 0.f;
+#pragma unroll
+              for (int n = 0; n < K; ++n) v[k] = fmaf(fmaf(Cv[n], y[k], carry[k][n]), xp[k][n], v[k]);
+            }
+            const float dot = reduce_states<L>(v, q);
+            const float fm = s_f[tl * kDT + my_ch];
+            r_exact = fm * dot;
+            deep_m = fm < kDeepGate;
+          }
+#pragma unroll
+          for (int k = 0; k < kC; ++k) {
+            gs[k] = 0.f;
+#pragma unroll
+            for (int n = 0; n < K; ++n) {
+              const float dx = fmaf(Cv[n], y[k], carry[k][n]);
+              gs[k] = fmaf(dx, Bv[n], gs[k]);
+              db[n] = k == 0 ? dx * w[0] : fmaf(dx, w[k], db[n]);
+              carry[k][n] = f[k] * dx;
             }
           }
-          for (int tt = 0; tt < t; ++tt) {  // inputs of steps < t are still intact in smem
-            const float f2 = sigmoid_f(to_f32(s_fl[tt * kDT + tid]));
-            const float w2 = sigmoid_f(to_f32(s_il[tt * kDT + tid])) * to_f32(s_u[tt * kDT + tid]);
-            const float4* B2 = reinterpret_cast<const float4*>(s_B + tt * NS);
-#pragma unroll
-            for (int q = 0; q < NS / 4; ++q) {
-              const float4 bv = B2[q];
-              xp[4 * q + 0] = fmaf(f2, xp[4 * q + 0], w2 * bv.x);
-              xp[4 * q + 1] = fmaf(f2, xp[4 * q + 1], w2 * bv.y);
-              xp[4 * q + 2] = fmaf(f2, xp[4 * q + 2], w2 * bv.z);
-              xp[4 * q + 3] = fmaf(f2, xp[4 * q + 3], w2 * bv.w);
-            }
+          const float gm = reduce_states<L>(gs, q);
+          r += a - wm * gm;
+          if (deep_m) r = r_exact;
+          __syncwarp();   // the group's lanes have read dy and a of this step
+          if (ch_writer) {
+            s_dy[tl * kDT + my_ch] = gm;
+            s_a[t * kDT + my_ch] = r;
           }
-          float dot = 0.f;
+          RG::run(db, g);
+          if (part_writer)
 #pragma unroll
-          for (int q = 0; q < NS / 4; ++q) {
-            const float4 cv = Ct[q];
-            dot = fmaf(fmaf(cv.x, dyt, carry[4 * q + 0]), xp[4 * q + 0], dot);
-            dot = fmaf(fmaf(cv.y, dyt, carry[4 * q + 1]), xp[4 * q + 1], dot);
-            dot = fmaf(fmaf(cv.z, dyt, carry[4 * q + 2]), xp[4 * q + 2], dot);
-            dot = fmaf(fmaf(cv.w, dyt, carry[4 * q + 3]), xp[4 * q + 3], dot);
-          }
-          r_exact = f * dot;
+            for (int j = 0; j < RG::count; ++j) s_part[(warp * G + gg) * NS + part_n + j] = db[j];
         }
-        float gsum = 0.f;
-        float db[NS];
-#pragma unroll
-        for (int q = 0; q < NS / 4; ++q) {
-          const float4 bv = Bt[q];
-          const float4 cv = Ct[q];
-          const float dx0 = fmaf(cv.x, dyt, carry[4 * q + 0]);
-          const float dx1 = fmaf(cv.y, dyt, carry[4 * q + 1]);
-          const float dx2 = fmaf(cv.z, dyt, carry[4 * q + 2]);
-          const float dx3 = fmaf(cv.w, dyt, carry[4 * q + 3]);
-          gsum = fmaf(dx0, bv.x, gsum);
-          gsum = fmaf(dx1, bv.y, gsum);
-          gsum = fmaf(dx2, bv.z, gsum);
-          gsum = fmaf(dx3, bv.w, gsum);
-          db[4 * q + 0] = dx0 * w; db[4 * q + 1] = dx1 * w;
-          db[4 * q + 2] = dx2 * w; db[4 * q + 3] = dx3 * w;
-          carry[4 * q + 0] = f * dx0; carry[4 * q + 1] = f * dx1;
-          carry[4 * q + 2] = f * dx2; carry[4 * q + 3] = f * dx3;
-        }
-        r += s_a[t * kDT + tid] - w * gsum;
-        if (deep) r = r_exact;
-        s_u[t * kDT + tid] = from_f32<TA>(fmaf(ig.s, gsum, Dv * dyt));
-        s_fl[t * kDT + tid] = from_f32<TG>(fg.one_minus * r);
-        s_il[t * kDT + tid] = from_f32<TG>(gsum * w * ig.one_minus);
-        WarpRS<NS>::run(db, lane);
-        if (writer) {
-#pragma unroll
-          for (int j = 0; j < OC; ++j) s_part[(warp * kG + g) * NS + nbase + j] = db[j];
-        }
+        flush(p.dBpart, h * kSB + tg);
       }
-    }
-    __syncthreads();
-    for (int e = tid; e < kG * NS; e += kThreads) {
-      const int g = e / NS, n = e % NS;
-      if (tg + g < len) {
-        float s = 0.f;
-#pragma unroll
-        for (int wq = 0; wq < kWarps; ++wq) s += s_part[(wq * kG + g) * NS + n];
-        p.dBpart[(part_row0 + static_cast<int64_t>(tg + g) * p.ndt) * NS + n] = s;
+      // ---------------- the elementwise gradients of this piece, four channels of one step per thread
+      const int v = 4 * lane, n = p.D - d0 - v, th = t0 + h * kSB, lenh = len - h * kSB;
+      const int64_t row0 = (static_cast<int64_t>(b) * p.T + th) * p.D + d0 + v;
+      const TG* fl = reinterpret_cast<const TG*>(p.fl) + b * p.fl_sb + static_cast<int64_t>(th) * p.fl_st + d0 + v;
+      const TG* il = reinterpret_cast<const TG*>(p.il) + b * p.il_sb + static_cast<int64_t>(th) * p.il_st + d0 + v;
+      const TA* dy = reinterpret_cast<const TA*>(p.dy) + row0;
+      TG* dfl = reinterpret_cast<TG*>(p.dfl) + row0;
+      TG* dil = reinterpret_cast<TG*>(p.dil) + row0;
+      TA* du = reinterpret_cast<TA*>(p.du) + row0;
+      const bool vf = vec4_ok(fl, p.fl_st), vi = vec4_ok(il, p.il_st), vy = vec4_ok(dy, p.D), vof = vec4_ok(dfl, p.D),
+                 voi = vec4_ok(dil, p.D), vou = vec4_ok(du, p.D);
+      const float4 Dv = load4(p.Dskip + d0 + v, n, vec4_ok(p.Dskip + d0 + v, 4));
+      const bool skip = Dv.x != 0.f || Dv.y != 0.f || Dv.z != 0.f || Dv.w != 0.f;
+#pragma unroll 2
+      for (int tl = warp; tl < min(kSB, lenh); tl += W) {
+        const float4 fv = load4(fl + static_cast<int64_t>(tl) * p.fl_st, n, vf);
+        const float4 iv = load4(il + static_cast<int64_t>(tl) * p.il_st, n, vi);
+        const float4 gg = *reinterpret_cast<const float4*>(s_dy + tl * kDT + v);
+        const float4 rr = *reinterpret_cast<const float4*>(s_a + (h * kSB + tl) * kDT + v);
+        const float4 ww = *reinterpret_cast<const float4*>(s_w + tl * kDT + v);
+        const Gate i0 = gate(iv.x), i1 = gate(iv.y), i2 = gate(iv.z), i3 = gate(iv.w);
+        float4 o = make_float4(i0.s * gg.x, i1.s * gg.y, i2.s * gg.z, i3.s * gg.w);
+        if (skip) {
+          const float4 y = load4(dy + static_cast<int64_t>(tl) * p.D, n, vy);
+          o = make_float4(fmaf(Dv.x, y.x, o.x), fmaf(Dv.y, y.y, o.y), fmaf(Dv.z, y.z, o.z), fmaf(Dv.w, y.w, o.w));
+        }
+        if (p.u_sd > 1) *reinterpret_cast<float4*>(s_f + tl * kDT + v) = o;
+        else store4(du + static_cast<int64_t>(tl) * p.D, o, n, vou);
+        store4(dfl + static_cast<int64_t>(tl) * p.D,
+               make_float4(gate(fv.x).one_minus * rr.x, gate(fv.y).one_minus * rr.y, gate(fv.z).one_minus * rr.z,
+                           gate(fv.w).one_minus * rr.w), n, vof);
+        store4(dil + static_cast<int64_t>(tl) * p.D,
+               make_float4(gg.x * ww.x * i0.one_minus, gg.y * ww.y * i1.one_minus, gg.z * ww.z * i2.one_minus,
+                           gg.w * ww.w * i3.one_minus), n, voi);
       }
+      if (p.u_sd > 1) {   // du in the layout of a time-contiguous u
+        __syncthreads();
+        store_tmajor<TA, NT>(reinterpret_cast<TA*>(p.du) + b * p.u_sb + th + static_cast<int64_t>(d0) * p.u_sd, s_f, p.u_sd,
+                             min(kSB, lenh), cols, tid);
+      }
+      if (h > 0) __syncthreads();   // the next piece is staged over this one
     }
-    __syncthreads();
-  }
-
-  const int64_t out_off = (static_cast<int64_t>(b) * p.T + t0) * p.D + d0;
-  if (p.u_sd > 1)   // du in the layout of a time-contiguous u
-    store_tile_tmajor(reinterpret_cast<TA*>(p.du) + b * p.u_sb + t0 + d0 * p.u_sd, s_u, p.u_sd, len, cols, tid);
-  else
-    store_tile(reinterpret_cast<TA*>(p.du) + out_off, s_u, static_cast<int64_t>(p.D), len, cols, tid);
-  store_tile(reinterpret_cast<TG*>(p.dfl) + out_off, s_fl, static_cast<int64_t>(p.D), len, cols, tid);
-  store_tile(reinterpret_cast<TG*>(p.dil) + out_off, s_il, static_cast<int64_t>(p.D), len, cols, tid);
   }
 }
 
-// out[row][n] = sum_k part[row][k][n] for n < N, written in the caller's dtype
-__global__ void finalize_bc_kernel(const float* __restrict__ part, void* __restrict__ out,
-                                   int64_t rows, int ndt, int NS, int N, int dtype) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= rows * N) return;
-  const int64_t row = i / N;
-  const int n = static_cast<int>(i % N);
-  float s = 0.f;
-  for (int k = 0; k < ndt; ++k) s += part[(row * ndt + k) * NS + n];
-  store_dyn(out, dtype, i, s);
-}
+// ------------------------------------------------------------------------------ finalize
+// dB[row][n] = sum_k part[row][k][n] for n < N (and dC), written in the caller's dtype; dD[d] = the sum over its
+// partial rows.  One launch: blocks [0, nbc) take dB, [nbc, 2 nbc) dC, the rest 32 channels of dD each, in a
+// fixed order throughout.  If a bounded wait of this call or of its forward ran out (or `inject` asks for it),
+// every output is overwritten with all-ones bytes (NaN) instead.
+struct PoisonList {
+  void* ptr[4];
+  unsigned long long bytes[4];
+};
 
-// dD[d] = sum_rows part[row][d]; block = 32 channels x 32 row lanes, fixed-order tree
-__global__ void finalize_dD_kernel(const float* __restrict__ part, float* __restrict__ dD,
-                                   int rows, int rows_tc, const int* __restrict__ fwd_form, int ld, int D) {
-  __shared__ float red[32][33];
-  // the tensor-core backward writes two partial rows per batch row, the recurrent one per chunk
-  if (rows_tc > 0 && (*fwd_form & 3) == 1) rows = rows_tc;
-  const int dl = threadIdx.x, rl = threadIdx.y;
-  const int d = blockIdx.x * 32 + dl;
+__global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* __restrict__ dB, void* __restrict__ dC,
+                                                       float* __restrict__ dD, int NS, int nbc, int dd_rows, int dd_rows_tc,
+                                                       int inject, const PoisonList list) {
+  __shared__ float red[8][33];
+  pdl_wait();
+  if (inject && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
+  const int form = *p.fwd_form;
+  const bool bad = inject || *reinterpret_cast<volatile int*>(&p.hdr->status) != 0 || (form & 4) != 0;
+  const int blk = blockIdx.x;
+  const float nan = __int_as_float(-1);
+  if (bad) {
+    for (int k = 0; k < 4; ++k)
+      for (unsigned long long i = static_cast<unsigned long long>(blk) * 256 + threadIdx.x; i < list.bytes[k];
+           i += static_cast<unsigned long long>(gridDim.x) * 256)
+        static_cast<unsigned char*>(list.ptr[k])[i] = 0xFF;
+  }
+  if (blk < 2 * nbc) {
+    const float* part = blk < nbc ? p.dBpart : p.dCpart;
+    void* out = blk < nbc ? dB : dC;
+    const int64_t i = static_cast<int64_t>(blk < nbc ? blk : blk - nbc) * 256 + threadIdx.x;
+    if (i >= static_cast<int64_t>(p.B) * p.T * p.N) return;
+    const int64_t row = i / p.N;
+    const float* src = part + row * p.ndt * NS + (i - row * p.N);
+    float s = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < p.ndt; ++k) s += src[static_cast<int64_t>(k) * NS];
+    store_dyn(out, p.bc_dtype, i, bad ? nan : s);
+    return;
+  }
+  // the tensor-core backward writes four partial rows per batch row, the recurrent one per chunk
+  const int rows = (dd_rows_tc > 0 && (form & 3) == 1) ? dd_rows_tc : dd_rows;
+  const int dl = threadIdx.x & 31, rl = threadIdx.x >> 5, d = (blk - 2 * nbc) * 32 + dl, ld = p.ndt * kDT;
   float s = 0.f;
-  if (d < D)
-    for (int r = rl; r < rows; r += 32) s += part[static_cast<int64_t>(r) * ld + d];
+  if (d < p.D)
+    for (int r = rl; r < rows; r += 8) s += p.dDpart[static_cast<int64_t>(r) * ld + d];
   red[rl][dl] = s;
   __syncthreads();
-  if (rl == 0 && d < D) {
+  if (rl == 0 && d < p.D) {
     float tot = 0.f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) tot += red[k][dl];
-    dD[d] = tot;
+    for (int k = 0; k < 8; ++k) tot += red[k][dl];
+    dD[d] = bad ? nan : tot;
   }
 }
 
-template <typename TA, typename TG, int NS>
-static int launch_ns(const BwdParams& p, const Geometry& g, cudaStream_t st) {
-  constexpr int TC = (NS <= 32) ? 64 : 32;
-  const size_t smem = static_cast<size_t>(TC) * kDT * (2 * sizeof(TA) + 2 * sizeof(TG)) +
-                      2 * static_cast<size_t>(TC) * NS * 4 + static_cast<size_t>(TC) * kDT * 4 +
-                      static_cast<size_t>(kWarps) * kG * NS * 4;
-  auto kern = bwd_simt_kernel<TA, TG, NS, TC>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
+int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act, int gate, void* dB, void* dC, float* dD, bool inject,
+                        void* stream) {
+  const int64_t ntd = static_cast<int64_t>(g.B) * g.T * g.D, nbc = (static_cast<int64_t>(g.B) * g.T * g.N + 255) / 256;
+  const int64_t blocks = 2 * nbc + (g.D + 31) / 32;
+  if (blocks > 0x7fffffff) return NAJU_E_SHAPE;
+  PoisonList list = {{p.du, p.dfl, p.dil, p.dh0},
+                     {static_cast<unsigned long long>(ntd) * dtype_size(act), static_cast<unsigned long long>(ntd) * dtype_size(gate),
+                      static_cast<unsigned long long>(ntd) * dtype_size(gate),
+                      p.dh0 ? static_cast<unsigned long long>(g.B) * g.D * g.N * 4 : 0ull}};
+  return launch_pdl(finalize_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), p, dB,
+                    dC, dD, g.NS, static_cast<int>(nbc), g.nchunks * g.B, p.tc_launched ? 4 * g.B : 0, inject ? 1 : 0, list);
+}
+
+template <typename TA, typename TG, int NS, int NH>
+static int launch_nh(const BwdParams& p, const Geometry& g, cudaStream_t st) {
+  using S = BwdShape<NS>;
+  constexpr size_t smem = 4 * (static_cast<size_t>(kSB) * kDT * (3 + NH) + 2 * static_cast<size_t>(NH) * kSB * NS +
+                               std::max(S::part_floats, S::W * kDT));
+  auto kern = bwd_simt_kernel<TA, TG, NS, NH>;
+  static std::atomic<unsigned long long> allowed{0};
+  const int rc = allow_smem(kern, smem, allowed);
+  if (rc != 0) return rc;
   // persistent grid: what fits on the GPU at once (the look-back needs every waiting CTA's
   // predecessors to be resident or done, which ticket order guarantees for any grid size)
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const int64_t grid = std::min<int64_t>(g.ntiles, static_cast<int64_t>(sms) * per_sm);
-  kern<<<static_cast<unsigned>(grid), kThreads, smem, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  static std::atomic<int> per_sm_cache{0};
+  int per_sm = per_sm_cache.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, S::NT, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    per_sm_cache.store(per_sm, std::memory_order_relaxed);
+  }
+  const int64_t grid = std::min<int64_t>(g.ntiles, static_cast<int64_t>(tmah::sm_count()) * per_sm);
+  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(S::NT), smem, st, p);
 }
 
 template <typename TA, typename TG>
 static int launch_types(const BwdParams& p, const Geometry& g, cudaStream_t st) {
-  switch (g.NS) {
-    case 16: return launch_ns<TA, TG, 16>(p, g, st);
-    case 32: return launch_ns<TA, TG, 32>(p, g, st);
-    case 64: return launch_ns<TA, TG, 64>(p, g, st);
-    default: return launch_ns<TA, TG, 128>(p, g, st);
+  if (g.NS == 16) {
+    if constexpr (sizeof(TA) == 2)
+      if (g.TC == 64) return launch_nh<TA, TG, 16, 2>(p, g, st);
+    return launch_nh<TA, TG, 16, 1>(p, g, st);
   }
+  if (g.NS == 32) return launch_nh<TA, TG, 32, 1>(p, g, st);
+  if (g.NS == 64) return launch_nh<TA, TG, 64, 1>(p, g, st);
+  return launch_nh<TA, TG, 128, 1>(p, g, st);
 }
 
-int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act, int gate, void* dB, void* dC,
-                    float* dD, void* stream) {
+int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act, int gate, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc;
-  if (act == NAJU_F32 && gate == NAJU_F32) rc = launch_types<float, float>(p, g, st);
-  else if (act == NAJU_BF16 && gate == NAJU_BF16) rc = launch_types<__nv_bfloat16, __nv_bfloat16>(p, g, st);
-  else if (act == NAJU_BF16 && gate == NAJU_F32) rc = launch_types<__nv_bfloat16, float>(p, g, st);
-  else if (act == NAJU_F16 && gate == NAJU_F16) rc = launch_types<__half, __half>(p, g, st);
-  else if (act == NAJU_F16 && gate == NAJU_F32) rc = launch_types<__half, float>(p, g, st);
-  else return NAJU_E_DTYPE;
-  if (rc != 0) return rc;
-
-  const int64_t rows = static_cast<int64_t>(g.B) * g.T;
-  const int64_t total = rows * g.N;
-  const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-  finalize_bc_kernel<<<blocks, 256, 0, st>>>(p.dBpart, dB, rows, g.ndt, g.NS, g.N, p.bc_dtype);
-  finalize_bc_kernel<<<blocks, 256, 0, st>>>(p.dCpart, dC, rows, g.ndt, g.NS, g.N, p.bc_dtype);
-  finalize_dD_kernel<<<(g.D + 31) / 32, dim3(32, 32), 0, st>>>(p.dDpart, dD, g.nchunks * g.B,
-                                                              p.tc_launched ? 4 * g.B : 0, p.fwd_form,
-                                                              g.ndt * kDT, g.D);
-  return static_cast<int>(cudaGetLastError());
+  if (act == NAJU_F32 && gate == NAJU_F32) return launch_types<float, float>(p, g, st);
+  if (act == NAJU_BF16 && gate == NAJU_BF16) return launch_types<__nv_bfloat16, __nv_bfloat16>(p, g, st);
+  if (act == NAJU_BF16 && gate == NAJU_F32) return launch_types<__nv_bfloat16, float>(p, g, st);
+  if (act == NAJU_F16 && gate == NAJU_F16) return launch_types<__half, __half>(p, g, st);
+  if (act == NAJU_F16 && gate == NAJU_F32) return launch_types<__half, float>(p, g, st);
+  return NAJU_E_DTYPE;
 }
 
 }  // namespace naju

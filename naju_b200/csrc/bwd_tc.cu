@@ -186,6 +186,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
   __shared__ float s_Rend[kDT];      // 1 / (retention product of the whole chunk)
   __shared__ float s_seed[2][kDT];   // r at the chunk end: <lam, x_end>
 
+  pdl_wait();
   // stand down unless the forward ran in the chunked form and met no deep-gate tile
   if ((*fwd_form & 3) != 1) return;
 
@@ -856,11 +857,11 @@ template <typename TA, typename TG, bool UTM>
 int launch_bwd_tc_t(const BwdParams& p, const tcb::Maps& maps, const int* fwd_form, int64_t ctiles, cudaStream_t st) {
   constexpr size_t smem = tcb::SmemT<TG>::total;
   auto kern = tcb::bwd_tc_kernel<TA, TG, UTM>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
+  static std::atomic<unsigned long long> allowed{0};
+  const int rc = allow_smem(kern, smem, allowed);
+  if (rc != 0) return rc;
   const int64_t grid = std::min<int64_t>(ctiles, tmah::sm_count());
-  kern<<<static_cast<unsigned>(grid), tcb::NTHREADS, smem, st>>>(p, maps, fwd_form);
-  return static_cast<int>(cudaGetLastError());
+  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(tcb::NTHREADS), smem, st, p, maps, fwd_form);
 }
 }  // namespace
 

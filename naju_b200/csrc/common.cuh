@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "naju_b200.h"
 
 namespace naju {
@@ -104,6 +106,19 @@ inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, 
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
+// Raises a kernel's dynamic shared-memory limit once per device (`done`: a bit per device ordinal, one
+// word per kernel).
+template <typename K>
+inline int allow_smem(K* kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_relaxed) & bit)) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return static_cast<int>(e);
 }
 
 // ---------------------------------------------------------------- async tile movement

@@ -1,5 +1,4 @@
-// Tile-level building blocks of the forward scan shared by the exact recurrent kernel and
-// by the tensor-core kernel's per-tile exact path.
+// Building blocks shared by the forward kernels.
 #pragma once
 
 #include "common.cuh"
@@ -30,30 +29,6 @@ __device__ __forceinline__ bool decode_tile(unsigned ticket, int B, int T, int D
   tc.d = tc.d0 + tid;
   tc.d_ok = tc.d < D;
   return tc.c < nchunks;
-}
-
-// pass 1: local scan of the staged tile from a zero state -> x = chunk-end state, P = prod f
-template <typename TA, typename TG, int NS>
-__device__ __forceinline__ void tile_pass1(const TA* s_u, const TG* s_fl, const TG* s_il,
-                                           const float* s_B, int len, int tid, float (&x)[NS],
-                                           float& P) {
-#pragma unroll
-  for (int n = 0; n < NS; ++n) x[n] = 0.f;
-  P = 1.f;
-  for (int t = 0; t < len; ++t) {
-    const float f = sigmoid_f(to_f32(s_fl[t * kDT + tid]));
-    const float w = sigmoid_f(to_f32(s_il[t * kDT + tid])) * to_f32(s_u[t * kDT + tid]);
-    P *= f;
-    const float4* Bt = reinterpret_cast<const float4*>(s_B + t * NS);
-#pragma unroll
-    for (int q = 0; q < NS / 4; ++q) {
-      const float4 bv = Bt[q];
-      x[4 * q + 0] = fmaf(f, x[4 * q + 0], w * bv.x);
-      x[4 * q + 1] = fmaf(f, x[4 * q + 1], w * bv.y);
-      x[4 * q + 2] = fmaf(f, x[4 * q + 2], w * bv.z);
-      x[4 * q + 3] = fmaf(f, x[4 * q + 3], w * bv.w);
-    }
-  }
 }
 
 // Carry across chunks.  In: (P, S) the tile's local aggregate.  Out: h = state entering the
@@ -131,35 +106,6 @@ __device__ __forceinline__ void carry_lookback(const FwdParams& p, const TileCoo
   }
 }
 
-// pass 2: scan from the true carry-in, y written into the u tile; x ends as the chunk-end state
-template <typename TA, typename TG, int NS>
-__device__ __forceinline__ void tile_pass2(TA* s_u, const TG* s_fl, const TG* s_il,
-                                           const float* s_B, const float* s_C, int len, int tid,
-                                           float Dv, float (&x)[NS]) {
-  for (int t = 0; t < len; ++t) {
-    const float ut = to_f32(s_u[t * kDT + tid]);
-    const float f = sigmoid_f(to_f32(s_fl[t * kDT + tid]));
-    const float w = sigmoid_f(to_f32(s_il[t * kDT + tid])) * ut;
-    const float4* Bt = reinterpret_cast<const float4*>(s_B + t * NS);
-    const float4* Ct = reinterpret_cast<const float4*>(s_C + t * NS);
-    float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-    for (int q = 0; q < NS / 4; ++q) {
-      const float4 bv = Bt[q];
-      const float4 cv = Ct[q];
-      x[4 * q + 0] = fmaf(f, x[4 * q + 0], w * bv.x);
-      x[4 * q + 1] = fmaf(f, x[4 * q + 1], w * bv.y);
-      x[4 * q + 2] = fmaf(f, x[4 * q + 2], w * bv.z);
-      x[4 * q + 3] = fmaf(f, x[4 * q + 3], w * bv.w);
-      acc0 = fmaf(cv.x, x[4 * q + 0], acc0);
-      acc1 = fmaf(cv.y, x[4 * q + 1], acc1);
-      acc0 = fmaf(cv.z, x[4 * q + 2], acc0);
-      acc1 = fmaf(cv.w, x[4 * q + 3], acc1);
-    }
-    s_u[t * kDT + tid] = from_f32<TA>(fmaf(Dv, ut, acc0 + acc1));
-  }
-}
-
 // final state / total decay outputs of the last chunk
 template <int NS>
 __device__ __forceinline__ void write_final(const FwdParams& p, const TileCoord& tc,
@@ -173,6 +119,37 @@ __device__ __forceinline__ void write_final(const FwdParams& p, const TileCoord&
     }
     if (p.pT != nullptr) p.pT[static_cast<int64_t>(tc.b) * p.D + tc.d] = Ptot;
   }
+}
+
+// End of a forward kernel, called by every thread of every CTA after its last write.  The last CTA to
+// get here looks at the status word: if a bounded wait ran out anywhere (or `inject` asks for it), it
+// overwrites every output with all-ones bytes (NaN in fp32, bf16 and fp16 alike) and marks the checkpoints, so
+// that a timeout can never pass for a result; no host round trip and no extra launch is needed for that.
+template <typename TA>
+__device__ __forceinline__ void finish_forward(const FwdParams& p) {
+  __shared__ int s_bad;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_bad = 0;
+    if (atomicAdd(&p.hdr->done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      if (p.inject) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
+      if (*reinterpret_cast<volatile int*>(&p.hdr->status) != 0) {
+        s_bad = 1;
+        atomicOr(p.fwd_form, 4);
+      }
+    }
+  }
+  __syncthreads();
+  if (!s_bad) return;
+  auto fill = [&](void* ptr, int64_t bytes) {
+    if (ptr != nullptr)
+      for (int64_t i = threadIdx.x; i < bytes; i += blockDim.x) static_cast<unsigned char*>(ptr)[i] = 0xFF;
+  };
+  fill(p.y, static_cast<int64_t>(p.B) * p.T * p.D * static_cast<int64_t>(sizeof(TA)));
+  fill(p.hT, static_cast<int64_t>(p.B) * p.D * p.N * 4);
+  fill(p.pT, static_cast<int64_t>(p.B) * p.D * 4);
 }
 
 }  // namespace naju

@@ -625,6 +625,7 @@ fwd_tc2_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int n
   }
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+  finish_forward<TA>(p);
 }
 
 }  // namespace tc2
@@ -648,12 +649,13 @@ template <typename TA, typename TG>
 int launch_tc2_m(const FwdParams& p, const Geometry& g, const tc2::Maps& maps, cudaStream_t st) {
   const size_t smem = tc2::Smem<TG>::total;
   auto kern = tc2::fwd_tc2_kernel<TA, TG>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
+  static std::atomic<unsigned long long> allowed{0};
+  int rc = allow_smem(kern, smem, allowed);
+  if (rc == 0) rc = launch_init(p.hdr, static_cast<size_t>(256 + g.ntiles * 4), p.fwd_form, st);
+  if (rc != 0) return rc;
   // one persistent CTA per SM; in walk mode one CTA per channel tile
   const int64_t grid = std::min<int64_t>(g.ntiles, tmah::sm_count());
-  kern<<<static_cast<unsigned>(grid), tc2::NTHREADS, smem, st>>>(p, maps, static_cast<int>(g.ntiles));
-  return static_cast<int>(cudaGetLastError());
+  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(tc2::NTHREADS), smem, st, p, maps, static_cast<int>(g.ntiles));
 }
 
 template <typename TA, typename TG>

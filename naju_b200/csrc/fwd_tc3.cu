@@ -230,10 +230,6 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
     }
     mbar_init(smem_u32(&bars.h_ready), NCARRY / 32);
     mbar_init_fence();
-    if (blockIdx.x == 0) {
-      atomicOr(p.fwd_form, 1);  // tell the backward how the forward ran
-      p.hdr->form = NAJU_FORM_TC_WALK;
-    }
   }
   if (warp == 0) tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
   // the upper triangle of g1/g2 is never written again: clear the shared operands once
@@ -244,6 +240,11 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
+  pdl_wait();   // nothing above touches global memory
+  if (blockIdx.x == 0 && tid == 0) {
+    atomicOr(p.fwd_form, 1);  // tell the backward how the forward ran
+    p.hdr->form = NAJU_FORM_TC_WALK;
+  }
   auto timeout = [&]() { atomicOr(&p.hdr->status, NAJU_ST_MMA_TIMEOUT); };
   // u is time-contiguous: its slabs sit in shared memory as [channel][step].  (A compile-time
   // switch: as a run-time one it cost the usual layout 5 %.)
@@ -685,6 +686,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   }
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+  finish_forward<TA>(p);
 }
 
 }  // namespace tc3
@@ -696,12 +698,13 @@ template <typename TA, typename TG, bool UTM>
 int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, cudaStream_t st) {
   const size_t smem = tc3::Smem<TG>::total;
   auto kern = tc3::fwd_tc3_kernel<TA, TG, UTM>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
+  static std::atomic<unsigned long long> allowed{0};
+  int rc = allow_smem(kern, smem, allowed);
+  if (rc == 0) rc = launch_init(p.hdr, 256, p.fwd_form, st);
+  if (rc != 0) return rc;
   // one persistent CTA per SM; channel tiles are dealt round-robin
   const int64_t grid = std::min<int64_t>(static_cast<int64_t>(g.B) * g.ndt, tmah::sm_count());
-  kern<<<static_cast<unsigned>(grid), tc3::NTHREADS, smem, st>>>(p, maps);
-  return static_cast<int>(cudaGetLastError());
+  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(tc3::NTHREADS), smem, st, p, maps);
 }
 
 }  // namespace

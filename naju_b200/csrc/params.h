@@ -1,6 +1,7 @@
 // Host/device parameter blocks and workspace layouts of the scan kernels.
 #pragma once
 
+#include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
 
@@ -10,8 +11,13 @@ namespace naju {
 
 // Padded state width: the kernels are instantiated for these widths and pad B/C with zeros.
 inline int padded_states(int N) { return N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128; }
-// Chunk length (time steps per tile); the spacing of the saved chunk-boundary states.
-inline int chunk_len_for(int NS) { return NS <= 32 ? 64 : 32; }
+// Chunk length (time steps per tile); the spacing of the saved chunk-boundary states.  64 for the types
+// and the state width that the tensor-core kernels take (their tiles are 64 steps), 32 for everything
+// else: half the shared memory per tile of the recurrent kernels, so three instead of one of their
+// backward's CTAs fit on an SM.
+inline int chunk_len_for(const naju_scan_desc& d) {
+  return (d.N == 16 && d.act_dtype != NAJU_F32 && d.bc_dtype == NAJU_BF16) ? 64 : 32;
+}
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -24,7 +30,7 @@ inline Geometry make_geometry(const naju_scan_desc& d) {
   Geometry g;
   g.B = d.B; g.T = d.T; g.D = d.D; g.N = d.N;
   g.NS = padded_states(d.N);
-  g.TC = chunk_len_for(g.NS);
+  g.TC = chunk_len_for(d);
   g.nchunks = (d.T + g.TC - 1) / g.TC;
   g.ndt = (d.D + 127) / 128;
   g.ntiles = static_cast<int64_t>(g.nchunks) * d.B * g.ndt;
@@ -60,6 +66,7 @@ struct ScratchHeader {
   int status;            // NAJU_ST_* bits
   unsigned int ticket;   // dynamic tile counter
   int form;              // NAJU_FORM_* of the kernel that did the work (written by that kernel)
+  unsigned int done;     // CTAs that have finished
 };
 
 // Forward scratch: header | flags[ntiles] | aggP[ntiles][128] | aggS[ntiles][128][NS]
@@ -115,6 +122,7 @@ struct FwdParams {
   float* aggP;
   float* aggS;
   int B, T, D, N, nchunks, ndt, bc_dtype;
+  int inject;  // fault injection: the last CTA behaves as if a bounded wait had run out
   int64_t u_sb, u_st, fl_sb, fl_st, il_sb, il_st, bm_sb, bm_st, cm_sb, cm_st;
   int64_t u_sd;  // element stride between channels of u: 1, or > 1 for a time-contiguous u (then u_st == 1)
 };
@@ -143,6 +151,9 @@ struct BwdParams {
 };
 
 // launchers implemented in the .cu files; return a CUDA runtime error code (0 = ok)
+
+// Zeroes the header (and flags) of a scratch buffer, and the checkpoint trailer where given, in one launch.
+int launch_init(ScratchHeader* hdr, size_t bytes, int* trailer, cudaStream_t stream);
 int launch_fwd_simt(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype,
                     void* stream);
 // TMA-fed persistent tensor-core forward; returns -1000 when the problem cannot take it
@@ -151,8 +162,10 @@ int launch_fwd_tc2(const FwdParams& p, const Geometry& g, int act_dtype, int gat
 // walk-along-time tensor-core forward (two threads per channel); -1000 when it cannot take the problem
 int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
                    void* stream);
-int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype,
-                    void* dB, void* dC, float* dD, void* stream);
+int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);
+// dB, dC and dD from the partial sums; overwrites every output with NaN if the call (or its forward) failed
+int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* dB, void* dC, float* dD,
+                        bool inject, void* stream);
 // tensor-core backward; returns -1000 when the problem cannot take it
 int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
                   const int* fwd_form, void* stream);

@@ -201,6 +201,7 @@ float* mfptr(const Tensor& t) { return static_cast<float*>(mptr(t)); }
 // ------------------------------------------------------------------------------ forward / backward
 struct FwdOut {
   Tensor y, hT, pT, ckpt;
+  naju_scan_desc desc;   // of the call as it was made (states padded where the rule says so)
 };
 
 FwdOut forward(const Args& in, const Tensor& h0_in, bool want_final, bool want_decay, int flags) {
@@ -215,6 +216,7 @@ FwdOut forward(const Args& in, const Tensor& h0_in, bool want_final, bool want_d
   c10::cuda::CUDAGuard guard(a.u.device());
   const auto f32 = a.u.options().dtype(at::kFloat);
   FwdOut o;
+  o.desc = d;
   o.y = at::empty({B, T, D}, a.u.options());
   if (want_final) o.hT = at::empty({B, D, Np}, f32);
   if (want_decay) o.pT = at::empty({B, D}, f32);
@@ -421,6 +423,7 @@ PyMethodDef kFast[] = {
 
 using OptTensor = std::optional<Tensor>;
 Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+py::bytes desc_bytes(const naju_scan_desc& d) { return py::bytes(reinterpret_cast<const char*>(&d), sizeof(d)); }
 OptTensor ret(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
 
 }  // namespace
@@ -435,7 +438,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("describe", [](const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm) {
     const naju_scan_desc d = describe({u, fl, il, Bm, Cm, Tensor()}, call_flags());
-    return py::bytes(reinterpret_cast<const char*>(&d), sizeof(d));
+    return desc_bytes(d);
   });
   m.def("state_arg", [](const OptTensor& h, int64_t B, int64_t D, int64_t N, const std::string& name) {
     return ret(state_arg(opt(h), B, D, N, name.c_str()));
@@ -444,7 +447,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                       const OptTensor& h0, bool want_final, bool want_decay) {
     at::NoGradGuard ng;
     const FwdOut o = forward({u, fl, il, Bm, Cm, D}, opt(h0), want_final, want_decay, call_flags());
-    return std::make_tuple(o.y, ret(o.hT), ret(o.pT), o.ckpt);
+    return std::make_tuple(o.y, ret(o.hT), ret(o.pT), o.ckpt, desc_bytes(o.desc));
   });
   m.def("backward", [](int flags, const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm,
                        const Tensor& D, const OptTensor& h0, const Tensor& dy, const OptTensor& dhT, const Tensor& ckpt,
@@ -453,7 +456,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const BwdOut o = backward({u, fl, il, Bm, Cm, D}, opt(h0), dy, opt(dhT), ckpt, want_dh0, flags);
     return std::make_tuple(o.du, o.dfl, o.dil, o.dB, o.dC, o.dD, ret(o.dh0));
   });
-  m.def("pads_states", [](const Tensor& u, const Tensor& Bm) { return pad_to_group(u, Bm, form_flags()); });
   m.def("forms", []() { return std::make_pair(g_form_fwd.load(), g_form_bwd.load()); });
   m.def("take_guarded", []() {
     std::lock_guard<std::mutex> lock(g_guard_mutex);

@@ -101,8 +101,8 @@ _GROUP = 16
 
 def scan_forward(u, f_logit, i_logit, Bm, Cm, D_skip, h0=None, want_final=False, want_decay=False):
     """Raw forward over prepared tensors.  Returns (y, hT|None, pT|None, ckpt, desc)."""
-    y, hT, pT, ckpt = _native().forward(u, f_logit, i_logit, Bm, Cm, D_skip, h0, want_final, want_decay)
-    return y, hT, pT, ckpt, _desc(u, f_logit, i_logit, Bm, Cm)
+    y, hT, pT, ckpt, desc = _native().forward(u, f_logit, i_logit, Bm, Cm, D_skip, h0, want_final, want_decay)
+    return y, hT, pT, ckpt, _lib.ScanDesc.from_buffer_copy(desc)
 
 
 def scan_backward(d, u, f_logit, i_logit, Bm, Cm, D_skip, h0, dy, dhT, ckpt, want_dh0=False):
@@ -117,11 +117,11 @@ def scan_backward(d, u, f_logit, i_logit, Bm, Cm, D_skip, h0, dy, dhT, ckpt, wan
 # the graph at the scan (the reference's scan is a graph break: naju/README.md:99-100) and
 # NajuBlock(use_ckpt=True) (naju/mixer.py:139-141) composes.  Used while compiling; eager calls
 # go to the native autograd node (naju_b200/csrc/torch_host.cpp).
-def _ckpt_bytes_formula(B, T, D, N):
+def _ckpt_bytes_formula(B, T, D, N, act, bdt):
     """Size of the checkpoint buffer (naju_b200_ckpt_bytes) as arithmetic that also works on the
     symbolic sizes of fake tensors."""
     NS = 16 if N <= 16 else 32 if N <= 32 else 64 if N <= 64 else 128
-    TC = 64 if NS <= 32 else 32
+    TC = 64 if (N == 16 and act in (torch.bfloat16, torch.float16) and bdt == torch.bfloat16) else 32
     ntiles = ((T + TC - 1) // TC) * B * ((D + 127) // 128)
     a256 = lambda x: (x + 255) // 256 * 256
     return a256(ntiles * 128 * NS * 4) + a256(ntiles * 128 * 4) + 256
@@ -156,7 +156,7 @@ def _(u, f_logit, i_logit, Bm, Cm, D_skip, h0, want_final):
     bdt = Bm.dtype if Bm.dtype == Cm.dtype else torch.float32
     if _pads_to_group(B * T * D, T, N, u.dtype, bdt):
         N = _GROUP
-    ckpt = u.new_empty(_ckpt_bytes_formula(B, T, D, N), dtype=torch.uint8)
+    ckpt = u.new_empty(_ckpt_bytes_formula(B, T, D, N, u.dtype, bdt), dtype=torch.uint8)
     return u.new_empty((B, T, D)), hT, ckpt
 
 
