@@ -174,10 +174,6 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
   int rck = -1000;
   if (!(desc->flags & NAJU_FLAG_RECURRENT_ONLY)) {
     rck = launch_fwd_tc3(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
-    // (the ticket kernel reads u channel-contiguous only; a time-contiguous u that the walk kernel
-    // declines goes to the recurrent kernel, which transposes its tile while staging it)
-    if (rck == -1000 && p.u_sd == 1)
-      rck = launch_fwd_tc2(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
     if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;
   }
   if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);

@@ -50,16 +50,17 @@ namespace tc3 {
 using namespace tcx;
 
 constexpr int Q = 64, NS = 16, SLAB = 16, NSLAB = Q / SLAB, NSTAGE = 2;
-#ifndef NAJU_RING16
-#define NAJU_RING16 7
-#endif
 constexpr int RING_MAX = 8;                 // input-slab ring: as deep as shared memory allows (see Smem)
 constexpr int NGRP = NSLAB;                 // main-warp groups: one slab of every chunk each
 constexpr int NBUILD = 2;                   // operand-builder warps sharing a tile's work
 constexpr int NHALF = 128, NMAIN = NGRP * 128, NCARRY = 128;
 // (builder warp k reads accumulator rows 32k .. 32k+31: its index must be k modulo 4)
 constexpr int W_CARRY = NMAIN / 32, W_BUILD = W_CARRY + NCARRY / 32, W_PROD = W_BUILD + NBUILD,
-              W_MMA = W_PROD + 1, W_STORE = W_MMA + 1, NTHREADS = 32 * (W_STORE + 1);
+              W_MMA = W_PROD + 1, W_STORE = W_MMA + 1;
+// The cluster form has no store warp: its main warps write y themselves.  24 instead of 25 warps leave them 80 instead
+// of 72 registers (the register file is handed out four warps at a time), which its extra bookkeeping needs.
+template <bool CLUSTER>
+constexpr int kThreadsOf = 32 * (CLUSTER ? W_STORE : W_STORE + 1);
 static_assert(W_BUILD % 4 == 0 && NBUILD == 2, "builder warps sit on TMEM lane quarters 0 and 1");
 constexpr int AW_W1 = 0, AW_W2 = 8;
 constexpr uint32_t SBO_AW = 16 * 128, AW_BYTES = 16 * SBO_AW;  // operand rows [w1 64 | w2 64], per stage
@@ -90,33 +91,33 @@ struct Maps {
   CUtensorMap u, fl, il, bm, cm, y;
 };
 
-template <typename TG>
+template <typename TG, bool CLUSTER>
 struct Smem {
   static constexpr uint32_t slab_bytes = SLAB * kDT * (2 + 2 * sizeof(TG));  // u, f_logit, i_logit
   // Input slabs are requested as far ahead as the ring is deep, and a slab is on its way for a
   // microsecond or more: with 16-bit logits the ring holds 7 slabs (1.75 tiles), with fp32 logits
   // (larger slabs) 4.
-  static constexpr int RING = sizeof(TG) == 2 ? NAJU_RING16 : 4;
-#ifndef NAJU_NY16
-#define NAJU_NY16 1
-#endif
-  static constexpr int NY = sizeof(TG) == 2 ? NAJU_NY16 : 1;   // output staging tiles
+  static constexpr int RING = sizeof(TG) == 2 ? 7 : 4;
+  static constexpr int NY = 1;   // output staging tiles (of the form with a store warp)
   static constexpr uint32_t off_ring = 0;
   static constexpr uint32_t off_Y = off_ring + RING * slab_bytes;    // [NY][Q][128]
   // The builders' MMA addresses the 64 C rows of a stage as a 128-row operand: the 18 KB after a
   // stage's B1 buffer must be readable shared memory, so the large operand-row buffers come last.
-  static constexpr uint32_t off_B1 = off_Y + NY * Q * kDT * 2;       // [NSTAGE]
+  static constexpr uint32_t off_B1 = off_Y + (CLUSTER ? 0 : NY * Q * kDT * 2);   // [NSTAGE]
   static constexpr uint32_t off_BB = off_B1 + NSTAGE * B1_BYTES;     // [NSTAGE]
   static constexpr uint32_t off_bc = off_BB + NSTAGE * BB_BYTES;     // [2 tiles][B raw | C raw]
   static constexpr uint32_t off_AH = off_bc + 2 * 2 * BC_BYTES;
   static constexpr uint32_t off_AW = off_AH + AH_BYTES;              // [NSTAGE]
-  static constexpr uint32_t total = off_AW + NSTAGE * AW_BYTES;
+  static constexpr uint32_t off_mail = off_AW + NSTAGE * AW_BYTES;   // [4][128] quads of states | [128] decay, fp32
+  static constexpr uint32_t mail_bytes = (NS + 1) * kDT * 4;
+  static constexpr uint32_t total = off_mail + (CLUSTER ? mail_bytes : 0);
+  static_assert(total + 6144 <= 232448, "with the static arrays, within an SM's 227 KB");
   static_assert(off_B1 + (NSTAGE + 1) * B1_BYTES <= total, "the 128-row view of a stage's C rows stays inside shared memory");
 };
 
 struct Bars {
   unsigned long long full[RING_MAX], empty[RING_MAX];   // input slabs (producer <-> the group that owns the slab)
-  unsigned long long bc_full[2], bc_empty[2];   // raw B/C rows per tile parity
+  unsigned long long bc_full[2], bc_empty[2];   // raw B/C rows of a tile
   unsigned long long lprod[NSTAGE][NGRP];       // a group's retention products are published
   unsigned long long part[NSTAGE][NSLAB];       // operand-row chunks of one slab written (128 threads)
   unsigned long long g_full[NSTAGE];            // the builders' own MMA (G = C B^T) is complete
@@ -126,6 +127,8 @@ struct Bars {
   unsigned long long d1_full[NSTAGE];           // D1 complete (and the stage's shared operands read)
   unsigned long long y_staged[NSTAGE];          // main warps: outputs staged, accumulators read -> store warp, MMA issuer
   unsigned long long acc_free[NSTAGE];          // carry warps: D2 and the tile's flags read -> MMA issuer, last group
+  unsigned long long mail_full;                 // CLUSTER: the rank before has sent the carry
+  unsigned long long mail_empty;                // CLUSTER: the rank after has taken this rank's
   unsigned long long stage_free[NSTAGE];        // store warp: staging tile read by the store -> epilogue two tiles on
 };
 
@@ -134,7 +137,8 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// Two-term bf16 split of a pair: v ~= hi + lo, both truncations (see split_bf16x2); packed subtraction.
+// Two-term bf16 split of a pair: v ~= hi + lo, both truncations (the first one's error is exactly what the second
+// term carries), so it costs integer and FMA-pipe operations only; residual <= 2^-16 relative.
 __device__ __forceinline__ void split_pair(float2 v, uint32_t& hi, uint32_t& lo) {
   const uint32_t ua = __float_as_uint(v.x), ub = __float_as_uint(v.y);
   hi = __byte_perm(ua, ub, 0x7632);
@@ -184,13 +188,24 @@ __device__ __noinline__ void exact_tile_from_global(const FwdParams& p, const Ti
   write_final<NS>(p, tc, hw, Pw);
 }
 
-// Channel tiles (one batch row x 128 channels) are dealt round-robin over the grid; a CTA walks
-// each of its channel tiles along time, chunk by chunk.  `it` counts the (channel tile, chunk)
-// pairs a CTA has seen and selects the pipeline stage and barrier phases.
-template <typename TA, typename TG, bool UTM>
-__global__ void __launch_bounds__(NTHREADS, 1)
-fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
-  using SM = Smem<TG>;
+// Channel tiles (one batch row x 128 channels) are dealt round-robin over the grid's thread-block clusters and
+// walked along time, chunk by chunk.  `it` counts the (channel tile, chunk) pairs a CTA has seen and selects
+// the pipeline stage and barrier phases.
+//   CLUSTER = false  clusters of one CTA: the carry stays in the carry warps' registers and its operand row is
+//                    posted a tile ahead.
+//   CLUSTER = true   the cs CTAs of a cluster walk their channel tiles together, consecutive chunks on consecutive
+//                    ranks, so that fewer channel tiles than SMs still fill the GPU.  Everything but the carry is
+//                    independent of the chunks before; the carry goes from rank to rank through distributed shared
+//                    memory, by asynchronous stores that count as bytes on the receiver's barrier (1.2 us a hop),
+//                    and the MMAs that need it are issued after the next tile's.
+//   (Measured on the way, B=4, T=65536, D=2048, where a walk takes 2.9 us per tile on 64 of 148 SMs: tiles by
+//   ticket with a look-back through global memory 9.5 us per tile; the carry by releasing arrivals 7 us; every
+//   rank sending its aggregate to all others and folding theirs 4.9 us; this form 4.1 us on twice the SMs.)
+template <typename TA, typename TG, bool UTM, bool CLUSTER>
+__global__ void __launch_bounds__(kThreadsOf<CLUSTER>, 1)
+fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int form) {
+  using SM = Smem<TG, CLUSTER>;
+  constexpr int NTHREADS = kThreadsOf<CLUSTER>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ Bars bars;
   __shared__ int s_stage_deep[NSTAGE];
@@ -202,9 +217,27 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t sbase = smem_u32(smem);
   const int nchunks = p.nchunks, ctiles = p.B * p.ndt;
-  const int x_first = static_cast<int>(blockIdx.x), x_step = static_cast<int>(gridDim.x);
-  // (channel tile, chunk) pairs this CTA walks
-  const int ntotal = (x_first < ctiles ? (ctiles - x_first + x_step - 1) / x_step : 0) * nchunks;
+  const int cs = CLUSTER ? static_cast<int>(cluster_size()) : 1, rank = CLUSTER ? static_cast<int>(cluster_rank()) : 0;
+  const int x_first = static_cast<int>(blockIdx.x) / cs, x_step = static_cast<int>(gridDim.x) / cs;
+  // (channel tile, chunk) pairs this cluster walks, and those that are this CTA's: every cs-th
+  const int npairs = (x_first < ctiles ? (ctiles - x_first + x_step - 1) / x_step : 0) * nchunks;
+  const int ntotal = !CLUSTER ? npairs : rank < npairs ? (npairs - rank + cs - 1) / cs : 0;
+  struct Pair { int x, c; };   // CLUSTER: channel tile and chunk of a trip
+  auto settle = [&](Pair& t) {
+    while (t.c >= nchunks) {
+      t.c -= nchunks;
+      t.x += x_step;
+    }
+  };
+  auto first_pair = [&]() {
+    Pair t{x_first, rank};
+    settle(t);
+    return t;
+  };
+  auto next_pair = [&](Pair& t) {
+    t.c += cs;
+    settle(t);
+  };
 
   if (tid == 0) {
     for (int i = 0; i < RING_MAX; ++i) {
@@ -229,6 +262,8 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       mbar_init(smem_u32(&bars.stage_free[i]), 1);   // (indexed by staging tile)
     }
     mbar_init(smem_u32(&bars.h_ready), NCARRY / 32);
+    mbar_init(smem_u32(&bars.mail_full), 1);
+    mbar_init(smem_u32(&bars.mail_empty), NCARRY / 32);
     mbar_init_fence();
   }
   if (warp == 0) tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
@@ -238,12 +273,13 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
+  if constexpr (CLUSTER) cluster_sync();   // every rank's barriers are initialised before anyone arrives on them
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   pdl_wait();   // nothing above touches global memory
   if (blockIdx.x == 0 && tid == 0) {
     atomicOr(p.fwd_form, 1);  // tell the backward how the forward ran
-    p.hdr->form = NAJU_FORM_TC_WALK;
+    p.hdr->form = form;
   }
   auto timeout = [&]() { atomicOr(&p.hdr->status, NAJU_ST_MMA_TIMEOUT); };
   // u is time-contiguous: its slabs sit in shared memory as [channel][step].  (A compile-time
@@ -255,14 +291,12 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
     if (lane == 0) {
       uint32_t slab = 0;
       int it = 0;
-      for (int x = x_first; x < ctiles; x += x_step) {
-        const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
-        for (int c = 0; c < nchunks; ++c, ++it) {
+      auto load_tile = [&](int b, int d0, int c) {
           const int t0 = c * Q;
-          if (it >= 2 && !mbar_wait(smem_u32(&bars.bc_empty[it & 1]), ((it >> 1) & 1) ^ 1)) timeout();
+          if (it >= 2 && !mbar_wait(smem_u32(&bars.bc_empty[it % 2]), ((it / 2) & 1) ^ 1)) timeout();
           {
-            const uint32_t bar = smem_u32(&bars.bc_full[it & 1]);
-            const uint32_t dst = sbase + SM::off_bc + (it & 1) * 2 * BC_BYTES;
+            const uint32_t bar = smem_u32(&bars.bc_full[it % 2]);
+            const uint32_t dst = sbase + SM::off_bc + (it % 2) * 2 * BC_BYTES;
             mbar_arrive_expect_tx(bar, 2 * BC_BYTES);
             tma_load_3d(dst, &maps.bm, 0, t0, b, bar);
             tma_load_3d(dst + BC_BYTES, &maps.cm, 0, t0, b, bar);
@@ -279,6 +313,17 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
             tma_load_3d(dst + SLAB * kDT * 2, &maps.fl, d0, t0 + k * SLAB, b, bar);
             tma_load_3d(dst + SLAB * kDT * (2 + sizeof(TG)), &maps.il, d0, t0 + k * SLAB, b, bar);
           }
+      };
+      if constexpr (CLUSTER) {
+        Pair t = first_pair();
+        for (; it < ntotal; ++it, next_pair(t)) {
+          const int b = t.x / p.ndt;
+          load_tile(b, (t.x - b * p.ndt) * kDT, t.c);
+        }
+      } else {
+        for (int x = x_first; x < ctiles; x += x_step) {
+          const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
+          for (int c = 0; c < nchunks; ++c, ++it) load_tile(b, d0, c);
         }
       }
     }
@@ -291,12 +336,13 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
     for (int it = 0; it < ntotal; ++it) {
       const int st = it & 1;
       const uint32_t par = (it >> 1) & 1;
-      if (!mbar_wait(smem_u32(&bars.bc_full[st]), par)) timeout();
+      const int rb = it % 2;
+      if (!mbar_wait(smem_u32(&bars.bc_full[rb]), (it / 2) & 1)) timeout();
       // stage st: the MMAs of the tile two back must have read B1 / BB (its epilogue may still run)
       if (it >= NSTAGE && !mbar_wait(smem_u32(&bars.d1_full[st]), par ^ 1)) timeout();
       unsigned char* s_B1 = smem + SM::off_B1 + st * B1_BYTES;
       unsigned char* s_BB = smem + SM::off_BB + st * BB_BYTES;
-      const __nv_bfloat16* Braw = reinterpret_cast<const __nv_bfloat16*>(smem + SM::off_bc + st * 2 * BC_BYTES);
+      const __nv_bfloat16* Braw = reinterpret_cast<const __nv_bfloat16*>(smem + SM::off_bc + rb * 2 * BC_BYTES);
       const __nv_bfloat16* Craw = Braw + Q * NS;
       // the chunk's C and B rows in operand layout: 32 bytes per row, two 16-byte pieces
 #pragma unroll
@@ -311,7 +357,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       bar_sync<3, 32 * NBUILD>();                  // both warps: rows written, last tile's G read
       tc_fence_after();
       if (blane == 0) {
-        mbar_arrive(smem_u32(&bars.bc_empty[st]));  // the raw rows have been read
+        mbar_arrive(smem_u32(&bars.bc_empty[rb]));  // the raw rows have been read
         // G[t, s] = <C_t, B_s>: M = 128 rows of which the 64 steps are real (the rest of the A
         // operand is whatever follows the C rows in shared memory; those accumulator rows are
         // never read), N = 64, K = 16 states
@@ -389,31 +435,47 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         umma_commit(smem_u32(&bars.d2_full[st]));
         // (the accumulators of a deep-gate tile are junk and are simply never read; the carry-in MMAs
         // run for it all the same, which keeps the barrier phases aligned)
-        if (!mbar_wait(smem_u32(&bars.h_ready), it & 1)) timeout();
-        tc_fence_after();
-        umma_bf16(tst + TM_D1, dAH + off(AH_H1 * 128), dB1 + off(B1_C * 128), id64, 1u);  // D1 += (h1 + h2) . C
-        umma_bf16(tst + TM_D1, dAH + off(AH_H2 * 128), dB1 + off(B1_C * 128), id64, 1u);
-        umma_commit(smem_u32(&bars.d1_full[st]));
+        if constexpr (!CLUSTER) {
+          if (!mbar_wait(smem_u32(&bars.h_ready), it & 1)) timeout();
+          tc_fence_after();
+          umma_bf16(tst + TM_D1, dAH + off(AH_H1 * 128), dB1 + off(B1_C * 128), id64, 1u);  // D1 += (h1 + h2) . C
+          umma_bf16(tst + TM_D1, dAH + off(AH_H2 * 128), dB1 + off(B1_C * 128), id64, 1u);
+          umma_commit(smem_u32(&bars.d1_full[st]));
+        } else {
+          // the carry of this tile is still on its way: the previous tile's MMAs go out now (and after the last
+          // tile its own)
+          for (int k = it - 1; k <= it; ++k) {
+            if (k < 0 || (k == it && it + 1 < ntotal)) continue;
+            if (!mbar_wait(smem_u32(&bars.h_ready), k & 1)) timeout();
+            tc_fence_after();
+            const uint32_t d1 = tmem + (k & 1) * TM_STAGE + TM_D1;
+            const uint64_t cr = dB10 + off((k & 1) * B1_BYTES + B1_C * 128);
+            umma_bf16(d1, dAH + off(AH_H1 * 128), cr, id64, 1u);
+            umma_bf16(d1, dAH + off(AH_H2 * 128), cr, id64, 1u);
+            umma_commit(smem_u32(&bars.d1_full[k & 1]));
+          }
+        }
       }
     }
-  } else if (warp == W_STORE) {
+  } else if (!CLUSTER && warp == W_STORE) {
     // ===================================================================== store warp
     if (lane == 0) {
       int it = 0;
+      auto store_tile_out = [&](int b, int d0, int c) {
+        const int st = it & 1;
+        if (!mbar_wait(smem_u32(&bars.y_staged[st]), (it >> 1) & 1)) timeout();
+        if (!s_store_deep[st]) {
+          // the staged tile leaves by TMA (steps past T and channels past D are clipped); the stage
+          // is released once the store has read it
+          tma_store_3d(&maps.y, d0, c * Q, b, sbase + SM::off_Y + (it % SM::NY) * Q * kDT * 2);
+          tma_store_commit();
+          tma_store_wait_read();
+        }
+        mbar_arrive(smem_u32(&bars.stage_free[it % SM::NY]));
+      };
       for (int x = x_first; x < ctiles; x += x_step) {
         const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
-        for (int c = 0; c < nchunks; ++c, ++it) {
-          const int st = it & 1;
-          if (!mbar_wait(smem_u32(&bars.y_staged[st]), (it >> 1) & 1)) timeout();
-          if (!s_store_deep[st]) {
-            // the staged tile leaves by TMA (steps past T and channels past D are clipped); the stage
-            // is released once the store has read it
-            tma_store_3d(&maps.y, d0, c * Q, b, sbase + SM::off_Y + (it % SM::NY) * Q * kDT * 2);
-            tma_store_commit();
-            tma_store_wait_read();
-          }
-          mbar_arrive(smem_u32(&bars.stage_free[it % SM::NY]));
-        }
+        for (int c = 0; c < nchunks; ++c, ++it) store_tile_out(b, d0, c);
       }
       tma_store_wait_all();
     }
@@ -434,6 +496,20 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       tc_fence_before();
       mbar_arrive_warp(smem_u32(&bars.h_ready));
     };
+    [[maybe_unused]] auto set_coord = [&](TileCoord& tcd, int x, int c) {
+      tcd.per_chunk = ctiles;
+      tcd.rem = x;
+      tcd.b = x / p.ndt;
+      tcd.dt = x - tcd.b * p.ndt;
+      tcd.d0 = tcd.dt * kDT;
+      tcd.cols = min(kDT, p.D - tcd.d0);
+      tcd.d = tcd.d0 + q;
+      tcd.d_ok = tcd.d < p.D;
+      tcd.c = c;
+      tcd.tile = static_cast<int64_t>(c) * ctiles + x;
+      tcd.t0 = c * Q;
+      tcd.len = min(Q, p.T - tcd.t0);
+    };
     // state / cumulative decay entering the current chunk
     float hc[NS];
     float Pc = 1.f;
@@ -444,6 +520,97 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         hc[n] = (p.h0 != nullptr && d < p.D && n < p.N) ? p.h0[(static_cast<int64_t>(b) * p.D + d) * p.N + n] : 0.f;
       Pc = 1.f;
     };
+    if constexpr (CLUSTER) {
+      const float4* mail = reinterpret_cast<const float4*>(smem + SM::off_mail) + q;
+      const float* mail_P = reinterpret_cast<const float*>(smem + SM::off_mail + NS * kDT * 4) + q;
+      const uint32_t next = static_cast<uint32_t>(rank + 1 == cs ? 0 : rank + 1), prev = static_cast<uint32_t>(rank == 0 ? cs - 1 : rank - 1);
+      const uint32_t out_mail = map_cluster(smem_u32(mail), next), out_P = map_cluster(smem_u32(mail_P), next),
+                     out_full = map_cluster(smem_u32(&bars.mail_full), next), out_empty = map_cluster(smem_u32(&bars.mail_empty), prev);
+      if (q == 0) mbar_arrive_expect_tx(smem_u32(&bars.mail_full), SM::mail_bytes);   // the first mail may come
+      int sent = 0, got = 0;
+      // Once a wait for mail has run out nothing is armed or sent any more: the barriers' byte counts would leave
+      // their range.  (The status word turns the outputs into NaN.)
+      bool alive = true;
+      Pair t = first_pair();
+      for (int it = 0; it < ntotal; ++it, next_pair(t)) {
+        const int st = it & 1;
+        const uint32_t par = (it >> 1) & 1;
+        if (!mbar_wait(smem_u32(&bars.d2_full[st]), par)) timeout();
+        if (!mbar_wait(smem_u32(&bars.part[st][NGRP - 1]), par)) timeout();  // (the writers of s_Rend arrived here)
+        const float Rend = s_Rend[st][q];
+        const bool deep = bar_or<2, NCARRY>(!(Rend < kRMax));
+        if (q == 0) s_stage_deep[st] = deep ? 1 : 0;
+        tc_fence_after();
+        float e[NS], Ph = 1.f, Pe = 1.f;      // (hc, Ph) enters the chunk, (e, Pe) leaves it
+        if (!deep) {
+          uint32_t sr[16];
+          tmem_ld16_async(tmem + st * TM_STAGE + lane_off + TM_D2, sr);
+          tmem_ld_wait16(sr);
+          Pe = __frcp_rn(Rend);
+#pragma unroll
+          for (int n = 0; n < NS; ++n) e[n] = __uint_as_float(sr[n]);
+        }
+        // D2 and s_Rend have been read, the tile's deep flag is written: one arrival per warp
+        tc_fence_before();
+        mbar_arrive_warp(smem_u32(&bars.acc_free[st]));
+        if (t.c == 0) {
+          load_h0(t.x);
+        } else {
+          if (alive && !mbar_wait(smem_u32(&bars.mail_full), got & 1)) {
+            timeout();
+            alive = false;
+          }
+#pragma unroll
+          for (int k = 0; k < NS / 4; ++k) {
+            const float4 v = mail[k * kDT];
+            hc[4 * k] = v.x; hc[4 * k + 1] = v.y; hc[4 * k + 2] = v.z; hc[4 * k + 3] = v.w;
+          }
+          Ph = *mail_P;
+        }
+        TileCoord tcd;
+        if (deep) {
+          if (q == 0) atomicOr(p.fwd_form, 2);
+          Pe = Ph;
+#pragma unroll
+          for (int n = 0; n < NS; ++n) e[n] = hc[n];
+          set_coord(tcd, t.x, t.c);
+          exact_tile_from_global<TA, TG>(p, tcd, q, e, Pe);
+        } else {
+#pragma unroll
+          for (int n = 0; n < NS; ++n) e[n] = Pe * (hc[n] + e[n]);
+          Pe *= Ph;
+        }
+        if (t.c + 1 < nchunks) {
+          // (the rank after has taken the mail before)
+          if (alive && sent > 0 && !mbar_wait(smem_u32(&bars.mail_empty), (sent - 1) & 1)) {
+            timeout();
+            alive = false;
+          }
+          ++sent;
+          if (alive) {
+#pragma unroll
+            for (int k = 0; k < NS / 4; ++k)
+              st_async_v4(out_mail + k * kDT * 16, e[4 * k], e[4 * k + 1], e[4 * k + 2], e[4 * k + 3], out_full);
+            st_async_f32(out_P, Pe, out_full);
+          }
+        }
+        if (t.c > 0 && alive) {   // the mail has been used: the next one may come
+          ++got;
+          if (q == 0) mbar_arrive_expect_tx(smem_u32(&bars.mail_full), SM::mail_bytes);
+          mbar_arrive_cluster_relaxed_warp(out_empty);
+        }
+        // this tile's carry-in row, once the previous tile's MMAs have read theirs
+        if (it > 0 && !mbar_wait(smem_u32(&bars.d1_full[st ^ 1]), ((it - 1) >> 1) & 1)) timeout();
+        write_h_row(hc);
+        set_coord(tcd, t.x, t.c);
+        const int64_t slot = tcd.tile * kDT + q;
+        float4* dstS = reinterpret_cast<float4*>(p.ckS + slot * NS);
+#pragma unroll
+        for (int q4 = 0; q4 < NS / 4; ++q4) dstS[q4] = make_float4(e[4 * q4], e[4 * q4 + 1], e[4 * q4 + 2], e[4 * q4 + 3]);
+        p.ckP[slot] = Pe;
+        write_final<NS>(p, tcd, e, Pe);
+      }
+    } else {
     // One carry-in row (one h_ready phase) is posted per tile, one tile ahead.
     if (x_first < ctiles) {
       load_h0(x_first);
@@ -507,6 +674,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         }
       }
     }
+    }
   } else {
     // ===================================================================== main warps
     const int grp = warp >> 2;                     // owns steps [16 grp, 16 grp + 16) of every chunk
@@ -526,7 +694,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();
       // the staging tile was last used NY tiles back: that store must have read it
       const int ys = e_it % SM::NY;
-      if (e_it >= SM::NY && !mbar_wait(smem_u32(&bars.stage_free[ys]), ((e_it / SM::NY) & 1) ^ 1)) timeout();
+      if (!CLUSTER && e_it >= SM::NY && !mbar_wait(smem_u32(&bars.stage_free[ys]), ((e_it / SM::NY) & 1) ^ 1)) timeout();
       tc_fence_after();
       const bool deep = s_stage_deep[st] != 0;
       if (tid == 0) s_store_deep[st] = deep ? 1 : 0;
@@ -535,7 +703,10 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         const uint32_t tb = tmem + st * TM_STAGE + lane_off + SLAB * grp;
         tmem_ld16_async(tb + TM_D1, v);
         tmem_ld16_async(tb + TM_P, pv);
-        unsigned char* dst = smem + SM::off_Y + ys * (Q * kDT * 2) + (SLAB * grp) * (kDT * 2) + q * 2;
+        [[maybe_unused]] unsigned short* gy = reinterpret_cast<unsigned short*>(p.y) +
+            (static_cast<int64_t>(e_b) * p.T + e_t0 + SLAB * grp) * p.D + e_d0 + q;
+        [[maybe_unused]] const int nout = e_d0 + q < p.D ? e_len - SLAB * grp : 0;   // steps of this thread that exist
+        [[maybe_unused]] unsigned char* dst = smem + SM::off_Y + ys * (Q * kDT * 2) + (SLAB * grp) * (kDT * 2) + q * 2;
         const TA* gu = reinterpret_cast<const TA*>(p.u) + e_b * p.u_sb + static_cast<int64_t>(e_t0 + SLAB * grp) * p.u_st +
                        static_cast<int64_t>(e_d0 + q) * p.u_sd;
         tmem_ld_wait16(v);
@@ -561,10 +732,15 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
             o0 = __half_as_ushort(__low2half(pk));
             o1 = __half_as_ushort(__high2half(pk));
           }
-          *reinterpret_cast<unsigned short*>(dst + (2 * j2) * (kDT * 2)) = o0;
-          *reinterpret_cast<unsigned short*>(dst + (2 * j2 + 1) * (kDT * 2)) = o1;
+          if constexpr (CLUSTER) {
+            if (2 * j2 < nout) gy[static_cast<int64_t>(2 * j2) * p.D] = o0;
+            if (2 * j2 + 1 < nout) gy[static_cast<int64_t>(2 * j2 + 1) * p.D] = o1;
+          } else {
+            *reinterpret_cast<unsigned short*>(dst + (2 * j2) * (kDT * 2)) = o0;
+            *reinterpret_cast<unsigned short*>(dst + (2 * j2 + 1) * (kDT * 2)) = o1;
+          }
         }
-        fence_async_smem();
+        if constexpr (!CLUSTER) fence_async_smem();
       }
       tc_fence_before();
       mbar_arrive_warp(smem_u32(&bars.y_staged[st]));
@@ -572,12 +748,12 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
 
     // one trip more than there are tiles: trip `it` writes the operand rows of tile `it` (if there is
     // one) and then finishes tile `it - 1`
-    int x = x_first, c = 0, b = 0, d0 = 0;
+    int x = CLUSTER ? first_pair().x : x_first, c = CLUSTER ? first_pair().c : 0, b = 0, d0 = 0;
     float Dv = 0.f;
 #pragma unroll 1
     for (int it = 0; it <= ntotal; ++it) {
       if (it < ntotal) {
-        if (c == 0) {
+        if (CLUSTER ? (it == 0 || c < cs) : c == 0) {   // a new channel tile
           b = x / p.ndt;
           d0 = (x - b * p.ndt) * kDT;
           Dv = (d0 + q < p.D) ? __ldg(p.Dskip + d0 + q) : 0.f;
@@ -677,13 +853,19 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       if (it > 0) epilogue();
       if (it < ntotal) {
         e_b = b; e_d0 = d0; e_t0 = c * Q; e_len = min(Q, p.T - c * Q); e_it = it; e_Dv = Dv;
-        if (++c == nchunks) {
+        if constexpr (CLUSTER) {
+          Pair t{x, c};
+          next_pair(t);
+          x = t.x;
+          c = t.c;
+        } else if (++c == nchunks) {
           c = 0;
           x += x_step;
         }
       }
     }
   }
+  if constexpr (CLUSTER) cluster_sync();   // no rank leaves while another may still write to its mailbox
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
   finish_forward<TA>(p);
@@ -694,31 +876,85 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
 // ------------------------------------------------------------------------------ host side
 namespace {
 
+// Clusters of `cs` CTAs that fit on the current device at once (cached per device; a racing first call asks twice).
+template <typename K>
+int max_clusters(K* kern, size_t smem, int cs, std::atomic<int> (&cache)[64]) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) dev = 0;
+  int n = cache[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cs));
+  cfg.blockDim = dim3(tc3::kThreadsOf<true>);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(cs);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = 1;
+  }
+  cache[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+#ifndef NAJU_C2
+#define NAJU_C2 41
+#define NAJU_C4 48
+#define NAJU_CSMAX 4
+#endif
+// Trips of the busiest CTA with clusters of `cs`, and how many clusters there are.
+int64_t trips_of(const Geometry& g, int cs, int64_t fit, int64_t& clusters) {
+  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
+  clusters = std::min<int64_t>(ctiles, fit);
+  return ((ctiles + clusters - 1) / clusters * g.nchunks + cs - 1) / cs;
+}
+
 template <typename TA, typename TG, bool UTM>
-int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, cudaStream_t st) {
-  const size_t smem = tc3::Smem<TG>::total;
-  auto kern = tc3::fwd_tc3_kernel<TA, TG, UTM>;
-  static std::atomic<unsigned long long> allowed{0};
-  int rc = allow_smem(kern, smem, allowed);
+int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, int form, cudaStream_t st) {
+  auto walk = tc3::fwd_tc3_kernel<TA, TG, UTM, false>;
+  auto shared = tc3::fwd_tc3_kernel<TA, TG, UTM, true>;
+  constexpr size_t smem1 = tc3::Smem<TG, false>::total, smemc = tc3::Smem<TG, true>::total;
+  static std::atomic<unsigned long long> ok1{0}, okc{0};
+  static std::atomic<int> fit[3][64];
+  int rc = allow_smem(walk, smem1, ok1);
+  if (rc == 0) rc = allow_smem(shared, smemc, okc);
   if (rc == 0) rc = launch_init(p.hdr, 256, p.fwd_form, st);
   if (rc != 0) return rc;
-  // one persistent CTA per SM; channel tiles are dealt round-robin
-  const int64_t grid = std::min<int64_t>(static_cast<int64_t>(g.B) * g.ndt, tmah::sm_count());
-  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(tc3::NTHREADS), smem, st, p, maps);
+  // The cluster size with the shortest busiest CTA.  With fewer channel tiles than SMs more CTAs per channel tile win
+  // until the carry sets the pace; a tile takes 2.9 us in a cluster of one, 4.1 us in one of two, 4.8 us in
+  // one of four (1.2 us for each hop of the carry), and clusters of eight (9.6 us) do not pay.
+  int best = 1;
+  int64_t clusters, n, cost = trips_of(g, 1, tmah::sm_count(), clusters) * 29;
+  for (int k = 0, cs = 2; cs <= NAJU_CSMAX; ++k, cs *= 2) {
+    const int64_t c = trips_of(g, cs, max_clusters(shared, smemc, cs, fit[k]), n) * (cs == 2 ? NAJU_C2 : NAJU_C4);
+    if (c < cost) {
+      cost = c;
+      best = cs;
+      clusters = n;
+    }
+  }
+  const dim3 grid(static_cast<unsigned>(clusters * best)), block(best > 1 ? tc3::kThreadsOf<true> : tc3::kThreadsOf<false>);
+  return best == 1 ? launch_pdl(walk, grid, block, smem1, st, p, maps, form)
+                   : launch_cluster(shared, grid, block, smemc, best, st, p, maps, form);
 }
 
 }  // namespace
 
-// Walk-along-time forward; returns -1000 if this problem cannot take it (too few channel tiles to
-// fill the GPU, or shapes / strides TMA cannot describe): the caller then uses another kernel.
+// Tensor-core forward; returns -1000 if this problem cannot take it (shapes / strides TMA cannot describe, or a
+// small problem that the recurrent kernel does better): the caller then uses another kernel.
 int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int bc, void* stream) {
   const bool act16 = act == NAJU_BF16 || act == NAJU_F16;
   if (!(g.N == tc3::NS && g.TC == tc3::Q && act16 && bc == NAJU_BF16 && (gate == act || gate == NAJU_F32)))
     return -1000;
   if (g.ntiles >= (1LL << 31)) return -1000;
-  // (with fewer than about a quarter of the SMs busy the ticket-mode kernel, which spreads over time as
-  // well, is the faster one)
-  if (static_cast<int64_t>(g.B) * g.ndt * 4 < tmah::sm_count() || g.nchunks < 4) return -1000;
+  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt, sms = tmah::sm_count();
+  // A time-contiguous u of a problem with fewer tiles than SMs stays with the recurrent kernel.
+  if (p.u_sd > 1 && g.ntiles < sms) return -1000;
+  const int form = (ctiles * 4 >= sms && g.nchunks >= 4) ? NAJU_FORM_TC_WALK : NAJU_FORM_TC_TICKET;
   tc3::Maps maps;
   const bool ok =
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, tc3::SLAB, kDT)
@@ -730,17 +966,16 @@ int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int
       tmah::make_map(&maps.y, p.y, act, g.B, g.T, g.D, static_cast<int64_t>(g.T) * g.D, g.D, kDT, tc3::Q);
   if (!ok) return -1000;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (p.u_sd > 1) {
-    if (act == NAJU_BF16 && gate == NAJU_BF16) return launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, st);
-    if (act == NAJU_BF16 && gate == NAJU_F32) return launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, st);
-    if (act == NAJU_F16 && gate == NAJU_F16) return launch_tc3_t<__half, __half, true>(p, g, maps, st);
-    if (act == NAJU_F16 && gate == NAJU_F32) return launch_tc3_t<__half, float, true>(p, g, maps, st);
-  }
-  if (act == NAJU_BF16 && gate == NAJU_BF16) return launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, st);
-  if (act == NAJU_BF16 && gate == NAJU_F32) return launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, st);
-  if (act == NAJU_F16 && gate == NAJU_F16) return launch_tc3_t<__half, __half, false>(p, g, maps, st);
-  if (act == NAJU_F16 && gate == NAJU_F32) return launch_tc3_t<__half, float, false>(p, g, maps, st);
-  return -1000;
+  const bool utm = p.u_sd > 1;
+  if (act == NAJU_BF16 && gate == NAJU_BF16)
+    return utm ? launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, form, st)
+               : launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, form, st);
+  if (act == NAJU_BF16 && gate == NAJU_F32)
+    return utm ? launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, form, st)
+               : launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, form, st);
+  if (act == NAJU_F16 && gate == NAJU_F16)
+    return utm ? launch_tc3_t<__half, __half, true>(p, g, maps, form, st) : launch_tc3_t<__half, __half, false>(p, g, maps, form, st);
+  return utm ? launch_tc3_t<__half, float, true>(p, g, maps, form, st) : launch_tc3_t<__half, float, false>(p, g, maps, form, st);
 }
 
 }  // namespace naju

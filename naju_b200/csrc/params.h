@@ -156,10 +156,7 @@ struct BwdParams {
 int launch_init(ScratchHeader* hdr, size_t bytes, int* trailer, cudaStream_t stream);
 int launch_fwd_simt(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype,
                     void* stream);
-// TMA-fed persistent tensor-core forward; returns -1000 when the problem cannot take it
-int launch_fwd_tc2(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
-                   void* stream);
-// walk-along-time tensor-core forward (two threads per channel); -1000 when it cannot take the problem
+// tensor-core forward; returns -1000 when it cannot take the problem
 int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
                    void* stream);
 int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);

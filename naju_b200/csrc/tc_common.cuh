@@ -154,6 +154,36 @@ __device__ __forceinline__ bool mbar_try_once(uint32_t mbar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same without parking: a look.
+__device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(mbar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// One try that parks for at most about `ns` nanoseconds.
+__device__ __forceinline__ bool mbar_try_for(uint32_t mbar, uint32_t parity, uint32_t ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(mbar), "r"(parity), "r"(ns)
+      : "memory");
+  return ok != 0;
+}
+
 // (kept out of line: the retry loop is cold code, and the kernels' hot loops must stay small
 // enough for the instruction caches)
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity) {
@@ -183,6 +213,47 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parit
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   if (mbar_try_once(mbar, parity)) return true;
   return mbar_wait_slow(mbar, parity);
+}
+
+// ---- thread-block clusters: a neighbour CTA's shared memory
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// the shared::cluster address of a location of this CTA's layout in the CTA of rank `rank`
+__device__ __forceinline__ uint32_t map_cluster(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+// Asynchronous stores to another CTA's shared memory that count as received bytes on one of its barriers: the data
+// is visible to whoever sees that phase complete.  No fence is involved (a releasing arrival at cluster scope
+// would first wait for this thread's global stores: 3.5 us instead of 1 us per hop).
+__device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, float c, float d, uint32_t mbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(a),
+               "f"(b), "f"(c), "f"(d), "r"(mbar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t mbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v), "r"(mbar) : "memory");
+}
+// One arrival for the whole warp on a barrier of another CTA of the cluster, ordered after nothing: it says that
+// values this warp has read into registers, and used, may be overwritten.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed_warp(uint32_t addr) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0)
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// every thread of every CTA of the cluster
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // (Waits that sleep between polls -- 32 ns to 1 us, for the roles with slack -- were measured in both
@@ -249,18 +320,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {  // lo -> 
 __device__ __forceinline__ float bf16lo_f32(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float bf16hi_f32(uint32_t p) { return __uint_as_float(p & 0xFFFF0000u); }
 
-// Two-term bf16 split of a pair of floats: v ~= hi + lo with 16 mantissa bits kept.  Both terms
-// are truncations (the first one's error is exactly what the second term carries), so the split
-// costs only integer and FMA-pipe operations: the conversion instructions share the SFU pipe with
-// ex2/rcp, which is the busiest pipe of the gate warps.  Residual <= 2^-16 relative.
-__device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
-  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-  const uint32_t ha = ua & 0xFFFF0000u, hb = ub & 0xFFFF0000u;
-  hi = __byte_perm(ha, hb, 0x7632);  // {hb[31:16], ha[31:16]}
-  const uint32_t la = __float_as_uint(a - __uint_as_float(ha)), lb = __float_as_uint(b - __uint_as_float(hb));
-  lo = __byte_perm(la, lb, 0x7632);
-}
-
 // shared-memory element -> fp32 without the conversion unit where the format allows it
 __device__ __forceinline__ float ld_as_f32(const __nv_bfloat16* p, int i) {
   return __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const unsigned short*>(p)[i]) << 16);
@@ -274,16 +333,6 @@ __device__ __forceinline__ float2 ld_pair_as_f32(const __nv_bfloat16* p) {
 }
 __device__ __forceinline__ float2 ld_pair_as_f32(const __half* p) {
   return __half22float2(*reinterpret_cast<const __half2*>(p));
-}
-
-// D(16x8, fp32) += A(16x16, bf16, row) . B(16x8, bf16, col)
-__device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                                 uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // byte offset of bf16 element (row, k) in a K-major no-swizzle operand (8 elements per chunk)
