@@ -229,8 +229,9 @@ int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     // The tensor-core backward stands down on the device unless the forward of these inputs ran
     // chunked and met no deep-gate tile; the recurrent backward launched after it does the
     // opposite, so exactly one of the two does the work and no host round trip is needed.
-    const int rc2 = launch_bwd_tc(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, p.fwd_form, stream);
-    if (rc2 == 0) p.tc_launched = 1;
+    int cs = 0;
+    const int rc2 = launch_bwd_tc(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, p.fwd_form, cs, stream);
+    if (rc2 == 0) p.tc_launched = cs;
     else if (rc2 != -1000) return rc2;
   }
   rc = launch_bwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);

@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* 
     store_dyn(out, p.bc_dtype, i, bad ? nan : s);
     return;
   }
-  // the tensor-core backward writes four partial rows per batch row, the recurrent one per chunk
+  // the tensor-core backward writes four partial rows per rank and batch row, the recurrent one per chunk
   const int rows = (dd_rows_tc > 0 && (form & 3) == 1) ? dd_rows_tc : dd_rows;
   const int dl = threadIdx.x & 31, rl = threadIdx.x >> 5, d = (blk - 2 * nbc) * 32 + dl, ld = p.ndt * kDT;
   float s = 0.f;
@@ -429,7 +429,7 @@ int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act, int gate
                       static_cast<unsigned long long>(ntd) * dtype_size(gate),
                       p.dh0 ? static_cast<unsigned long long>(g.B) * g.D * g.N * 4 : 0ull}};
   return launch_pdl(finalize_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), p, dB,
-                    dC, dD, g.NS, static_cast<int>(nbc), g.nchunks * g.B, p.tc_launched ? 4 * g.B : 0, inject ? 1 : 0, list);
+                    dC, dD, g.NS, static_cast<int>(nbc), g.nchunks * g.B, 4 * p.tc_launched * g.B, inject ? 1 : 0, list);
 }
 
 template <typename TA, typename TG, int NS, int NH>

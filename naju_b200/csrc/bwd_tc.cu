@@ -168,13 +168,24 @@ struct Bars {
   unsigned long long ops_full[2];      // builders: C | g1 | g2 and B rows of a tile built
   unsigned long long g_full[2];        // the builders' own MMA is complete
   unsigned long long d1_full, d4_full; // MMA rounds complete: first (Yt, gt, dL), cross-channel
+  unsigned long long d0_full;          // CLUSTER: dL (and what else does not need the adjoint) complete
+  unsigned long long mail_full;        // CLUSTER: the rank before has sent the adjoint, into this CTA's lt rows
+  unsigned long long cts;              // CLUSTER: the rank after has its lt rows clear for this rank's mail
   unsigned long long d5_full[2];       // second round (and with it every read of the tile's BG / BB)
   unsigned long long m2_full;          // builders: M2 operand written; carry warps: U / V read
   unsigned long long x_free;           // carry warps: second-round results read
   unsigned long long acc_free;         // main + carry warps: Yt, gt, dL, coefficients read
 };
 
-template <typename TA, typename TG, bool UTM>
+// Channel tiles go round-robin over the grid's thread-block clusters.
+//   CLUSTER = false  clusters of one CTA: the adjoint stays in the carry warps' registers.
+//   CLUSTER = true   the cs CTAs of a cluster walk their channel tiles together, consecutive chunks (in reverse time) on
+//                    consecutive ranks, so that fewer channel tiles than SMs still fill the GPU.  The states come
+//                    from the checkpoints; only the adjoint goes from rank to rank, as soon as the chunk's dL is complete,
+//                    by asynchronous stores straight into the receiver's lt rows (which the receiver rescales in
+//                    place: no shared memory is left for a mailbox), once the receiver has said that the MMAs reading
+//                    its previous rows are done.
+template <typename TA, typename TG, bool UTM, bool CLUSTER>
 __global__ void __launch_bounds__(NTHREADS, 1)
 bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* __restrict__ fwd_form) {
   using Smem = SmemT<TG>;
@@ -195,9 +206,27 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
   // channel tiles (one batch row x 128 channels) are dealt round-robin over the grid; `it` counts
   // the (channel tile, chunk) pairs a CTA has seen and selects the barrier phases
   const int per_chunk = p.B * p.ndt;
-  const int x_first = static_cast<int>(blockIdx.x), x_step = static_cast<int>(gridDim.x);
+  const int cs = CLUSTER ? static_cast<int>(cluster_size()) : 1, rank = CLUSTER ? static_cast<int>(cluster_rank()) : 0;
+  const int x_first = static_cast<int>(blockIdx.x) / cs, x_step = static_cast<int>(gridDim.x) / cs;
   const int nchunks = p.nchunks;
-  const int ntotal = (x_first < per_chunk ? (per_chunk - x_first + x_step - 1) / x_step : 0) * nchunks;
+  const int npairs = (x_first < per_chunk ? (per_chunk - x_first + x_step - 1) / x_step : 0) * nchunks;
+  const int ntotal = !CLUSTER ? npairs : rank < npairs ? (npairs - rank + cs - 1) / cs : 0;
+  struct Pair { int x, ci; };   // CLUSTER: channel tile and chunk (counted from the end) of a trip
+  auto settle = [&](Pair& t) {
+    while (t.ci >= nchunks) {
+      t.ci -= nchunks;
+      t.x += x_step;
+    }
+  };
+  auto first_pair = [&]() {
+    Pair t{x_first, rank};
+    settle(t);
+    return t;
+  };
+  auto next_pair = [&](Pair& t) {
+    t.ci += cs;
+    settle(t);
+  };
 
   if (tid == 0) {
     if (blockIdx.x == 0) p.hdr->form = NAJU_FORM_TC_WALK;
@@ -223,6 +252,9 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
     mbar_init(smem_u32(&bars.lt_full), NCARRY / 32);
     mbar_init(smem_u32(&bars.d1_full), 1);
     mbar_init(smem_u32(&bars.d4_full), 1);
+    mbar_init(smem_u32(&bars.d0_full), 1);
+    mbar_init(smem_u32(&bars.mail_full), 1);
+    mbar_init(smem_u32(&bars.cts), NCARRY / 32);
     mbar_init(smem_u32(&bars.m2_full), NCARRY / 32 + NBUILD);
     mbar_init(smem_u32(&bars.x_free), NCARRY / 32);
     mbar_init(smem_u32(&bars.acc_free), NMAIN / 32 + NCARRY / 32);
@@ -238,6 +270,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
+  if constexpr (CLUSTER) cluster_sync();   // every rank's barriers are initialised before anyone arrives on them
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   auto timeout = [&]() { atomicOr(&p.hdr->status, NAJU_ST_MMA_TIMEOUT); };
@@ -250,9 +283,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
     if (lane == 0) {
       uint32_t slab = 0;
       int it = 0;
-      for (int x = x_first; x < per_chunk; x += x_step) {
-        const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
-        for (int ci = 0; ci < nchunks; ++ci, ++it) {
+      auto load_tile = [&](int b, int d0, int ci) {
           const int c = nchunks - 1 - ci, t0 = c * Q, par = it & 1;
           if (it >= 2 && !mbar_wait(smem_u32(&bars.bc_empty[par]), ((it >> 1) & 1) ^ 1)) timeout();
           {
@@ -275,6 +306,17 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
             tma_load_3d(dst + Smem::off_sil, &maps.il, d0, t0 + k * SLAB, b, bar);
             tma_load_3d(dst + Smem::off_sdy, &maps.dy, d0, t0 + k * SLAB, b, bar);
           }
+      };
+      if constexpr (CLUSTER) {
+        Pair t = first_pair();
+        for (; it < ntotal; ++it, next_pair(t)) {
+          const int b = t.x / p.ndt;
+          load_tile(b, (t.x - b * p.ndt) * kDT, t.ci);
+        }
+      } else {
+        for (int x = x_first; x < per_chunk; x += x_step) {
+          const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
+          for (int ci = 0; ci < nchunks; ++ci, ++it) load_tile(b, d0, ci);
         }
       }
     }
@@ -433,6 +475,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
           umma_bf16(tmem + TM_G, dRk + off((R_A1 + 2 * ks) * 128), g2t, iKM64, 1u);
           umma_bf16(tmem + TM_DL, dRk + off((R_A2 + 2 * ks) * 128), cg1, iKM80, 1u);
         }
+        if constexpr (CLUSTER) umma_commit(smem_u32(&bars.d0_full));   // the adjoint can go on to the next rank
         // gt += (l1 + l2).B   (K = n): the only MMAs that need the whole chunk's retention product
         if (!mbar_wait(smem_u32(&bars.lt_full), par)) timeout();
         tc_fence_after();
@@ -525,6 +568,147 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
       for (int n = 0; n < NS; ++n) seed = fmaf(lam[n], xe[n], seed);
       fetch_state(xx, nchunks - 2, hv);
     };
+    // dC / dB partial rows: carry part (UV) + intra-chunk part from the second round, one row per step of the chunk
+    auto put_partials = [&](const float (&UV)[NS], int b, int dt, int t0) {
+      uint32_t xr[16];
+      tmem_ld16_async(trow + (cid < 64 ? TM_DCI : TM_DBI), xr);
+      tmem_ld_wait16(xr);
+      const int tt = cid & 63;
+      if (tt < min(Q, p.T - t0)) {
+        float* dst = (cid < 64 ? p.dCpart : p.dBpart) + ((static_cast<int64_t>(b) * p.T + t0 + tt) * p.ndt + dt) * NS;
+#pragma unroll
+        for (int q4 = 0; q4 < NS / 4; ++q4)
+          reinterpret_cast<float4*>(dst)[q4] =
+              make_float4(UV[4 * q4] + __uint_as_float(xr[4 * q4]), UV[4 * q4 + 1] + __uint_as_float(xr[4 * q4 + 1]),
+                          UV[4 * q4 + 2] + __uint_as_float(xr[4 * q4 + 2]), UV[4 * q4 + 3] + __uint_as_float(xr[4 * q4 + 3]));
+      }
+    };
+    if constexpr (CLUSTER) {
+      const uint32_t next = static_cast<uint32_t>(rank + 1 == cs ? 0 : rank + 1), prev = static_cast<uint32_t>(rank == 0 ? cs - 1 : rank - 1);
+      const uint32_t out_row = map_cluster(smem_u32(my_row), next), out_full = map_cluster(smem_u32(&bars.mail_full), next),
+                     out_cts = map_cluster(smem_u32(&bars.cts), prev);
+      constexpr int mail_chunk[4] = {R_L1, R_L1 + 1, R_L2, R_L2 + 1};   // 16 bytes of a channel's mail in each
+      int sent = 0, got = 0;
+      // Once a wait for mail has run out nothing is armed or sent any more: the barriers' byte counts would leave
+      // their range.  (The status word turns the outputs into NaN.)
+      bool alive = true;
+      auto clear_to_send = [&]() {   // this CTA's lt rows may be overwritten by the next mail
+        if (!alive) return;
+        if (cid == 0) mbar_arrive_expect_tx(smem_u32(&bars.mail_full), NCARRY * NS * 4);
+        mbar_arrive_cluster_relaxed_warp(out_cts);
+      };
+      auto post_h = [&]() {
+        write_split_rows(hv, R_H1, R_H2);
+        fence_async_smem();
+        mbar_arrive_warp(smem_u32(&bars.h_full));
+      };
+      Pair t = first_pair();
+      if (ntotal > 0) {
+        fetch_state(t.x, nchunks - 2 - t.ci, hv);
+        post_h();
+        if (t.ci > 0) clear_to_send();
+      }
+#pragma unroll 1
+      for (int it = 0; it < ntotal; ++it) {
+        const int c = nchunks - 1 - t.ci, t0 = c * Q;
+        const uint32_t par = it & 1, st = it % Smem::NBG, par2 = (it / Smem::NBG) & 1;
+        float xe[NS];
+        fetch_state(t.x, c, xe);                     // state at the end of the chunk
+        if (!mbar_wait(smem_u32(&bars.rq_ready), par)) timeout();
+        const float Rend = s_Rend[cid];
+        if (!(Rend < kRMax)) atomicOr(&p.hdr->status, NAJU_ST_DEEP_TILE);  // never expected here
+        const float PQ = __frcp_rn(Rend);
+        b = t.x / p.ndt;
+        dt = t.x - b * p.ndt;
+        d = dt * kDT + cid;
+        if (t.ci == 0) {
+#pragma unroll
+          for (int n = 0; n < NS; ++n)
+            lam[n] = (p.dhT != nullptr && d < p.D && n < p.N) ? p.dhT[(static_cast<int64_t>(b) * p.D + d) * p.N + n] : 0.f;
+        } else {
+          if (alive && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.mail_full), got & 1))) {
+            timeout();
+            alive = false;
+          }
+          ++got;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(my_row + mail_chunk[k] * 128);
+            lam[4 * k] = v.x; lam[4 * k + 1] = v.y; lam[4 * k + 2] = v.z; lam[4 * k + 3] = v.w;
+          }
+        }
+        // adjoint leaving the chunk, to the next rank (or, from chunk 0, the gradient of h0)
+        auto pass_on = [&]() {
+          if (!mbar_wait(smem_u32(&bars.d0_full), par)) timeout();
+          tc_fence_after();
+          uint32_t dl[16];
+          tmem_ld16_async(trow + TM_DL, dl);
+          tmem_ld_wait16(dl);
+          tc_fence_before();
+          mbar_arrive_warp(smem_u32(&bars.acc_free));
+          if (c > 0) {
+            if (alive && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.cts), sent & 1))) {
+              timeout();
+              alive = false;
+            }
+            ++sent;
+            if (alive) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                st_async_v4(out_row + mail_chunk[k] * 128, fmaf(PQ, lam[4 * k], __uint_as_float(dl[4 * k])),
+                            fmaf(PQ, lam[4 * k + 1], __uint_as_float(dl[4 * k + 1])), fmaf(PQ, lam[4 * k + 2], __uint_as_float(dl[4 * k + 2])),
+                            fmaf(PQ, lam[4 * k + 3], __uint_as_float(dl[4 * k + 3])), out_full);
+            }
+          } else if (p.dh0 != nullptr && d < p.D) {
+            float* o = p.dh0 + (static_cast<int64_t>(b) * p.D + d) * p.N;
+#pragma unroll
+            for (int n = 0; n < NS; ++n)
+              if (n < p.N) o[n] = fmaf(PQ, lam[n], __uint_as_float(dl[n]));
+          }
+        };
+        const bool first = __all_sync(0xffffffffu, mbar_test(smem_u32(&bars.d0_full), par));   // dL is there already: the next rank comes first
+        if (first) pass_on();
+        {
+          float lt[NS];
+#pragma unroll
+          for (int n = 0; n < NS; ++n) lt[n] = PQ * lam[n];
+          write_split_rows(lt, R_L1, R_L2);
+        }
+        fence_async_smem();
+        mbar_arrive_warp(smem_u32(&bars.lt_full));
+        seed = 0.f;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) seed = fmaf(lam[n], xe[n], seed);
+        s_seed[it & 1][cid] = seed;
+        mbar_arrive_warp(smem_u32(&bars.seed_ready[it & 1]));
+        if (!first) pass_on();
+        const bool more = it + 1 < ntotal;
+        next_pair(t);
+        if (more) fetch_state(t.x, nchunks - 2 - t.ci, hv);
+        // ---- cross-channel block complete, and with it every MMA that reads the channel rows
+        if (!mbar_wait(smem_u32(&bars.d4_full), par)) timeout();
+        tc_fence_after();
+        if (more) {
+          if (t.ci > 0) clear_to_send();
+          post_h();
+        }
+        float UV[NS];
+        {
+          uint32_t xr[16];
+          tmem_ld16_async(trow + TM_X + (cid < 64 ? 64 : 80), xr);  // U[t,:] or V[s,:]
+          tmem_ld_wait16(xr);
+#pragma unroll
+          for (int n = 0; n < NS; ++n) UV[n] = __uint_as_float(xr[n]);
+        }
+        tc_fence_before();
+        mbar_arrive_warp(smem_u32(&bars.m2_full));
+        if (!mbar_wait(smem_u32(&bars.d5_full[st]), par2)) timeout();
+        tc_fence_after();
+        put_partials(UV, b, dt, t0);
+        tc_fence_before();
+        mbar_arrive_warp(smem_u32(&bars.x_free));
+      }
+    } else {
     // h rows and the seed of the r recurrence of tile `jt` (from hv / seed)
     auto post_tile = [&](int jt) {
       write_split_rows(hv, R_H1, R_H2);
@@ -629,6 +813,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
         x += x_step;
       }
     }
+    }
   } else {
     // ===================================================================== main warps
     const int grp = warp >> 2;                     // owns steps [16 grp, 16 grp + 16) of every chunk
@@ -638,13 +823,14 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
     const float2 kk = make_float2(kNegLog2e, kNegLog2e), one2 = make_float2(1.f, 1.f);
     float dDsum = 0.f;
     int it = 0;
-    for (int x = x_first; x < per_chunk; x += x_step) {
+    for (int x = CLUSTER ? first_pair().x : x_first, ci0 = CLUSTER ? first_pair().ci : 0; CLUSTER ? it < ntotal : x < per_chunk; x += x_step) {
       const int b = x / p.ndt, dt = x - b * p.ndt, d0 = dt * kDT, d = d0 + cid;
       const bool d_ok = d < p.D;
       const float Dv = d_ok ? __ldg(p.Dskip + d) : 0.f;
       dDsum = 0.f;
+      int ci = ci0;
 #pragma unroll 1
-      for (int ci = 0; ci < nchunks; ++ci, ++it) {
+      for (; ci < nchunks; ci += cs, ++it) {
         const int c = nchunks - 1 - ci, t0 = c * Q, len = min(Q, p.T - t0);
         const uint32_t par = it & 1;
         const int nvalid = len - SLAB * grp;       // real steps among this thread's 16
@@ -839,10 +1025,12 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
         tc_fence_before();
         mbar_arrive_warp(smem_u32(&bars.acc_free));      // Yt, gt and the coefficients have been read
       }
-      // channel tile done: D_skip partials (one row per group and batch row)
-      p.dDpart[(static_cast<int64_t>(grp) * p.B + b) * (p.ndt * kDT) + d0 + cid] = dDsum;
+      // channel tile done: D_skip partials (one row per rank, group and batch row)
+      p.dDpart[(static_cast<int64_t>(rank * NGRP + grp) * p.B + b) * (p.ndt * kDT) + d0 + cid] = dDsum;
+      ci0 = CLUSTER ? ci - nchunks : 0;
     }
   }
+  if constexpr (CLUSTER) cluster_sync();   // no rank leaves while another may still write to its rows
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
@@ -854,27 +1042,47 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
 // The kernel itself stands down unless *fwd_form says the forward ran chunked without deep tiles.
 namespace {
 template <typename TA, typename TG, bool UTM>
-int launch_bwd_tc_t(const BwdParams& p, const tcb::Maps& maps, const int* fwd_form, int64_t ctiles, cudaStream_t st) {
+int launch_bwd_tc_t(const BwdParams& p, const Geometry& g, const tcb::Maps& maps, const int* fwd_form, int& cs_used, cudaStream_t st) {
   constexpr size_t smem = tcb::SmemT<TG>::total;
-  auto kern = tcb::bwd_tc_kernel<TA, TG, UTM>;
-  static std::atomic<unsigned long long> allowed{0};
-  const int rc = allow_smem(kern, smem, allowed);
+  auto walk = tcb::bwd_tc_kernel<TA, TG, UTM, false>;
+  auto shared = tcb::bwd_tc_kernel<TA, TG, UTM, true>;
+  static std::atomic<unsigned long long> ok1{0}, okc{0};
+  static std::atomic<int> fit[2][64];
+  int rc = allow_smem(walk, smem, ok1);
+  if (rc == 0) rc = allow_smem(shared, smem, okc);
   if (rc != 0) return rc;
-  const int64_t grid = std::min<int64_t>(ctiles, tmah::sm_count());
-  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(tcb::NTHREADS), smem, st, p, maps, fwd_form);
+  // The cluster size with the shortest busiest CTA, in units of 0.1 us: a tile takes 5.7 us in a cluster of one and
+  // somewhat longer when ranks wait for each other's adjoint.
+#ifndef NAJU_B2
+#define NAJU_B2 62
+#define NAJU_B4 72
+#endif
+  int best = 1;
+  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 57;
+  for (int k = 0, cs = 2; cs <= 4 && cs <= g.nchunks; ++k, cs *= 2) {
+    const int64_t fits = tmah::max_clusters(shared, tcb::NTHREADS, smem, cs, fit[k]);
+    const int64_t c = tmah::cluster_trips(g, cs, fits, n) * (cs == 2 ? NAJU_B2 : NAJU_B4);
+    if (c < cost) {
+      cost = c;
+      best = cs;
+      clusters = n;
+    }
+  }
+  // The exact recurrent backward spreads over time too: it takes about 0.3 us per tile of 64 steps x 128 channels on a
+  // full GPU, and 15 us at least.  (Every tile here has its own carry to wait for, 10 us in all.)
+  if (cost + 100 > 150 + 3 * g.ntiles) return -1000;
+  cs_used = best;
+  const dim3 grid(static_cast<unsigned>(clusters * best)), block(tcb::NTHREADS);
+  return best == 1 ? launch_pdl(walk, grid, block, smem, st, p, maps, fwd_form)
+                   : launch_cluster(shared, grid, block, smem, best, st, p, maps, fwd_form);
 }
 }  // namespace
 
-int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act, int gate, int bc, const int* fwd_form,
+int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act, int gate, int bc, const int* fwd_form, int& cs_used,
                   void* stream) {
   if (!(g.N == tcb::NS && g.TC == tcb::Q && act == NAJU_BF16 && (gate == NAJU_BF16 || gate == NAJU_F32) &&
         bc == NAJU_BF16))
     return -1000;
-  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
-  // One persistent CTA per SM walks whole channel tiles: with fewer than about a quarter of the SMs
-  // busy the exact recurrent backward (which spreads over time as well) is the faster one
-  // (measured at D=2048, T=65536: 48 channel tiles 22 against 15 M tokens/s, 32 tiles even).
-  if (!(ctiles * 4 >= tmah::sm_count() && g.nchunks >= 4)) return -1000;
   tcb::Maps maps = {};
   const bool ok =
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, tcb::SLAB, kDT)
@@ -887,10 +1095,10 @@ int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act, int gate, int 
   if (!ok) return -1000;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (p.u_sd > 1)
-    return gate == NAJU_F32 ? launch_bwd_tc_t<__nv_bfloat16, float, true>(p, maps, fwd_form, ctiles, st)
-                            : launch_bwd_tc_t<__nv_bfloat16, __nv_bfloat16, true>(p, maps, fwd_form, ctiles, st);
-  return gate == NAJU_F32 ? launch_bwd_tc_t<__nv_bfloat16, float, false>(p, maps, fwd_form, ctiles, st)
-                          : launch_bwd_tc_t<__nv_bfloat16, __nv_bfloat16, false>(p, maps, fwd_form, ctiles, st);
+    return gate == NAJU_F32 ? launch_bwd_tc_t<__nv_bfloat16, float, true>(p, g, maps, fwd_form, cs_used, st)
+                            : launch_bwd_tc_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, fwd_form, cs_used, st);
+  return gate == NAJU_F32 ? launch_bwd_tc_t<__nv_bfloat16, float, false>(p, g, maps, fwd_form, cs_used, st)
+                          : launch_bwd_tc_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, fwd_form, cs_used, st);
 }
 
 }  // namespace naju

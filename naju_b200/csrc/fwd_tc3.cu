@@ -556,7 +556,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
         if (t.c == 0) {
           load_h0(t.x);
         } else {
-          if (alive && !mbar_wait(smem_u32(&bars.mail_full), got & 1)) {
+          if (alive && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.mail_full), got & 1))) {
             timeout();
             alive = false;
           }
@@ -582,7 +582,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
         }
         if (t.c + 1 < nchunks) {
           // (the rank after has taken the mail before)
-          if (alive && sent > 0 && !mbar_wait(smem_u32(&bars.mail_empty), (sent - 1) & 1)) {
+          if (alive && sent > 0 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.mail_empty), (sent - 1) & 1))) {
             timeout();
             alive = false;
           }
@@ -690,6 +690,15 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
       // stage's staging tile (step t -> 256 contiguous bytes); P_t comes back from TMEM
       const int st = e_it & 1;
       const uint32_t par = (e_it >> 1) & 1;
+      // (D_skip is zero from the mixer, naju/mixer.py:120-124; where it is not, the steps' u comes from L2, all loads
+      // in flight while the accumulators are waited for: one at a time they took longer than the tile)
+      float us[SLAB];
+      if (e_Dv != 0.f) {
+        const TA* gu = reinterpret_cast<const TA*>(p.u) + e_b * p.u_sb + static_cast<int64_t>(e_t0 + SLAB * grp) * p.u_st +
+                       static_cast<int64_t>(e_d0 + q) * p.u_sd;
+#pragma unroll
+        for (int j = 0; j < SLAB; ++j) us[j] = SLAB * grp + j < e_len ? to_f32(gu[static_cast<int64_t>(j) * p.u_st]) : 0.f;
+      }
       if (!mbar_wait(smem_u32(&bars.acc_free[st]), par)) timeout();   // (the deep flag's writers arrived here)
       if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();
       // the staging tile was last used NY tiles back: that store must have read it
@@ -707,21 +716,13 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
             (static_cast<int64_t>(e_b) * p.T + e_t0 + SLAB * grp) * p.D + e_d0 + q;
         [[maybe_unused]] const int nout = e_d0 + q < p.D ? e_len - SLAB * grp : 0;   // steps of this thread that exist
         [[maybe_unused]] unsigned char* dst = smem + SM::off_Y + ys * (Q * kDT * 2) + (SLAB * grp) * (kDT * 2) + q * 2;
-        const TA* gu = reinterpret_cast<const TA*>(p.u) + e_b * p.u_sb + static_cast<int64_t>(e_t0 + SLAB * grp) * p.u_st +
-                       static_cast<int64_t>(e_d0 + q) * p.u_sd;
         tmem_ld_wait16(v);
         tmem_ld_wait16(pv);
 #pragma unroll
         for (int j2 = 0; j2 < SLAB / 2; ++j2) {
           float2 y = mul2(make_float2(__uint_as_float(pv[2 * j2]), __uint_as_float(pv[2 * j2 + 1])),
                           make_float2(__uint_as_float(v[2 * j2]), __uint_as_float(v[2 * j2 + 1])));
-          if (e_Dv != 0.f) {  // (the mixer passes a zero D_skip: naju/mixer.py:120-124)
-            const int t = SLAB * grp + 2 * j2;
-            float u0 = 0.f, u1 = 0.f;
-            if (t < e_len) u0 = to_f32(gu[static_cast<int64_t>(2 * j2) * p.u_st]);
-            if (t + 1 < e_len) u1 = to_f32(gu[static_cast<int64_t>(2 * j2 + 1) * p.u_st]);
-            y = fma2(make_float2(e_Dv, e_Dv), make_float2(u0, u1), y);
-          }
+          if (e_Dv != 0.f) y = fma2(make_float2(e_Dv, e_Dv), make_float2(us[2 * j2], us[2 * j2 + 1]), y);
           unsigned short o0, o1;
           if constexpr (std::is_same<TA, __nv_bfloat16>::value) {
             const uint32_t pk = pack_bf16x2(y.x, y.y);  // one conversion for two steps
@@ -876,43 +877,11 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
 // ------------------------------------------------------------------------------ host side
 namespace {
 
-// Clusters of `cs` CTAs that fit on the current device at once (cached per device; a racing first call asks twice).
-template <typename K>
-int max_clusters(K* kern, size_t smem, int cs, std::atomic<int> (&cache)[64]) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) dev = 0;
-  int n = cache[dev].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(cs));
-  cfg.blockDim = dim3(tc3::kThreadsOf<true>);
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(cs);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-    cudaGetLastError();
-    n = 1;
-  }
-  cache[dev].store(n, std::memory_order_relaxed);
-  return n;
-}
-
 #ifndef NAJU_C2
 #define NAJU_C2 41
 #define NAJU_C4 48
 #define NAJU_CSMAX 4
 #endif
-// Trips of the busiest CTA with clusters of `cs`, and how many clusters there are.
-int64_t trips_of(const Geometry& g, int cs, int64_t fit, int64_t& clusters) {
-  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
-  clusters = std::min<int64_t>(ctiles, fit);
-  return ((ctiles + clusters - 1) / clusters * g.nchunks + cs - 1) / cs;
-}
-
 template <typename TA, typename TG, bool UTM>
 int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, int form, cudaStream_t st) {
   auto walk = tc3::fwd_tc3_kernel<TA, TG, UTM, false>;
@@ -928,9 +897,9 @@ int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, i
   // until the carry sets the pace; a tile takes 2.9 us in a cluster of one, 4.1 us in one of two, 4.8 us in
   // one of four (1.2 us for each hop of the carry), and clusters of eight (9.6 us) do not pay.
   int best = 1;
-  int64_t clusters, n, cost = trips_of(g, 1, tmah::sm_count(), clusters) * 29;
+  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 29;
   for (int k = 0, cs = 2; cs <= NAJU_CSMAX; ++k, cs *= 2) {
-    const int64_t c = trips_of(g, cs, max_clusters(shared, smemc, cs, fit[k]), n) * (cs == 2 ? NAJU_C2 : NAJU_C4);
+    const int64_t c = tmah::cluster_trips(g, cs, tmah::max_clusters(shared, tc3::kThreadsOf<true>, smemc, cs, fit[k]), n) * (cs == 2 ? NAJU_C2 : NAJU_C4);
     if (c < cost) {
       cost = c;
       best = cs;

@@ -97,7 +97,8 @@ inline BwdScratchLayout bwd_scratch_layout(const Geometry& g) {
   const size_t sP = align_up(static_cast<size_t>(g.ntiles) * 128 * 4, 256);
   const size_t sS = align_up(static_cast<size_t>(g.ntiles) * 128 * g.NS * 4, 256);
   const size_t sBC = align_up(static_cast<size_t>(g.B) * g.T * g.ndt * g.NS * 4, 256);
-  const size_t sD = align_up(static_cast<size_t>(g.nchunks) * g.B * g.ndt * 128 * 4, 256);
+  // dD partial rows: one per chunk and batch row, or one per group and rank (up to 4 x 4) of the tensor-core backward
+  const size_t sD = align_up(static_cast<size_t>(g.nchunks < 16 ? 16 : g.nchunks) * g.B * g.ndt * 128 * 4, 256);
   l.off_aggL = l.off_aggP + sP;
   l.off_inclL = l.off_aggL + sS;
   l.off_dBpart = l.off_inclL + sS;
@@ -134,7 +135,7 @@ struct BwdParams {
   const float* dhT;
   const float* ckS;
   const int* fwd_form;  // CkptTrailer::fwd_form; when (fwd_form & 3) == 1 the tensor-core backward runs
-  int tc_launched;      // the tensor-core backward was launched for this call (host decision)
+  int tc_launched;      // CTAs per channel tile of the tensor-core backward launched for this call (0: none was)
   void *du, *dfl, *dil;
   float* dh0;
   ScratchHeader* hdr;
@@ -163,9 +164,9 @@ int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int ga
 // dB, dC and dD from the partial sums; overwrites every output with NaN if the call (or its forward) failed
 int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* dB, void* dC, float* dD,
                         bool inject, void* stream);
-// tensor-core backward; returns -1000 when the problem cannot take it
+// tensor-core backward; returns -1000 when it cannot take the problem.  cs_used: CTAs that share a channel tile.
 int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
-                  const int* fwd_form, void* stream);
+                  const int* fwd_form, int& cs_used, void* stream);
 int launch_step(const naju_scan_desc& d, float* state, const void* u, const void* fl,
                 const void* il, const void* Bm, const void* Cm, const float* Dskip, void* y,
                 void* stream);

@@ -7,7 +7,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "naju_b200.h"
+#include "params.h"
 
 namespace naju {
 namespace tmah {
@@ -88,6 +91,39 @@ inline int sm_count() {
   if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
   if (dev >= 0 && dev < kMaxDev) __atomic_store_n(&cache[dev], n, __ATOMIC_RELAXED);
   return n;
+}
+
+// Clusters of `cs` CTAs that fit on the current device at once (cached per device; a racing first call asks twice).
+template <typename K>
+int max_clusters(K* kern, int threads, size_t smem, int cs, std::atomic<int> (&cache)[64]) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) dev = 0;
+  int n = cache[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cs));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(cs);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = 1;
+  }
+  cache[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Trips of the busiest CTA when clusters of `cs` CTAs walk the channel tiles, `fit` of them at once; `clusters` = how many
+// clusters there are then.
+inline int64_t cluster_trips(const Geometry& g, int cs, int64_t fit, int64_t& clusters) {
+  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
+  clusters = ctiles < fit ? ctiles : fit;
+  return ((ctiles + clusters - 1) / clusters * g.nchunks + cs - 1) / cs;
 }
 
 }  // namespace tmah
