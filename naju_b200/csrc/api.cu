@@ -174,7 +174,8 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
   int rck = -1000;
   if (!(desc->flags & NAJU_FLAG_RECURRENT_ONLY)) {
     rck = launch_fwd_tc3(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
-    if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;
+    if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;   // (the flag asks for the 16-state form)
+    if (rck == -1000) rck = launch_fwd_wide(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
   }
   if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
   return rck;
@@ -230,7 +231,11 @@ int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     // chunked and met no deep-gate tile; the recurrent backward launched after it does the
     // opposite, so exactly one of the two does the work and no host round trip is needed.
     int cs = 0;
-    const int rc2 = launch_bwd_tc(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, p.fwd_form, cs, stream);
+    int rc2 = launch_bwd_tc(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, p.fwd_form, cs, stream);
+    if (rc2 == -1000) {
+      rc2 = launch_bwd_wide(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
+      cs = 1;
+    }
     if (rc2 == 0) p.tc_launched = cs;
     else if (rc2 != -1000) return rc2;
   }

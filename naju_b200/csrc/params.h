@@ -108,6 +108,14 @@ inline BwdScratchLayout bwd_scratch_layout(const Geometry& g) {
   return l;
 }
 
+// Whether the walk kernels of 17 to 64 states (fwd_wide.cu, bwd_wide.cu) pay: a CTA takes a tile in about 50 times what the
+// recurrent kernels, spread over the whole GPU and over time, need per tile (64 states: 5.0 us against 0.10 us forward, 9.1
+// against 0.21 us backward; 32 states: 2.95 / 0.06 and 5.7 / 0.18 us).
+inline bool wide_walk_pays(const Geometry& g, int64_t sms) {
+  const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
+  return (ctiles + sms - 1) / sms * 50 <= ctiles;
+}
+
 struct FwdParams {
   const void *u, *fl, *il, *Bm, *Cm;
   const float* Dskip;
@@ -160,6 +168,9 @@ int launch_fwd_simt(const FwdParams& p, const Geometry& g, int act_dtype, int ga
 // tensor-core forward; returns -1000 when it cannot take the problem
 int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
                    void* stream);
+// tensor-core walks of 17 to 64 states
+int launch_fwd_wide(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
+int launch_bwd_wide(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
 int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);
 // dB, dC and dD from the partial sums; overwrites every output with NaN if the call (or its forward) failed
 int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* dB, void* dC, float* dD,

@@ -311,6 +311,43 @@ __device__ __forceinline__ bool bar_or(bool pred) {
   return out != 0;
 }
 
+// ---- gate arithmetic
+constexpr float kRMax = 1.0e24f;  // ~2^80: largest 1 / (retention product of a chunk) that the factorised form takes
+constexpr float kNegLog2e = -1.4426950408889634f;
+__device__ __forceinline__ float fast_ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// packed fp32 pairs (one instruction for two lanes of arithmetic)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 f2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
+
+// Two-term bf16 split of a pair: v ~= hi + lo, both truncations (the first one's error is exactly what the second
+// term carries), so it costs integer and FMA-pipe operations only; residual <= 2^-16 relative.
+__device__ __forceinline__ void split_pair(float2 v, uint32_t& hi, uint32_t& lo) {
+  const uint32_t ua = __float_as_uint(v.x), ub = __float_as_uint(v.y);
+  hi = __byte_perm(ua, ub, 0x7632);
+  const float2 h = make_float2(__uint_as_float(ua & 0xFFFF0000u), __uint_as_float(ub & 0xFFFF0000u));
+  const float2 l = fma2(h, make_float2(-1.f, -1.f), v);
+  lo = __byte_perm(__float_as_uint(l.x), __float_as_uint(l.y), 0x7632);
+}
+// The same with a third term: all 24 bits of the significand.
+__device__ __forceinline__ void split3(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t ua = __float_as_uint(v.x), ub = __float_as_uint(v.y);
+  hi = __byte_perm(ua, ub, 0x7632);
+  const float2 h = make_float2(__uint_as_float(ua & 0xFFFF0000u), __uint_as_float(ub & 0xFFFF0000u));
+  split_pair(fma2(h, make_float2(-1.f, -1.f), v), mid, lo);
+}
+
 // ---- bf16 helpers
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {  // lo -> bits [0,16)
   uint32_t r;

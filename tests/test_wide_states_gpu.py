@@ -1,0 +1,62 @@
+"""The tensor-core kernels of 17 to 64 states against the fp64 oracle, at the edges of their tiles (32 steps, 128
+channels, 16-step and 8-step slabs, state widths of 32 and 64)."""
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+WALK, RECURRENT = 3, 1
+BF, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.fixture(autouse=True)
+def _status_checks(monkeypatch):
+    monkeypatch.setenv("NAJU_B200_CHECK_STATUS", "1")
+
+
+def _round(x, dt):
+    return torch.tensor(x).to(dt).float().numpy()
+
+
+# B, T, D, N, f_shift, logits, time-contiguous u, fwd form, bwd form
+@pytest.mark.parametrize("case", [
+    (8, 1, 2432, 64, 2.0, BF, False, WALK, WALK),          # one step
+    (8, 31, 2432, 64, 2.0, BF, False, WALK, WALK),         # one short chunk
+    (4, 73, 4360, 64, 2.0, BF, False, WALK, WALK),         # ragged end, partial channel tile (D % 128 = 8)
+    (5, 96, 4096, 40, 4.0, BF, False, WALK, WALK),         # more channel tiles than SMs, padded states
+    (6, 104, 2560, 24, 2.0, BF, True, WALK, WALK),         # time-contiguous u, 32-state kernels
+    (6, 67, 2560, 32, 2.0, F32, False, WALK, RECURRENT),   # fp32 logits keep the recurrent backward
+    (6, 96, 2560, 64, 0.0, BF, False, WALK, WALK),         # retention about one half
+    (6, 96, 2560, 64, -3.0, BF, False, WALK, RECURRENT),   # deep gates: exact tiles, recurrent backward
+    (6, 96, 2560, 20, 2.0, BF, False, RECURRENT, RECURRENT),   # rows of B / C that TMA cannot describe
+    (1, 2048, 256, 64, 2.0, BF, False, RECURRENT, RECURRENT)])  # too few channel tiles
+def test_wide_state_kernels_match_the_oracle(case):
+    """16-bit outputs against the identically rounded oracle; the fp32 ones (final state, dD, dh0, and dfl with fp32
+    logits) to 1e-6, which the recurrent kernels' 1e-7 to 2e-7 leaves room for and a two-term operand (1e-5) would not."""
+    from naju_b200 import naju_scan
+    from naju_b200.scan import last_kernel_forms
+    B, T, D, N, fs, gdt, utm, ffwd, fbwd = case
+    d = oracle.make_inputs(B, T, D, N, seed=5, f_shift=fs, d_skip_scale=0.05, with_h0=True)
+    cast = {"u": BF, "Bm": BF, "Cm": BF, "dy": BF, "fl": gdt, "il": gdt}
+    q = {k: (_round(d[k], cast[k]) if k in cast else d[k]) for k in d}
+    t = {k: torch.tensor(q[k], device="cuda").to(cast.get(k, F32)) for k in ("u", "fl", "il", "Bm", "Cm", "Dskip", "h0")}
+    if utm:
+        t["u"] = t["u"].transpose(1, 2).contiguous().transpose(1, 2)
+    for k in t:
+        t[k].requires_grad_(True)
+    y, hT = naju_scan(t["u"], t["fl"], t["il"], t["Bm"], t["Cm"], t["Dskip"], h0=t["h0"], return_final_state=True)
+    torch.autograd.backward([y, hT], [torch.tensor(q["dy"], device="cuda").to(BF), torch.tensor(d["dhT"], device="cuda")])
+    torch.cuda.synchronize()
+    assert last_kernel_forms() == {"fwd": ffwd, "bwd": fbwd}
+    a = (q["u"], q["fl"], q["il"], q["Bm"], q["Cm"], q["Dskip"])
+    yo, hTo = oracle.oracle_fwd(*a, h0=q["h0"], return_final_state=True)
+    g = oracle.oracle_bwd(*a, q["dy"], h0=q["h0"], dhT=d["dhT"])
+    assert oracle.rel_l2(y.detach().float().cpu().numpy(), _round(yo, BF)) < 1e-3
+    assert oracle.rel_l2(hT.detach().cpu().numpy(), hTo) < 1e-6
+    for k, src in (("du", "u"), ("dfl", "fl"), ("dil", "il"), ("dB", "Bm"), ("dC", "Cm")):
+        ref = _round(g[k], gdt if k in ("dfl", "dil") else BF)
+        assert oracle.rel_l2(t[src].grad.float().cpu().numpy(), ref) < 2e-3, k
+    assert oracle.rel_l2(t["Dskip"].grad.cpu().numpy(), g["dD"]) < 1e-6
+    assert oracle.rel_l2(t["h0"].grad.cpu().numpy(), g["dh0"]) < 1e-6
