@@ -204,7 +204,7 @@ bwd_simt_kernel(const BwdParams p) {
         }
       }
       float accP[kC];
-      const int64_t src = look_back<NS, K>(p.flags, p.aggP, p.aggL, p.inclL, tile + per_chunk, per_chunk, p.nchunks - 1 - c, chan0,
+      const int64_t src = look_back<NS, K, NH == 2 ? 4 : 1>(p.flags, p.aggP, p.aggL, p.inclL, tile + per_chunk, per_chunk, p.nchunks - 1 - c, chan0,
                                            q, lane, carry, accP);
       if (src < 0) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
     }

@@ -82,40 +82,11 @@ constexpr uint32_t BC_BYTES = Q * NS * 2;
 // (dL sits directly before gt: one MMA with the B operand [C | g1] accumulates into both)
 constexpr uint32_t TM_Y = 0, TM_DL = 64, TM_G = 80, TM_X = 144, TM_DCI = TM_X, TM_DBI = TM_X + 16, TM_CF = 240,
                    TM_CI = 304, TM_CU = 368, TM_GB = 432, TMEM_COLS = 512;
-constexpr float kRMax = 1.0e24f;
-constexpr float kNegLog2e = -1.4426950408889634f;
 // Every wait parks the warp in mbarrier.try_wait (the hardware wakes it when the phase completes);
 // sleeping 32-64 ns between polls instead, in any of the roles, was measured and is 4 % slower.
 
-__device__ __forceinline__ float fast_ex2(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float fast_rcp(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 __device__ __forceinline__ uint32_t idesc_bf16(int N, uint32_t a_mn, uint32_t b_mn) {
   return umma_idesc(128, N, 1) | (a_mn << 15) | (b_mn << 16);
-}
-
-// packed fp32 pairs (one instruction for two lanes of arithmetic)
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 f2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
-
-// Two-term bf16 split of a pair: v ~= hi + lo, both truncations, so it costs integer and FMA-pipe
-// operations only; residual <= 2^-16 relative.
-__device__ __forceinline__ void split_pair(float2 v, uint32_t& hi, uint32_t& lo) {
-  const uint32_t ua = __float_as_uint(v.x), ub = __float_as_uint(v.y);
-  hi = __byte_perm(ua, ub, 0x7632);
-  const float2 h = make_float2(__uint_as_float(ua & 0xFFFF0000u), __uint_as_float(ub & 0xFFFF0000u));
-  const float2 l = fma2(h, make_float2(-1.f, -1.f), v);
-  lo = __byte_perm(__float_as_uint(l.x), __float_as_uint(l.y), 0x7632);
 }
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
@@ -827,6 +798,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
       const int b = x / p.ndt, dt = x - b * p.ndt, d0 = dt * kDT, d = d0 + cid;
       const bool d_ok = d < p.D;
       const float Dv = d_ok ? __ldg(p.Dskip + d) : 0.f;
+      const bool any_skip = __any_sync(0xffffffffu, Dv != 0.f);
       dDsum = 0.f;
       int ci = ci0;
 #pragma unroll 1
@@ -958,6 +930,8 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
         }
         mbar_arrive_warp(smem_u32(&bars.ssum[grp]));
         // ---------------- sweep (2): r_t = seed + (sums of the groups after) + S_t; the three gradients
+        // (where D_skip is not zero dy comes from L2 again, eight steps in flight: one at a time it took a third of the kernel's
+        // time, 2.26 against 1.53 ms at B=8, T=16384, D=2048)
         if (!mbar_wait(smem_u32(&bars.seed_ready[it & 1]), (it >> 1) & 1)) timeout();
         float rstart = s_seed[it & 1][cid];
         for (int g2 = NGRP - 1; g2 > grp; --g2) {
@@ -973,10 +947,17 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
                       : reinterpret_cast<TA*>(p.du) + row0;
         TG* gdfl = reinterpret_cast<TG*>(p.dfl) + row0;
         TG* gdil = reinterpret_cast<TG*>(p.dil) + row0;
-        const TA* gdy = reinterpret_cast<const TA*>(p.dy) + row0;
+        auto gradients = [&](auto with_skip) {
+          constexpr bool skip = decltype(with_skip)::value;
 #pragma unroll
         for (int j8 = SLAB / 8 - 1; j8 >= 0; --j8) {
           uint32_t g8[8], f8[8], i8[8], u8[8];
+          [[maybe_unused]] unsigned short dc[8];
+          if constexpr (skip) {
+            const unsigned short* gdy = reinterpret_cast<const unsigned short*>(p.dy) + row0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) dc[e] = d_ok && 8 * j8 + e < nvalid ? __ldg(gdy + static_cast<int64_t>(8 * j8 + e) * p.D) : 0;
+          }
           tmem_ld8_async(trow + TM_G + 8 * j8, g8);
           tmem_ld8_async(trow + TM_CF + 8 * j8, f8);
           tmem_ld_wait8(g8, f8);
@@ -992,10 +973,9 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
             float2 du = mul2(f2(u8[2 * jj], u8[2 * jj + 1]), gt);
             const float2 dil = mul2(f2(i8[2 * jj], i8[2 * jj + 1]), gt);
             const bool ok0 = d_ok && j < nvalid, ok1 = d_ok && j + 1 < nvalid;
-            if (Dv != 0.f) {
-              const float y0 = ok0 ? to_f32(gdy[static_cast<int64_t>(j) * p.D]) : 0.f;
-              const float y1 = ok1 ? to_f32(gdy[static_cast<int64_t>(j + 1) * p.D]) : 0.f;
-              du = fma2(Dv2, make_float2(y0, y1), du);
+            if constexpr (skip) {
+              if (Dv != 0.f) du = fma2(Dv2, make_float2(__uint_as_float(static_cast<uint32_t>(dc[2 * jj]) << 16),
+                                         __uint_as_float(static_cast<uint32_t>(dc[2 * jj + 1]) << 16)), du);
             }
             if constexpr (utm) dupk[jj] = pack_bf16x2(du.x, du.y);
             if (ok0) {
@@ -1022,6 +1002,10 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
             }
           }
         }
+        };
+        // (two copies: the one without D_skip needs fewer registers, and a spill there costs 15 % of the kernel's time)
+        if (any_skip) gradients(std::true_type{});
+        else gradients(std::false_type{});
         tc_fence_before();
         mbar_arrive_warp(smem_u32(&bars.acc_free));      // Yt, gt and the coefficients have been read
       }
@@ -1051,26 +1035,22 @@ int launch_bwd_tc_t(const BwdParams& p, const Geometry& g, const tcb::Maps& maps
   int rc = allow_smem(walk, smem, ok1);
   if (rc == 0) rc = allow_smem(shared, smem, okc);
   if (rc != 0) return rc;
-  // The cluster size with the shortest busiest CTA, in units of 0.1 us: a tile takes 5.7 us in a cluster of one and
-  // somewhat longer when ranks wait for each other's adjoint.
-#ifndef NAJU_B2
-#define NAJU_B2 62
-#define NAJU_B4 72
-#endif
+  // The cluster size with the shortest busiest CTA, in units of 0.1 us: a tile takes 6.0 us in a cluster of one, 10.0 us in
+  // one of two and 10.5 us in one of four, whose ranks wait for each other's adjoint.
   int best = 1;
-  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 57;
+  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 60;
   for (int k = 0, cs = 2; cs <= 4 && cs <= g.nchunks; ++k, cs *= 2) {
     const int64_t fits = tmah::max_clusters(shared, tcb::NTHREADS, smem, cs, fit[k]);
-    const int64_t c = tmah::cluster_trips(g, cs, fits, n) * (cs == 2 ? NAJU_B2 : NAJU_B4);
+    const int64_t c = tmah::cluster_trips(g, cs, fits, n) * (cs == 2 ? 100 : 105);
     if (c < cost) {
       cost = c;
       best = cs;
       clusters = n;
     }
   }
-  // The exact recurrent backward spreads over time too: it takes about 0.3 us per tile of 64 steps x 128 channels on a
-  // full GPU, and 15 us at least.  (Every tile here has its own carry to wait for, 10 us in all.)
-  if (cost + 100 > 150 + 3 * g.ntiles) return -1000;
+  // The exact recurrent backward spreads over time too: 15 us, and 0.3 to 0.39 us per tile of 64 steps x 128 channels on a full
+  // GPU or 1.5 us per chunk where the look-back sets the pace.  (Every tile here has its own carry to wait for, 10 us in all.)
+  if (cost + 100 > 150 + std::max<int64_t>(7 * g.ntiles / 2, 15 * static_cast<int64_t>(g.nchunks))) return -1000;
   cs_used = best;
   const dim3 grid(static_cast<unsigned>(clusters * best)), block(tcb::NTHREADS);
   return best == 1 ? launch_pdl(walk, grid, block, smem, st, p, maps, fwd_form)

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(Shape<NS>::NT, NS == 128 ? 1 : NS == 64 ? 2 : 
       st_release(p.flags + tile, 1);
     }
     float h[kC][K];
-    const int64_t src = look_back<NS, K>(p.flags, p.aggP, p.aggS, p.ckS, tile - per_chunk, -per_chunk, c, chan0, q, lane, h, Pin);
+    const int64_t src = look_back<NS, K, 1>(p.flags, p.aggP, p.aggS, p.ckS, tile - per_chunk, -per_chunk, c, chan0, q, lane, h, Pin);
     if (src < 0) {
       atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
     } else {

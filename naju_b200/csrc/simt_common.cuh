@@ -324,9 +324,9 @@ __device__ __forceinline__ void put_user_state(float* __restrict__ h, int64_t bd
 // state published.  On return acc = fold of the aggregates onto the first inclusive state met and accP the product
 // of the P's folded (without that tile's own); *incl_tile = that tile, or -1 when the wait ran out.
 // A window of 32 flags is looked at together, one per lane, so a long run of published aggregates costs one
-// round trip of flag reads, not one per tile.  (Fetching two or four aggregates at a time costs registers that
-// the walks need: B=4, T=2048, D=1024, N=16, fp32 backward 208 -> 264 us.)
-template <int NS, int K>
+// round trip of flag reads, not one per tile; DEPTH aggregates are fetched together.  (More than one where registers
+// are left only: B=4, T=2048, D=1024, N=16, fp32 backward 208 us with one, 264 with two.)
+template <int NS, int K, int DEPTH>
 __device__ __forceinline__ int64_t look_back(const int* __restrict__ flags, const float* __restrict__ aggP,
                                              const float* __restrict__ agg, const float* __restrict__ incl, int64_t tile0,
                                              int64_t step, int count, int chan0, int q, int lane, float (&acc)[kC][K],
@@ -346,20 +346,29 @@ __device__ __forceinline__ int64_t look_back(const int* __restrict__ flags, cons
     const int nready = ready == 0xffffffffu ? 32 : __ffs(~ready) - 1;
     const int first_inc = inc ? __ffs(inc) - 1 : 32;
     const int n = min(nready, first_inc + 1);
-    for (int k = 0; k < n; ++k) {
-      const int64_t t = tile0 + (done + k) * step;
-      const bool last = k == first_inc;
-      float v[kC][K];
-      get_state<NS, K>(last ? incl : agg, t * kDT + chan0, q, v);
-      const float4 pv = last ? make_float4(1.f, 1.f, 1.f, 1.f) : __ldcg(reinterpret_cast<const float4*>(aggP + t * kDT + chan0));
-      const float pc[kC] = {pv.x, pv.y, pv.z, pv.w};
+    for (int k = 0; k < n; k += DEPTH) {
+      float v[DEPTH][kC][K];
+      float4 pv[DEPTH];
 #pragma unroll
-      for (int c = 0; c < kC; ++c) {
-#pragma unroll
-        for (int j = 0; j < K; ++j) acc[c][j] = fmaf(accP[c], v[c][j], acc[c][j]);
-        accP[c] *= pc[c];
+      for (int m = 0; m < DEPTH; ++m) {
+        if (k + m >= n) break;
+        const int64_t t = tile0 + (done + k + m) * step;
+        const bool last = k + m == first_inc;
+        get_state<NS, K>(last ? incl : agg, t * kDT + chan0, q, v[m]);
+        pv[m] = last ? make_float4(1.f, 1.f, 1.f, 1.f) : __ldcg(reinterpret_cast<const float4*>(aggP + t * kDT + chan0));
       }
-      if (last) return t;
+#pragma unroll
+      for (int m = 0; m < DEPTH; ++m) {
+        if (k + m >= n) break;
+        const float pc[kC] = {pv[m].x, pv[m].y, pv[m].z, pv[m].w};
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+#pragma unroll
+          for (int j = 0; j < K; ++j) acc[c][j] = fmaf(accP[c], v[m][c][j], acc[c][j]);
+          accP[c] *= pc[c];
+        }
+        if (k + m == first_inc) return tile0 + (done + k + m) * step;
+      }
     }
     done += n;
     if (n == 0) {
