@@ -177,6 +177,7 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;   // (the flag asks for the 16-state form)
     if (rck == -1000) rck = launch_fwd_wide(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
   }
+  if (rck == -1000) rck = launch_fwd_chan(p, g, desc->act_dtype, desc->gate_dtype, stream);
   if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
   return rck;
 }

@@ -70,22 +70,9 @@ constexpr int B1_C = 0, B1_G1 = 2, B1_G2 = 10;
 constexpr uint32_t SBO_B1 = 18 * 128, B1_BYTES = 8 * SBO_B1;   // rows t: [C 16 | g1 64 | g2 64]
 constexpr uint32_t SBO_BB = 2 * 128, BB_BYTES = 8 * SBO_BB;    // rows s: [B 16]; read K-major (G) and MN-major (D2)
 constexpr uint32_t BC_BYTES = Q * NS * 2;
-constexpr uint32_t TM_D1 = 0, TM_D2 = 64, TM_P = 96, TM_G = 160, TM_STAGE = 224, TMEM_COLS = 512;
-constexpr float kRMax = 1.0e24f;  // ~2^80
-constexpr float kNegLog2e = -1.4426950408889634f;
+constexpr uint32_t TM_D1 = 0, TM_D2 = 64, TM_P = 96, TM_G = 160, TM_STAGE = 224, TM_U = 2 * TM_STAGE, TMEM_COLS = 512;
 // Every wait parks the warp in mbarrier.try_wait (the hardware wakes it when the phase completes);
 // sleeping between polls instead, for the roles with slack, was measured and is 1 % slower.
-
-__device__ __forceinline__ float fast_ex2(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float fast_rcp(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 
 struct Maps {
   CUtensorMap u, fl, il, bm, cm, y;
@@ -132,19 +119,17 @@ struct Bars {
   unsigned long long stage_free[NSTAGE];        // store warp: staging tile read by the store -> epilogue two tiles on
 };
 
-// packed fp32 pairs (one instruction for two lanes of arithmetic)
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-// Two-term bf16 split of a pair: v ~= hi + lo, both truncations (the first one's error is exactly what the second
-// term carries), so it costs integer and FMA-pipe operations only; residual <= 2^-16 relative.
-__device__ __forceinline__ void split_pair(float2 v, uint32_t& hi, uint32_t& lo) {
-  const uint32_t ua = __float_as_uint(v.x), ub = __float_as_uint(v.y);
-  hi = __byte_perm(ua, ub, 0x7632);
-  const float2 h = make_float2(__uint_as_float(ua & 0xFFFF0000u), __uint_as_float(ub & 0xFFFF0000u));
-  const float2 l = fma2(h, make_float2(-1.f, -1.f), v);
-  lo = __byte_perm(__float_as_uint(l.x), __float_as_uint(l.y), 0x7632);
+// two 16-bit elements, exact both ways
+template <typename TA>
+__device__ __forceinline__ uint32_t pack16(float2 v) {
+  if constexpr (std::is_same<TA, __nv_bfloat16>::value) return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632);
+  const __half2 h = __floats2half2_rn(v.x, v.y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename TA>
+__device__ __forceinline__ float2 unpack16(uint32_t v) {
+  if constexpr (std::is_same<TA, __nv_bfloat16>::value) return make_float2(bf16lo_f32(v), bf16hi_f32(v));
+  return __half22float2(*reinterpret_cast<const __half2*>(&v));
 }
 
 // Exact recurrence of one tile straight from global memory (deep-gate tiles only), run by the 128
@@ -684,21 +669,13 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
     // the tile whose epilogue is pending (it runs one tile late, after the next tile's operand rows)
     int e_b = 0, e_d0 = 0, e_t0 = 0, e_len = 0, e_it = -1;
     float e_Dv = 0.f;
+    bool e_skip = false;   // D_skip is not zero in some channel of the warp
 
     auto epilogue = [&]() {
       // y_t = P_t D1[d][t] + D_skip u_t for this thread's 16 steps of the pending tile, into the
       // stage's staging tile (step t -> 256 contiguous bytes); P_t comes back from TMEM
       const int st = e_it & 1;
       const uint32_t par = (e_it >> 1) & 1;
-      // (D_skip is zero from the mixer, naju/mixer.py:120-124; where it is not, the steps' u comes from L2, all loads
-      // in flight while the accumulators are waited for: one at a time they took longer than the tile)
-      float us[SLAB];
-      if (e_Dv != 0.f) {
-        const TA* gu = reinterpret_cast<const TA*>(p.u) + e_b * p.u_sb + static_cast<int64_t>(e_t0 + SLAB * grp) * p.u_st +
-                       static_cast<int64_t>(e_d0 + q) * p.u_sd;
-#pragma unroll
-        for (int j = 0; j < SLAB; ++j) us[j] = SLAB * grp + j < e_len ? to_f32(gu[static_cast<int64_t>(j) * p.u_st]) : 0.f;
-      }
       if (!mbar_wait(smem_u32(&bars.acc_free[st]), par)) timeout();   // (the deep flag's writers arrived here)
       if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();
       // the staging tile was last used NY tiles back: that store must have read it
@@ -716,13 +693,18 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
             (static_cast<int64_t>(e_b) * p.T + e_t0 + SLAB * grp) * p.D + e_d0 + q;
         [[maybe_unused]] const int nout = e_d0 + q < p.D ? e_len - SLAB * grp : 0;   // steps of this thread that exist
         [[maybe_unused]] unsigned char* dst = smem + SM::off_Y + ys * (Q * kDT * 2) + (SLAB * grp) * (kDT * 2) + q * 2;
+        // (D_skip is zero from the mixer, naju/mixer.py:120-124; where it is not, the steps' u comes back from the TMEM columns
+        // that are left: read again from L2 it took half the tile's time, 1.15 against 0.77 ms at B=8, T=16384, D=2048)
+        uint32_t us[SLAB / 2];
+        if (e_skip) tmem_ld8_async(tmem + TM_U + st * (Q / 2) + lane_off + (SLAB / 2) * grp, us);
         tmem_ld_wait16(v);
         tmem_ld_wait16(pv);
+        if (e_skip) tmem_ld_wait8(us);
 #pragma unroll
         for (int j2 = 0; j2 < SLAB / 2; ++j2) {
           float2 y = mul2(make_float2(__uint_as_float(pv[2 * j2]), __uint_as_float(pv[2 * j2 + 1])),
                           make_float2(__uint_as_float(v[2 * j2]), __uint_as_float(v[2 * j2 + 1])));
-          if (e_Dv != 0.f) y = fma2(make_float2(e_Dv, e_Dv), make_float2(us[2 * j2], us[2 * j2 + 1]), y);
+          if (e_Dv != 0.f) y = fma2(make_float2(e_Dv, e_Dv), unpack16<TA>(us[j2]), y);
           unsigned short o0, o1;
           if constexpr (std::is_same<TA, __nv_bfloat16>::value) {
             const uint32_t pk = pack_bf16x2(y.x, y.y);  // one conversion for two steps
@@ -751,6 +733,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
     // one) and then finishes tile `it - 1`
     int x = CLUSTER ? first_pair().x : x_first, c = CLUSTER ? first_pair().c : 0, b = 0, d0 = 0;
     float Dv = 0.f;
+    bool skip = false;
 #pragma unroll 1
     for (int it = 0; it <= ntotal; ++it) {
       if (it < ntotal) {
@@ -758,6 +741,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
           b = x / p.ndt;
           d0 = (x - b * p.ndt) * kDT;
           Dv = (d0 + q < p.D) ? __ldg(p.Dskip + d0 + q) : 0.f;
+          skip = __any_sync(0xffffffffu, Dv != 0.f);
         }
         const int st = it & 1;
         const uint32_t par = (it >> 1) & 1;
@@ -820,13 +804,14 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
         const uint32_t tP = tmem + st * TM_STAGE + lane_off + TM_P + SLAB * grp;
 #pragma unroll
         for (int j8 = 0; j8 < SLAB / 8; ++j8) {
-          uint32_t hi[4], lo[4], pv[8];
+          uint32_t hi[4], lo[4], pv[8], uk[4];
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
             const int j2 = 4 * j8 + jj;
             const float2 opb = opbv[j2];                                                   // 1 / i_t
             const float2 u2 = utm ? ld_pair_as_f32(s_ut + 2 * j2)
                                   : make_float2(ld_as_f32(s_u, (2 * j2) * kDT), ld_as_f32(s_u, (2 * j2 + 1) * kDT));
+            uk[jj] = pack16<TA>(u2);
             const float2 R = mul2(Rs2, L[j2]);
             const float2 x2 = mul2(R, opb);
             const float2 r = make_float2(fast_rcp(x2.x), fast_rcp(x2.y));
@@ -840,6 +825,9 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
           *reinterpret_cast<uint4*>(a_row + (AW_W2 + 2 * grp + j8) * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(tP + 8 * j8),
                        "r"(pv[0]), "r"(pv[1]), "r"(pv[2]), "r"(pv[3]), "r"(pv[4]), "r"(pv[5]), "r"(pv[6]), "r"(pv[7]));
+          if (skip)
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tmem + TM_U + st * (Q / 2) + lane_off +
+                         (SLAB / 2) * grp + 4 * j8), "r"(uk[0]), "r"(uk[1]), "r"(uk[2]), "r"(uk[3]));
         }
         mbar_arrive_warp(smem_u32(&bars.empty[slot]));            // the slab has been read
         // the last group holds the whole chunk's product: the carry warps' P_Q and deep-gate decision
@@ -853,7 +841,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
       // ---- (3) the previous tile's outputs for the same steps
       if (it > 0) epilogue();
       if (it < ntotal) {
-        e_b = b; e_d0 = d0; e_t0 = c * Q; e_len = min(Q, p.T - c * Q); e_it = it; e_Dv = Dv;
+        e_b = b; e_d0 = d0; e_t0 = c * Q; e_len = min(Q, p.T - c * Q); e_it = it; e_Dv = Dv; e_skip = skip;
         if constexpr (CLUSTER) {
           Pair t{x, c};
           next_pair(t);
@@ -877,35 +865,33 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
 // ------------------------------------------------------------------------------ host side
 namespace {
 
-#ifndef NAJU_C2
-#define NAJU_C2 41
-#define NAJU_C4 48
-#define NAJU_CSMAX 4
-#endif
 template <typename TA, typename TG, bool UTM>
 int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, int form, cudaStream_t st) {
   auto walk = tc3::fwd_tc3_kernel<TA, TG, UTM, false>;
   auto shared = tc3::fwd_tc3_kernel<TA, TG, UTM, true>;
   constexpr size_t smem1 = tc3::Smem<TG, false>::total, smemc = tc3::Smem<TG, true>::total;
   static std::atomic<unsigned long long> ok1{0}, okc{0};
-  static std::atomic<int> fit[3][64];
+  static std::atomic<int> fit[2][64];
   int rc = allow_smem(walk, smem1, ok1);
   if (rc == 0) rc = allow_smem(shared, smemc, okc);
-  if (rc == 0) rc = launch_init(p.hdr, 256, p.fwd_form, st);
   if (rc != 0) return rc;
-  // The cluster size with the shortest busiest CTA.  With fewer channel tiles than SMs more CTAs per channel tile win
-  // until the carry sets the pace; a tile takes 2.9 us in a cluster of one, 4.1 us in one of two, 4.8 us in
+  // The cluster size with the shortest busiest CTA, in units of 0.1 us.  With fewer channel tiles than SMs more CTAs per
+  // channel tile win until the carry sets the pace; a tile takes 3.0 us in a cluster of one, 4.5 us in one of two, 4.7 us in
   // one of four (1.2 us for each hop of the carry), and clusters of eight (9.6 us) do not pay.
   int best = 1;
-  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 29;
-  for (int k = 0, cs = 2; cs <= NAJU_CSMAX; ++k, cs *= 2) {
-    const int64_t c = tmah::cluster_trips(g, cs, tmah::max_clusters(shared, tc3::kThreadsOf<true>, smemc, cs, fit[k]), n) * (cs == 2 ? NAJU_C2 : NAJU_C4);
+  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 30;
+  for (int k = 0, cs = 2; cs <= 4; ++k, cs *= 2) {
+    const int64_t c = tmah::cluster_trips(g, cs, tmah::max_clusters(shared, tc3::kThreadsOf<true>, smemc, cs, fit[k]), n) * (cs == 2 ? 45 : 47);
     if (c < cost) {
       cost = c;
       best = cs;
       clusters = n;
     }
   }
+  // Few channel tiles and many chunks: the ticket kernel takes a chunk every 0.5 us or a tile every 0.1 us, whichever is longer.
+  if (p.u_sd == 1 && cost > std::max<int64_t>(5 * static_cast<int64_t>(g.nchunks), g.ntiles)) return -1001;
+  rc = launch_init(p.hdr, 256, p.fwd_form, st);
+  if (rc != 0) return rc;
   const dim3 grid(static_cast<unsigned>(clusters * best)), block(best > 1 ? tc3::kThreadsOf<true> : tc3::kThreadsOf<false>);
   return best == 1 ? launch_pdl(walk, grid, block, smem1, st, p, maps, form)
                    : launch_cluster(shared, grid, block, smemc, best, st, p, maps, form);
@@ -936,15 +922,18 @@ int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int
   if (!ok) return -1000;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool utm = p.u_sd > 1;
+  int rc;
   if (act == NAJU_BF16 && gate == NAJU_BF16)
-    return utm ? launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, form, st)
-               : launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, form, st);
-  if (act == NAJU_BF16 && gate == NAJU_F32)
-    return utm ? launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, form, st)
-               : launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, form, st);
-  if (act == NAJU_F16 && gate == NAJU_F16)
-    return utm ? launch_tc3_t<__half, __half, true>(p, g, maps, form, st) : launch_tc3_t<__half, __half, false>(p, g, maps, form, st);
-  return utm ? launch_tc3_t<__half, float, true>(p, g, maps, form, st) : launch_tc3_t<__half, float, false>(p, g, maps, form, st);
+    rc = utm ? launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, form, st)
+             : launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, form, st);
+  else if (act == NAJU_BF16)
+    rc = utm ? launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, form, st)
+             : launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, form, st);
+  else if (gate == NAJU_F16)
+    rc = utm ? launch_tc3_t<__half, __half, true>(p, g, maps, form, st) : launch_tc3_t<__half, __half, false>(p, g, maps, form, st);
+  else
+    rc = utm ? launch_tc3_t<__half, float, true>(p, g, maps, form, st) : launch_tc3_t<__half, float, false>(p, g, maps, form, st);
+  return rc == -1001 ? launch_fwd_tc2(p, g, act, gate, bc, stream) : rc;
 }
 
 }  // namespace naju

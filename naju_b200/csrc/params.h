@@ -14,9 +14,9 @@ inline int padded_states(int N) { return N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ?
 // Chunk length (time steps per tile); the spacing of the saved chunk-boundary states.  64 for the types
 // and the state width that the tensor-core kernels take (their tiles are 64 steps), 32 for everything
 // else: half the shared memory per tile of the recurrent kernels, so three instead of one of their
-// backward's CTAs fit on an SM.
+// backward's CTAs fit on an SM.  So too where rows are no multiple of 16 bytes and TMA cannot describe them.
 inline int chunk_len_for(const naju_scan_desc& d) {
-  return (d.N == 16 && d.act_dtype != NAJU_F32 && d.bc_dtype == NAJU_BF16) ? 64 : 32;
+  return (d.N == 16 && d.act_dtype != NAJU_F32 && d.bc_dtype == NAJU_BF16 && d.D % 8 == 0) ? 64 : 32;
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -168,6 +168,10 @@ int launch_fwd_simt(const FwdParams& p, const Geometry& g, int act_dtype, int ga
 // tensor-core forward; returns -1000 when it cannot take the problem
 int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype,
                    void* stream);
+// tensor-core forward that takes its tiles by ticket, for few channel tiles
+int launch_fwd_tc2(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
+// exact recurrent forward of 16 states and 16-bit inputs; returns -1000 when it cannot take the problem
+int launch_fwd_chan(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);
 // tensor-core walks of 17 to 64 states
 int launch_fwd_wide(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
 int launch_bwd_wide(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
