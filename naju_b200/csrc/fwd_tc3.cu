@@ -559,7 +559,15 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
 #pragma unroll
           for (int n = 0; n < NS; ++n) e[n] = hc[n];
           set_coord(tcd, t.x, t.c);
-          exact_tile_from_global<TA, TG>(p, tcd, q, e, Pe);
+          // (copies: what a call takes by reference lives in local memory everywhere)
+          const TileCoord at = tcd;
+          float hw[NS], Pw = Pe;
+#pragma unroll
+          for (int n = 0; n < NS; ++n) hw[n] = e[n];
+          exact_tile_from_global<TA, TG>(p, at, q, hw, Pw);
+#pragma unroll
+          for (int n = 0; n < NS; ++n) e[n] = hw[n];
+          Pe = Pw;
         } else {
 #pragma unroll
           for (int n = 0; n < NS; ++n) e[n] = Pe * (hc[n] + e[n]);
@@ -628,7 +636,14 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
         tc_fence_after();
         if (deep) {
           if (q == 0) atomicOr(p.fwd_form, 2);
-          exact_tile_from_global<TA, TG>(p, tcd, q, hc, Pc);
+          const TileCoord at = tcd;   // (copies, as above)
+          float hw[NS], Pw = Pc;
+#pragma unroll
+          for (int n = 0; n < NS; ++n) hw[n] = hc[n];
+          exact_tile_from_global<TA, TG>(p, at, q, hw, Pw);
+#pragma unroll
+          for (int n = 0; n < NS; ++n) hc[n] = hw[n];
+          Pc = Pw;
         } else {
           // chunk aggregate from D2: chunk-end state = next carry-in = checkpoint
           uint32_t sr[16];
@@ -876,7 +891,7 @@ int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, i
   if (rc == 0) rc = allow_smem(shared, smemc, okc);
   if (rc != 0) return rc;
   // The cluster size with the shortest busiest CTA, in units of 0.1 us.  With fewer channel tiles than SMs more CTAs per
-  // channel tile win until the carry sets the pace; a tile takes 3.0 us in a cluster of one, 4.5 us in one of two, 4.7 us in
+  // channel tile win until the carry sets the pace; a tile takes 2.8 to 3.0 us in a cluster of one, 4.5 us in one of two, 4.7 us in
   // one of four (1.2 us for each hop of the carry), and clusters of eight (9.6 us) do not pay.
   int best = 1;
   int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 30;

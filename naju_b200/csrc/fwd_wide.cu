@@ -10,7 +10,8 @@
 // and to 16 bits (2^-16 relative) where it enters y.
 //
 // What bounds it: the recurrent kernel does N multiply-adds and N loads' worth of B and C per channel and step on the
-// CUDA cores (64 states: 7 ms for 8 x 8192 x 4096); here that work is 22 MMAs a tile, and what is left per step is the gates.
+// CUDA cores (64 states: 6.7 ms for 8 x 8192 x 4096, 32 states 3.9 ms); here that work is 20 MMAs a tile, and what is left per
+// step is the gates and a tile's hand-offs: 1.95 and 1.35 ms, 3.8 and 2.6 us a tile.
 // Chunks are 32 steps, half the 16-state kernel's, because the carried rows are four times as wide; two sets of
 // main warps take the even and the odd tiles, so that one set's gates run while the other waits for its MMAs.
 //   warps 0-15   main warps: set s = warp / 8 takes the tiles of its parity, its half g steps [16g, 16g+16), a thread one
@@ -371,7 +372,15 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
           tcd.tile = static_cast<int64_t>(c) * ctiles + x;
           tcd.t0 = c * Q;
           tcd.len = min(Q, p.T - tcd.t0);
-          exact_tile<TA, TG, NSH>(p, tcd, q, half, reinterpret_cast<float*>(smem + SM::off_deep), hc, Pc);
+          // (copies: what a call takes by reference lives in local memory everywhere)
+          const TileCoord at = tcd;
+          float hw[NSH], Pw = Pc;
+#pragma unroll
+          for (int n = 0; n < NSH; ++n) hw[n] = hc[n];
+          exact_tile<TA, TG, NSH>(p, at, q, half, reinterpret_cast<float*>(smem + SM::off_deep), hw, Pw);
+#pragma unroll
+          for (int n = 0; n < NSH; ++n) hc[n] = hw[n];
+          Pc = Pw;
         } else {
           const float P = __frcp_rn(Rend);
 #pragma unroll
