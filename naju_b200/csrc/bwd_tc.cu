@@ -1051,6 +1051,9 @@ int launch_bwd_tc_t(const BwdParams& p, const Geometry& g, const tcb::Maps& maps
   // The exact recurrent backward spreads over time too: 15 us, and 0.3 to 0.39 us per tile of 64 steps x 128 channels on a full
   // GPU or 1.5 us per chunk where the look-back sets the pace.  (Every tile here has its own carry to wait for, 10 us in all.)
   if (cost + 100 > 150 + std::max<int64_t>(7 * g.ntiles / 2, 15 * static_cast<int64_t>(g.nchunks))) return -1000;
+  // The gradients of fp32 logits, and dh0, are fp32, and the two-term operands here are not (6e-5 and 1e-5 against the
+  // recurrent kernel's 2e-6 and 2e-7): with so few channel tiles that the walk alone would not be taken they stay there.
+  if (static_cast<int64_t>(g.B) * g.ndt * 4 < tmah::sm_count() && (std::is_same<TG, float>::value || p.dh0 != nullptr)) return -1000;
   cs_used = best;
   const dim3 grid(static_cast<unsigned>(clusters * best)), block(tcb::NTHREADS);
   return best == 1 ? launch_pdl(walk, grid, block, smem, st, p, maps, fwd_form)
