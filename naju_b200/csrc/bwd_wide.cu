@@ -7,8 +7,8 @@
 //   dC[t,n] = sum_d al[d,t] h[d,n] + sum_{s<=t} M2[t,s] B[s,n]   dB[s,n] = sum_d wt[d,s] lt[d,n] + sum_{t>=s} M2[t,s] C[t,n]
 //   r_t = r_{t+1} + al_t Yt_t - wt_t gt_t,   d f_logit = (1-f_t) r_t,   du = i_t R_t gt_t + D_skip dy_t,   d i_logit = wt_t (1-i_t) gt_t
 //
-// What bounds it: the recurrent kernel does 14 N operations per channel and step on the CUDA cores (64 states: 17 ms for
-// 8 x 8192 x 4096).  Here they are 62 MMAs a tile, and a tile is a chain of phases: gates, MMAs, sweep.  A channel's row is
+// What bounds it: the recurrent kernel does 14 N operations per channel and step on the CUDA cores (64 states: 13.9 ms for
+// 8 x 8192 x 4096, 32 states 11.6 ms; 4.5 and 2.9 ms here).  Here they are 62 MMAs a tile, and a tile is a chain of phases: gates, MMAs, sweep.  A channel's row is
 // [al 32 | wt 32 | h NS | lt NS] in two bf16 terms (al in three where it enters the adjoint of the states, which is
 // carried and returned in fp32): with 64 states 104 KB for 128 channels, so a chunk is 32 steps and there is one set of rows.
 //   warps 0-15   main warps, four threads per channel: group g owns steps [8g, 8g+8) of every chunk, gates and sweep;
@@ -378,21 +378,30 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
     auto post_h = [&](int xx, int c) {
       const int bb = xx / p.ndt, dd = (xx - bb * p.ndt) * kDT + cid;
       const float* src = c >= 0 ? state_row(xx, c) : nullptr;
+      // (64 states: sixteen in flight at a time, 2343 -> 2237 us at B=8, T=4096, D=4096, with the prefetch below; 32 states:
+      // eight, 1477 us against 1514)
+      constexpr int PER = NS == 64 ? 2 : 1;
 #pragma unroll
-      for (int k = 0; k < NSH / 8; ++k) {
-        float v[8];
+      for (int k = 0; k < NSH / 8; k += PER) {
+        float v[PER][8];
         if (c >= 0) {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(src) + 2 * k), e = __ldg(reinterpret_cast<const float4*>(src) + 2 * k + 1);
-          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-          v[4] = e.x; v[5] = e.y; v[6] = e.z; v[7] = e.w;
+          float4 a[2 * PER];
+#pragma unroll
+          for (int j = 0; j < 2 * PER; ++j) a[j] = __ldg(reinterpret_cast<const float4*>(src) + 2 * k + j);
+#pragma unroll
+          for (int j = 0; j < 2 * PER; ++j) {
+            float* o = &v[j >> 1][4 * (j & 1)];
+            o[0] = a[j].x; o[1] = a[j].y; o[2] = a[j].z; o[3] = a[j].w;
+          }
         } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
+          for (int j = 0; j < 8 * PER; ++j) {
             const int n = n0 + 8 * k + j;
-            v[j] = (p.h0 != nullptr && dd < p.D && n < p.N) ? p.h0[(static_cast<int64_t>(bb) * p.D + dd) * p.N + n] : 0.f;
+            v[j >> 3][j & 7] = (p.h0 != nullptr && dd < p.D && n < p.N) ? p.h0[(static_cast<int64_t>(bb) * p.D + dd) * p.N + n] : 0.f;
           }
         }
-        split_chunk(v, SM::R_H1 + k, SM::R_H2 + k);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) split_chunk(v[j], SM::R_H1 + k + j, SM::R_H2 + k + j);
       }
       fence_async_smem();
       mbar_arrive_warp(smem_u32(&bars.h_full));
@@ -420,6 +429,8 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       const int c = nchunks - 1 - ci, t0 = c * Q;
       const uint32_t par = it & 1, st = it & 1, par2 = (it >> 1) & 1;
       const bool more = it + 1 < ntotal;
+      // the states the next tile's h rows come from, towards L2 while there is time
+      if (NS == 64 && c > 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(state_row(x, c - 2)));
       // ---- the chunk's retention product is known: lt rows
       if (!mbar_wait(smem_u32(&bars.rq_ready), par)) timeout();
       const float Rend = s_Rend[cid];
