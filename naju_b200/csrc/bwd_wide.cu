@@ -8,9 +8,11 @@
 //   r_t = r_{t+1} + al_t Yt_t - wt_t gt_t,   d f_logit = (1-f_t) r_t,   du = i_t R_t gt_t + D_skip dy_t,   d i_logit = wt_t (1-i_t) gt_t
 //
 // What bounds it: the recurrent kernel does 14 N operations per channel and step on the CUDA cores (64 states: 13.9 ms for
-// 8 x 8192 x 4096, 32 states 11.6 ms; 4.5 and 2.9 ms here).  Here they are 62 MMAs a tile, and a tile is a chain of phases: gates, MMAs, sweep.  A channel's row is
-// [al 32 | wt 32 | h NS | lt NS] in two bf16 terms (al in three where it enters the adjoint of the states, which is
-// carried and returned in fp32): with 64 states 104 KB for 128 channels, so a chunk is 32 steps and there is one set of rows.
+// 8 x 8192 x 4096, 32 states 11.6 ms; 4.7 and 2.9 ms here).  Here they are MMAs, and a tile is a chain of phases: gates, MMAs, sweep.
+// Every operand is in three bf16 terms, all 24 bits of an fp32 significand, as the recurrent kernel computes in fp32 throughout; of
+// the nine products of two such operands the six that reach 24 bits are taken, the smallest first (an accumulating MMA truncates).
+// A channel's row is [al 32 | wt 32 | h NS | lt NS] three times: with 64 states 147 KB for 128 channels, so a chunk is 32 steps and
+// there is one set of rows.
 //   warps 0-15   main warps, four threads per channel: group g owns steps [8g, 8g+8) of every chunk, gates and sweep;
 //                everything per step stays in registers in between.
 //   warps 16-23  carry warps, two threads per channel with half of the states each: adjoint carry, h and lt rows from the
@@ -29,7 +31,7 @@ namespace wideb {
 
 using namespace tcx;
 
-constexpr int Q = 32, NGRP = 4, SLAB = Q / NGRP, RING = 8, NCARRY = 256;
+constexpr int Q = 32, NGRP = 4, SLAB = Q / NGRP, RING = 4, NCARRY = 256;
 constexpr int W_CARRY = 16, W_BUILD = 24, W_PROD = 25, W_MMA = 26, NTHREADS = 27 * 32;
 static_assert(W_BUILD % 4 == 0, "the builder warp reads accumulator rows 0-31");
 
@@ -40,15 +42,13 @@ struct Maps {
 template <int NS>
 struct Smem {
   static constexpr int NC = NS / 8;
-  // channel row (bf16, chunks of 8)
-  static constexpr int R_A1 = 0, R_W1 = 4, R_H1 = 8, R_L1 = 8 + NC, R_A2 = 8 + 2 * NC, R_W2 = R_A2 + 4, R_H2 = R_A2 + 8,
-                       R_L2 = R_A2 + 8 + NC, R_A3 = 16 + 4 * NC, R_CH = R_A3 + 4;
-  static constexpr uint32_t SBO_R = R_CH * 128, ROWS_BYTES = 16 * SBO_R;
-  static constexpr int BG_C = 0, BG_G1 = NC, BG_G2 = NC + 4;          // rows t: [C NS | g1 32 | g2 32]
-  static constexpr uint32_t SBO_BG = (NC + 8) * 128, BG_BYTES = 4 * SBO_BG;
+  // channel row (bf16, chunks of 8): term k from chunk k * R_TERM on
+  static constexpr int R_A = 0, R_W = 4, R_H = 8, R_L = 8 + NC, R_TERM = 8 + 2 * NC;
+  static constexpr uint32_t SBO_R = 3 * R_TERM * 128, ROWS_BYTES = 16 * SBO_R;
+  static constexpr int BG_C = 0, BG_G = NC;                           // rows t: [C NS | g1 32 | g2 32 | g3 32]
+  static constexpr uint32_t SBO_BG = (NC + 12) * 128, BG_BYTES = 4 * SBO_BG;
   static constexpr uint32_t SBO_BB = NC * 128, BB_BYTES = 4 * SBO_BB;
-  static constexpr int M_1 = 0, M_2 = 4;                              // M2 operand rows t: [m1 32 | m2 32]
-  static constexpr uint32_t SBO_M = 8 * 128, M_BYTES = 4 * SBO_M;
+  static constexpr uint32_t SBO_M = 12 * 128, M_BYTES = 4 * SBO_M;    // M2 operand rows t: [m1 32 | m2 32 | m3 32]
   static constexpr uint32_t BC_BYTES = Q * NS * 2;
   static constexpr uint32_t one = SLAB * kDT * 2, slab_bytes = 4 * one;  // u | f_logit | i_logit | dy
   static constexpr uint32_t off_ring = 0;
@@ -56,11 +56,12 @@ struct Smem {
   // it lies inside shared memory.
   static constexpr uint32_t off_BG = off_ring + RING * slab_bytes;   // [2]
   static constexpr uint32_t off_BB = off_BG + 2 * BG_BYTES;          // [2]
-  static constexpr uint32_t off_bc = off_BB + 2 * BB_BYTES;          // [2 tiles][B raw | C raw]
-  static constexpr uint32_t off_M = off_bc + 4 * BC_BYTES;
+  static constexpr uint32_t off_bc = off_BB + 2 * BB_BYTES;          // [B raw | C raw]
+  static constexpr uint32_t off_M = off_bc + 2 * BC_BYTES;
   static constexpr uint32_t off_rows = off_M + M_BYTES;
   static constexpr uint32_t total = off_rows + ROWS_BYTES;
   static_assert(total + 8192 <= 232448, "with the static arrays, within an SM's 227 KB");
+  static_assert(RING >= NGRP, "a group waits for its slab by parity: the slot's previous use was filled before the group's own previous slab");
   static_assert(off_M >= 4 * 128 && off_M + 16 * SBO_M <= total && off_BG + BG_BYTES + 16 * SBO_BG <= total, "");
   // (dL sits directly before gt: one MMA with the B operand [C | g1] feeds both)
   static constexpr uint32_t TM_Y = 0, TM_DL = 32, TM_G = 32 + NS, TM_GB = 64 + NS, TM_X = 96 + NS, TM_U = TM_X + 32, TM_V = TM_U + NS,
@@ -70,7 +71,7 @@ struct Smem {
 
 struct Bars {
   unsigned long long full[RING], empty[RING];
-  unsigned long long bc_full[2], bc_empty[2];
+  unsigned long long bc_full, bc_empty;
   unsigned long long lprod[NGRP];      // a group's retention product is published          (counts are in warps)
   unsigned long long ssum[NGRP];       // a group's sum of r-increments is published
   unsigned long long part[NGRP];       // a group's operand-row chunks written
@@ -117,8 +118,6 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       mbar_init(smem_u32(&bars.empty[i]), 4);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&bars.bc_full[i]), 1);
-      mbar_init(smem_u32(&bars.bc_empty[i]), 1);
       mbar_init(smem_u32(&bars.seed_ready[i]), NCARRY / 32);
       mbar_init(smem_u32(&bars.ops_full[i]), 1);
       mbar_init(smem_u32(&bars.g_full[i]), 1);
@@ -129,6 +128,8 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       mbar_init(smem_u32(&bars.ssum[i]), 4);
       mbar_init(smem_u32(&bars.part[i]), 4);
     }
+    mbar_init(smem_u32(&bars.bc_full), 1);
+    mbar_init(smem_u32(&bars.bc_empty), 1);
     mbar_init(smem_u32(&bars.rq_ready), 4);
     mbar_init(smem_u32(&bars.h_full), NCARRY / 32);
     mbar_init(smem_u32(&bars.lt_full), NCARRY / 32);
@@ -160,10 +161,10 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       for (int x = x_first; x < ctiles; x += x_step) {
         const int b = x / p.ndt, d0 = (x - b * p.ndt) * kDT;
         for (int ci = 0; ci < nchunks; ++ci, ++it) {
-          const int t0 = (nchunks - 1 - ci) * Q, rb = it & 1;
-          if (it >= 2 && !mbar_wait(smem_u32(&bars.bc_empty[rb]), ((it >> 1) & 1) ^ 1)) timeout();
+          const int t0 = (nchunks - 1 - ci) * Q;
+          if (it >= 1 && !mbar_wait(smem_u32(&bars.bc_empty), (it & 1) ^ 1)) timeout();
           {
-            const uint32_t bar = smem_u32(&bars.bc_full[rb]), dst = sbase + SM::off_bc + rb * 2 * SM::BC_BYTES;
+            const uint32_t bar = smem_u32(&bars.bc_full), dst = sbase + SM::off_bc;
             mbar_arrive_expect_tx(bar, 2 * SM::BC_BYTES);
             tma_load_3d(dst, &maps.bm, 0, t0, b, bar);
             tma_load_3d(dst + SM::BC_BYTES, &maps.cm, 0, t0, b, bar);
@@ -187,8 +188,8 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
     // Trip k builds the shared operands of tile k (one tile ahead of the MMAs), then the M2 operand of tile k-1.
     const int t = lane;
     const uint32_t idG = umma_idesc(128, Q, 1);
-    // row t of a 32 x 32 accumulator block, masked to s <= t, in two bf16 terms
-    auto tril_rows = [&](uint32_t tcol, unsigned char* row, int c_hi, int c_lo) {
+    // row t of a 32 x 32 accumulator block, masked to s <= t, in three bf16 terms of four chunks each
+    auto tril_rows = [&](uint32_t tcol, unsigned char* row) {
 #pragma unroll
       for (int c16 = 0; c16 < 2; ++c16) {
         uint32_t x[16];
@@ -198,15 +199,15 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         for (int h = 0; h < 2; ++h) {
           const int c8 = 2 * c16 + h;
           if (c8 <= (t >> 3)) {
-            uint32_t hi[4], lo[4];
+            uint32_t v[3][4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int s = 8 * c8 + 2 * k;
-              split_pair(make_float2(s <= t ? __uint_as_float(x[8 * h + 2 * k]) : 0.f,
-                                     s + 1 <= t ? __uint_as_float(x[8 * h + 2 * k + 1]) : 0.f), hi[k], lo[k]);
+              split3(make_float2(s <= t ? __uint_as_float(x[8 * h + 2 * k]) : 0.f,
+                                 s + 1 <= t ? __uint_as_float(x[8 * h + 2 * k + 1]) : 0.f), v[0][k], v[1][k], v[2][k]);
             }
-            *reinterpret_cast<uint4*>(row + (c_hi + c8) * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(row + (c_lo + c8) * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(row + (4 * k + c8) * 128) = make_uint4(v[k][0], v[k][1], v[k][2], v[k][3]);
           }
         }
         __syncwarp();
@@ -216,12 +217,12 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       if (it < ntotal) {
         const int st = it & 1;
         const uint32_t par = (it >> 1) & 1;
-        if (!mbar_wait(smem_u32(&bars.bc_full[st]), par)) timeout();
+        if (!mbar_wait(smem_u32(&bars.bc_full), it & 1)) timeout();
         // every MMA of the tile two back that reads BG / BB (or the M2 operand) is complete
         if (it >= 2 && !mbar_wait(smem_u32(&bars.d5_full[st]), par ^ 1)) timeout();
         unsigned char* s_BG = smem + SM::off_BG + st * SM::BG_BYTES;
         unsigned char* s_BB = smem + SM::off_BB + st * SM::BB_BYTES;
-        const unsigned char* raw = smem + SM::off_bc + st * 2 * SM::BC_BYTES;
+        const unsigned char* raw = smem + SM::off_bc;
 #pragma unroll 4
         for (int i = lane; i < Q * SM::NC; i += 32) {
           const int r = i / SM::NC, k = i % SM::NC;
@@ -234,7 +235,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         __syncwarp();
         if (lane == 0) {
           tc_fence_after();
-          mbar_arrive(smem_u32(&bars.bc_empty[st]));  // the raw rows have been read
+          mbar_arrive(smem_u32(&bars.bc_empty));  // the raw rows have been read
           const uint64_t dC = umma_desc(sbase + SM::off_BG + st * SM::BG_BYTES, 128, SM::SBO_BG),
                          dB = umma_desc(sbase + SM::off_BB + st * SM::BB_BYTES, 128, SM::SBO_BB);
 #pragma unroll
@@ -245,7 +246,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         if (!mbar_wait(smem_u32(&bars.g_full[st]), par)) timeout();
         __syncwarp();
         tc_fence_after();
-        tril_rows(tmem + SM::TM_GB, s_BG + static_cast<uint32_t>(t >> 3) * SM::SBO_BG + static_cast<uint32_t>(t & 7) * 16, SM::BG_G1, SM::BG_G2);
+        tril_rows(tmem + SM::TM_GB, s_BG + static_cast<uint32_t>(t >> 3) * SM::SBO_BG + static_cast<uint32_t>(t & 7) * 16 + SM::BG_G * 128);
         fence_async_smem();
         tc_fence_before();
         mbar_arrive_warp(smem_u32(&bars.ops_full[st]));
@@ -255,7 +256,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         if (!mbar_wait(smem_u32(&bars.d4_full), (it - 1) & 1)) timeout();
         __syncwarp();
         tc_fence_after();
-        tril_rows(tmem + SM::TM_X, smem + SM::off_M + static_cast<uint32_t>(t >> 3) * SM::SBO_M + static_cast<uint32_t>(t & 7) * 16, SM::M_1, SM::M_2);
+        tril_rows(tmem + SM::TM_X, smem + SM::off_M + static_cast<uint32_t>(t >> 3) * SM::SBO_M + static_cast<uint32_t>(t & 7) * 16);
         fence_async_smem();
         tc_fence_before();
         mbar_arrive_warp(smem_u32(&bars.m2_full));
@@ -278,73 +279,91 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         const int st = it & 1;
         const uint32_t par = it & 1, par2 = (it >> 1) & 1;
         const uint32_t aBG = sbase + SM::off_BG + st * SM::BG_BYTES, aBB = sbase + SM::off_BB + st * SM::BB_BYTES;
-        const uint64_t dGk = umma_desc(aBG, 128, SM::SBO_BG), dGm = umma_desc(aBG, SM::SBO_BG, 128);   // C | g1 | g2
+        const uint64_t dGk = umma_desc(aBG, 128, SM::SBO_BG), dGm = umma_desc(aBG, SM::SBO_BG, 128);   // C | g1 | g2 | g3
         const uint64_t dBk = umma_desc(aBB, 128, SM::SBO_BB), dBm = umma_desc(aBB, SM::SBO_BB, 128);   // B rows
         if (!mbar_wait(smem_u32(&bars.ops_full[st]), par2)) timeout();
         if (it >= 1 && !mbar_wait(smem_u32(&bars.acc_free), par ^ 1)) timeout();
         if (!mbar_wait(smem_u32(&bars.h_full), par)) timeout();
         tc_fence_after();
-        // Yt = (h1 + h2).C   (K = n)
+        // chunk `c` of term `k` of the channel rows / of g
+        auto row = [](int k, int c) { return static_cast<uint32_t>(k * SM::R_TERM + c) * 128; };
+        auto gch = [](int k, int c) { return static_cast<uint32_t>(SM::BG_G + 4 * k + c) * 128; };
+        // Yt = (h1 + h2 + h3).C   (K = n)
 #pragma unroll
-        for (int k = 0; k < NS / 16; ++k) {
-          umma_bf16(tmem + SM::TM_Y, dRk + off((SM::R_H1 + 2 * k) * 128), dGk + off((SM::BG_C + 2 * k) * 128), iKK, k > 0);
-          umma_bf16(tmem + SM::TM_Y, dRk + off((SM::R_H2 + 2 * k) * 128), dGk + off((SM::BG_C + 2 * k) * 128), iKK, 1u);
-        }
+        for (int k = 2; k >= 0; --k)
+#pragma unroll
+          for (int ks = 0; ks < NS / 16; ++ks)
+            umma_bf16(tmem + SM::TM_Y, dRk + off(row(k, SM::R_H + 2 * ks)), dGk + off((SM::BG_C + 2 * ks) * 128), iKK, k < 2 || ks > 0);
         for (int g = 0; g < NGRP; ++g)
           if (!mbar_wait(smem_u32(&bars.part[g]), par)) timeout();
         tc_fence_after();
-        // [dL | gt] += (al1 + al2).[C | g1]^T,  gt += al1.g2^T,  dL += al3.C^T   (K = t), the small terms first: the accumulator
-        // truncates, and dL carries the adjoint
-        uint32_t acc = 0;
+        // dL += (al1 + al2 + al3).C and gt += the products of al and g^T, those with g1 in one instruction with dL's: [dL | gt] += al.[C | g1]
+        auto al_cg = [&](int k) {
 #pragma unroll
-        for (int ks = 0; ks < Q / 16; ++ks, acc = 1u)
-          umma_bf16(tmem + SM::TM_DL, dRk + off((SM::R_A3 + 2 * ks) * 128), dGm + off(2 * ks * SM::SBO_BG), iKMc, acc);
+          for (int ks = 0; ks < Q / 16; ++ks)
+            umma_bf16(tmem + SM::TM_DL, dRk + off(row(k, SM::R_A + 2 * ks)), dGm + off(2 * ks * SM::SBO_BG), iKMc, k < 2 || ks > 0);
+        };
+        auto al_g = [&](int k, int j) {
 #pragma unroll
-        for (int ks = 0; ks < Q / 16; ++ks)
-          umma_bf16(tmem + SM::TM_DL, dRk + off((SM::R_A2 + 2 * ks) * 128), dGm + off(2 * ks * SM::SBO_BG), iKMc, 1u);
+          for (int ks = 0; ks < Q / 16; ++ks)
+            umma_bf16(tmem + SM::TM_G, dRk + off(row(k, SM::R_A + 2 * ks)), dGm + off(2 * ks * SM::SBO_BG + gch(j, 0)), iKM, 1u);
+        };
+        // Yt += the products of wt and g   (K = s)
+        auto w_g = [&](int k, int j) {
 #pragma unroll
-        for (int ks = 0; ks < Q / 16; ++ks) {
-          umma_bf16(tmem + SM::TM_DL, dRk + off((SM::R_A1 + 2 * ks) * 128), dGm + off(2 * ks * SM::SBO_BG), iKMc, 1u);
-          umma_bf16(tmem + SM::TM_G, dRk + off((SM::R_A1 + 2 * ks) * 128), dGm + off(2 * ks * SM::SBO_BG + SM::BG_G2 * 128), iKM, 1u);
-          // Yt += w1.g1 + w1.g2 + w2.g1   (K = s)
-          const uint64_t g1 = dGk + off((SM::BG_G1 + 2 * ks) * 128), g2 = dGk + off((SM::BG_G2 + 2 * ks) * 128);
-          umma_bf16(tmem + SM::TM_Y, dRk + off((SM::R_W1 + 2 * ks) * 128), g1, iKK, 1u);
-          umma_bf16(tmem + SM::TM_Y, dRk + off((SM::R_W1 + 2 * ks) * 128), g2, iKK, 1u);
-          umma_bf16(tmem + SM::TM_Y, dRk + off((SM::R_W2 + 2 * ks) * 128), g1, iKK, 1u);
-        }
-        // gt += (l1 + l2).B   (K = n)
+          for (int ks = 0; ks < Q / 16; ++ks)
+            umma_bf16(tmem + SM::TM_Y, dRk + off(row(k, SM::R_W + 2 * ks)), dGk + off(gch(j, 2 * ks)), iKK, 1u);
+        };
+        al_cg(2);
+        al_g(0, 2);
+        al_g(1, 1);
+        w_g(2, 0);
+        w_g(0, 2);
+        w_g(1, 1);
+        al_cg(1);
+        al_g(0, 1);
+        w_g(1, 0);
+        w_g(0, 1);
+        al_cg(0);
+        w_g(0, 0);
+        // gt += (l1 + l2 + l3).B   (K = n)
         if (!mbar_wait(smem_u32(&bars.lt_full), par)) timeout();
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < NS / 16; ++k) {
-          umma_bf16(tmem + SM::TM_G, dRk + off((SM::R_L1 + 2 * k) * 128), dBk + off(2 * k * 128), iKK, 1u);
-          umma_bf16(tmem + SM::TM_G, dRk + off((SM::R_L2 + 2 * k) * 128), dBk + off(2 * k * 128), iKK, 1u);
-        }
+        for (int k = 2; k >= 0; --k)
+#pragma unroll
+          for (int ks = 0; ks < NS / 16; ++ks)
+            umma_bf16(tmem + SM::TM_G, dRk + off(row(k, SM::R_L + 2 * ks)), dBk + off(2 * ks * 128), iKK, 1u);
         umma_commit(smem_u32(&bars.d1_full));  // the reverse sweep can start
         // cross-channel: X += [al | wt]^T . [wt | h | lt]   (K = 16 channels per step), once the previous tile's second-round
         // results, which lie in the same columns, have been read
         if (it >= 1 && !mbar_wait(smem_u32(&bars.x_free), par ^ 1)) timeout();
         tc_fence_after();
+        auto cross = [&](int k, int j, bool first) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t grp = dRm + off(2 * ks * SM::SBO_R);
-          umma_bf16(tmem + SM::TM_X, grp + off(SM::R_A1 * 128), grp + off(SM::R_W1 * 128), iMMx, ks > 0);
-          umma_bf16(tmem + SM::TM_X, grp + off(SM::R_A1 * 128), grp + off(SM::R_W2 * 128), iMMx, 1u);
-          umma_bf16(tmem + SM::TM_X, grp + off(SM::R_A2 * 128), grp + off(SM::R_W1 * 128), iMMx, 1u);
-        }
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16(tmem + SM::TM_X, dRm + off(2 * ks * SM::SBO_R + row(k, SM::R_A)), dRm + off(2 * ks * SM::SBO_R + row(j, SM::R_W)), iMMx,
+                      !first || ks > 0);
+        };
+        cross(2, 0, true);
+        cross(0, 2, false);
+        cross(1, 1, false);
+        cross(1, 0, false);
+        cross(0, 1, false);
+        cross(0, 0, false);
         umma_commit(smem_u32(&bars.d4_full));
         // second round, onto U (accumulator rows 0-31: steps) and V (rows 32-63)
         if (!mbar_wait(smem_u32(&bars.m2_full), par)) timeout();
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < Q / 16; ++ks) {
-          // dC[t,n] += sum_s M2[t,s] B[s,n]
-          umma_bf16(tmem + SM::TM_U, dMk + off((SM::M_1 + 2 * ks) * 128), dBm + off(2 * ks * SM::SBO_BB), iKMn, 1u);
-          umma_bf16(tmem + SM::TM_U, dMk + off((SM::M_2 + 2 * ks) * 128), dBm + off(2 * ks * SM::SBO_BB), iKMn, 1u);
-          // dB[32+s,n] += sum_t M2[t,s] C[t,n]
-          umma_bf16(tmem + SM::TM_V, dMm + off(2 * ks * SM::SBO_M + SM::M_1 * 128), dGm + off(2 * ks * SM::SBO_BG), iMMn, 1u);
-          umma_bf16(tmem + SM::TM_V, dMm + off(2 * ks * SM::SBO_M + SM::M_2 * 128), dGm + off(2 * ks * SM::SBO_BG), iMMn, 1u);
-        }
+        for (int k = 2; k >= 0; --k)
+#pragma unroll
+          for (int ks = 0; ks < Q / 16; ++ks) {
+            // dC[t,n] += sum_s M2[t,s] B[s,n]
+            umma_bf16(tmem + SM::TM_U, dMk + off((4 * k + 2 * ks) * 128), dBm + off(2 * ks * SM::SBO_BB), iKMn, 1u);
+            // dB[32+s,n] += sum_t M2[t,s] C[t,n]
+            umma_bf16(tmem + SM::TM_V, dMm + off(2 * ks * SM::SBO_M + 4 * k * 128), dGm + off(2 * ks * SM::SBO_BG), iMMn, 1u);
+          }
         umma_commit(smem_u32(&bars.d5_full[st]));
       }
     }
@@ -355,12 +374,12 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
     unsigned char* my_row = smem + SM::off_rows + static_cast<uint32_t>(cid >> 3) * SM::SBO_R + static_cast<uint32_t>(cid & 7) * 16 +
                             half * (NSH / 8) * 128;
     float lam[NSH];   // adjoint entering the current chunk from the future
-    auto split_chunk = [&](const float (&v)[8], int c_hi, int c_lo) {
-      uint32_t hi[4], lo[4];
+    auto split_chunk = [&](const float (&v)[8], int c) {
+      uint32_t o[3][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) split_pair(make_float2(v[2 * j], v[2 * j + 1]), hi[j], lo[j]);
-      *reinterpret_cast<uint4*>(my_row + c_hi * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(my_row + c_lo * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      for (int j = 0; j < 4; ++j) split3(make_float2(v[2 * j], v[2 * j + 1]), o[0][j], o[1][j], o[2][j]);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(my_row + (k * SM::R_TERM + c) * 128) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
     };
     auto state_row = [&](int xx, int c) { return p.ckS + ((static_cast<int64_t>(c) * ctiles + xx) * kDT + cid) * NS + n0; };
     // this thread's share of <lam, state at the end of chunk c of channel tile xx>
@@ -401,7 +420,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
           }
         }
 #pragma unroll
-        for (int j = 0; j < PER; ++j) split_chunk(v[j], SM::R_H1 + k + j, SM::R_H2 + k + j);
+        for (int j = 0; j < PER; ++j) split_chunk(v[j], SM::R_H + k + j);
       }
       fence_async_smem();
       mbar_arrive_warp(smem_u32(&bars.h_full));
@@ -444,7 +463,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
           lam[8 * k + j] *= PQ;
           v[j] = lam[8 * k + j];
         }
-        split_chunk(v, SM::R_L1 + k, SM::R_L2 + k);
+        split_chunk(v, SM::R_L + k);
       }
       fence_async_smem();
       mbar_arrive_warp(smem_u32(&bars.lt_full));
@@ -584,10 +603,8 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
           const float2 dy2 = make_float2(ld_as_f32(s_dy, (2 * j2) * kDT), ld_as_f32(s_dy, (2 * j2 + 1) * kDT));
           const float2 R = mul2(Rs2, L[j2]);
           const float2 Rprev = make_float2(j2 == 0 ? Rstart : Rstart * L[j2 == 0 ? 0 : j2 - 1].y, R.x);
-          const float2 x2 = mul2(R, opb);
-          const float2 r = make_float2(fast_rcp(x2.x), fast_rcp(x2.y));
-          const float2 P = mul2(opb, r);                          // 1 / R_t
-          const float2 ig = mul2(R, r);                           // i_t
+          const float2 P = make_float2(fast_rcp(R.x), fast_rcp(R.y));          // 1 / R_t
+          const float2 ig = make_float2(fast_rcp(opb.x), fast_rcp(opb.y));     // i_t
           cu[j2] = mul2(ig, R);                                   // i_t R_t
           wtr[j2] = mul2(u2, cu[j2]);
           alr[j2] = mul2(dy2, P);
@@ -600,17 +617,15 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         // the channel rows are free once every MMA of the previous tile that reads them is complete
         if (it >= 1 && !mbar_wait(smem_u32(&bars.d4_full), par ^ 1)) timeout();
         {
-          uint32_t a1[H], a2[H], a3[H], w1[H], w2[H];
+          auto put = [&](const float2 (&v)[H], int c) {
+            uint32_t o[3][H];
 #pragma unroll
-          for (int j2 = 0; j2 < H; ++j2) {
-            split3(alr[j2], a1[j2], a2[j2], a3[j2]);
-            split_pair(wtr[j2], w1[j2], w2[j2]);
-          }
-          *reinterpret_cast<uint4*>(my_row + (SM::R_A1 + grp) * 128) = make_uint4(a1[0], a1[1], a1[2], a1[3]);
-          *reinterpret_cast<uint4*>(my_row + (SM::R_A2 + grp) * 128) = make_uint4(a2[0], a2[1], a2[2], a2[3]);
-          *reinterpret_cast<uint4*>(my_row + (SM::R_A3 + grp) * 128) = make_uint4(a3[0], a3[1], a3[2], a3[3]);
-          *reinterpret_cast<uint4*>(my_row + (SM::R_W1 + grp) * 128) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-          *reinterpret_cast<uint4*>(my_row + (SM::R_W2 + grp) * 128) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+            for (int j2 = 0; j2 < H; ++j2) split3(v[j2], o[0][j2], o[1][j2], o[2][j2]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(my_row + (k * SM::R_TERM + c + grp) * 128) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+          };
+          put(alr, SM::R_A);
+          put(wtr, SM::R_W);
         }
         fence_async_smem();
         tc_fence_before();

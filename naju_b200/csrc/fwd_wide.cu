@@ -4,13 +4,13 @@
 //     y_t   = P_t [ <C_t, h> + sum_{s<=t} (C_t . B_s) wt_s ] + D_skip u_t,   wt_s = sigmoid(i_s) u_s / P_s
 //     x_end = P_Q [ h + sum_s wt_s B_s ]
 // as GEMMs with M = 128 channels (bf16 operands, fp32 accumulators in TMEM):
-//     D2[128 x NS] = (w1 + w2 + w3) . B^T                    chunk-local state increment
-//     D1[128 x 32] = w1.g1 + w1.g2 + w2.g1 + (h1 + h2).C     pre-scaled outputs (stored in 16 bits)
-// with wt = w1 + w2 + w3 to 24 bits where it enters the states, which are kept, checkpointed and returned in fp32,
-// and to 16 bits (2^-16 relative) where it enters y.
+//     D2[128 x NS] = (w1 + w2 + w3) . B^T                                                   chunk-local state increment
+//     D1[128 x 32] = sum of w_i . g_j, i + j <= 4, + (h1 + h2 + h3) . C                     pre-scaled outputs
+// with wt, tril(C B^T) = g and h in three bf16 terms each, all 24 bits of an fp32 significand: these problems are the recurrent
+// kernels' otherwise, whose arithmetic is fp32 throughout.  (Two-term operands, 16 bits, showed through y's rounding to 16 bits.)
 //
 // What bounds it: the recurrent kernel does N multiply-adds and N loads' worth of B and C per channel and step on the
-// CUDA cores (64 states: 6.7 ms for 8 x 8192 x 4096, 32 states 3.9 ms); here that work is 20 MMAs a tile, and what is left per
+// CUDA cores (64 states: 6.7 ms for 8 x 8192 x 4096, 32 states 3.9 ms); here that work is MMAs, and what is left per
 // step is the gates and a tile's hand-offs: 1.95 and 1.35 ms, 3.8 and 2.6 us a tile.
 // Chunks are 32 steps, half the 16-state kernel's, because the carried rows are four times as wide; two sets of
 // main warps take the even and the odd tiles, so that one set's gates run while the other waits for its MMAs.
@@ -46,10 +46,10 @@ struct Maps {
 template <typename TG, int NS>
 struct Smem {
   static constexpr int NC = NS / 8;                                  // 16-byte chunks of a state row
-  static constexpr int AH_H1 = 0, AH_H2 = NC;                        // carry-in rows [h1 NS | h2 NS]
-  static constexpr uint32_t SBO_AH = 2 * NC * 128, AH_BYTES = 16 * SBO_AH;
-  static constexpr int B1_C = 0, B1_G1 = NC, B1_G2 = NC + 4;         // rows t: [C NS | g1 32 | g2 32]
-  static constexpr uint32_t SBO_B1 = (NC + 8) * 128, B1_BYTES = 4 * SBO_B1;
+  static constexpr int AH_H1 = 0, AH_H2 = NC, AH_H3 = 2 * NC;        // carry-in rows [h1 NS | h2 NS | h3 NS]
+  static constexpr uint32_t SBO_AH = 3 * NC * 128, AH_BYTES = 16 * SBO_AH;
+  static constexpr int B1_C = 0, B1_G1 = NC, B1_G2 = NC + 4, B1_G3 = NC + 8;   // rows t: [C NS | g1 32 | g2 32 | g3 32]
+  static constexpr uint32_t SBO_B1 = (NC + 12) * 128, B1_BYTES = 4 * SBO_B1;
   static constexpr uint32_t SBO_BB = NC * 128, BB_BYTES = 4 * SBO_BB;  // rows s: [B NS]
   static constexpr uint32_t BC_BYTES = Q * NS * 2;
   static constexpr uint32_t slab_bytes = SLAB * kDT * (2 + 2 * sizeof(TG));
@@ -61,11 +61,14 @@ struct Smem {
   static constexpr uint32_t off_bc = off_BB + 2 * BB_BYTES;            // [2 tiles][B raw | C raw]
   static constexpr uint32_t off_AH = off_bc + 4 * BC_BYTES;
   static constexpr uint32_t off_AW = off_AH + AH_BYTES;                // [2]
-  static constexpr uint32_t off_deep = off_AW + 2 * AW_BYTES;          // [Q][128] fp32: deep-gate tiles only
-  static constexpr uint32_t total = off_deep + Q * kDT * 4;
+  static constexpr uint32_t total = off_AW + 2 * AW_BYTES;
+  static_assert(Q * kDT * 4 <= AW_BYTES, "a tile taken by the exact path uses its own operand rows as scratch");
+  static_assert(RING >= 4, "a half waits for its slab by parity: the slot's previous use was filled before the half's own previous slab");
   static_assert(total + 4096 <= 232448, "with the static arrays, within an SM's 227 KB");
   static_assert(off_B1 + B1_BYTES + 16 * SBO_B1 <= total, "the 128-row view of a stage's C rows stays inside shared memory");
-  static constexpr uint32_t TM_D1 = 0, TM_D2 = 32, TM_G = 32 + NS, TM_STAGE = 64 + NS, TMEM_COLS = 256;
+  // (D2's largest term has an accumulator of its own, see the MMA issuer)
+  static constexpr uint32_t TM_D1 = 0, TM_D2 = 32, TM_D2S = 32 + NS, TM_G = 32 + 2 * NS, TM_STAGE = 64 + 2 * NS,
+                            TMEM_COLS = NS == 64 ? 512 : 256;
   static_assert(2 * TM_STAGE <= TMEM_COLS, "");
 };
 
@@ -251,15 +254,16 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         for (int h = 0; h < 2; ++h) {
           const int c8 = 2 * c16 + h;
           if (c8 <= (t >> 3)) {
-            uint32_t hi[4], lo[4];
+            uint32_t g1[4], g2[4], g3[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int s = 8 * c8 + 2 * k;
-              split_pair(make_float2(s <= t ? __uint_as_float(x[8 * h + 2 * k]) : 0.f,
-                                     s + 1 <= t ? __uint_as_float(x[8 * h + 2 * k + 1]) : 0.f), hi[k], lo[k]);
+              split3(make_float2(s <= t ? __uint_as_float(x[8 * h + 2 * k]) : 0.f,
+                                 s + 1 <= t ? __uint_as_float(x[8 * h + 2 * k + 1]) : 0.f), g1[k], g2[k], g3[k]);
             }
-            *reinterpret_cast<uint4*>(row + (SM::B1_G1 + c8) * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(row + (SM::B1_G2 + c8) * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<uint4*>(row + (SM::B1_G1 + c8) * 128) = make_uint4(g1[0], g1[1], g1[2], g1[3]);
+            *reinterpret_cast<uint4*>(row + (SM::B1_G2 + c8) * 128) = make_uint4(g2[0], g2[1], g2[2], g2[3]);
+            *reinterpret_cast<uint4*>(row + (SM::B1_G3 + c8) * 128) = make_uint4(g3[0], g3[1], g3[2], g3[3]);
           }
         }
       }
@@ -288,29 +292,37 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         if (!mbar_wait(smem_u32(&bars.part[st][0]), par)) timeout();
         if (!mbar_wait(smem_u32(&bars.part[st][1]), par)) timeout();
         tc_fence_after();
-        // D2: the small terms first (the accumulator truncates: adding them last doubled the states' error)
-#pragma unroll
-        for (int term = 2; term >= 0; --term)
-#pragma unroll
-          for (int ks = 0; ks < NSLAB; ++ks)
-            umma_bf16(tst + SM::TM_D2, dAW + off((4 * term + 2 * ks) * 128), dBB + off(2 * ks * SM::SBO_BB), idN, term < 2 || ks > 0);
-        umma_commit(smem_u32(&bars.d2_full[st]));
+        // D2: the small terms in an accumulator of their own, added up by the carry warps.  (An accumulating MMA truncates;
+        // w1 . B alone hardly has bits to lose.)
 #pragma unroll
         for (int ks = 0; ks < NSLAB; ++ks) {
-          const uint64_t w1 = dAW + off((AW_W1 + 2 * ks) * 128), w2 = dAW + off((AW_W2 + 2 * ks) * 128);
-          const uint64_t g1 = dB1 + off((SM::B1_G1 + 2 * ks) * 128), g2 = dB1 + off((SM::B1_G2 + 2 * ks) * 128);
-          umma_bf16(tst + SM::TM_D1, w1, g1, id32, ks > 0);
-          umma_bf16(tst + SM::TM_D1, w1, g2, id32, 1u);
-          umma_bf16(tst + SM::TM_D1, w2, g1, id32, 1u);
+          const uint64_t bb = dBB + off(2 * ks * SM::SBO_BB);
+          umma_bf16(tst + SM::TM_D2S, dAW + off((AW_W3 + 2 * ks) * 128), bb, idN, ks > 0);
+          umma_bf16(tst + SM::TM_D2, dAW + off((AW_W1 + 2 * ks) * 128), bb, idN, ks > 0);
         }
-        // (the accumulators of a deep-gate tile are junk and are never read)
+#pragma unroll
+        for (int ks = 0; ks < NSLAB; ++ks) umma_bf16(tst + SM::TM_D2S, dAW + off((AW_W2 + 2 * ks) * 128), dBB + off(2 * ks * SM::SBO_BB), idN, 1u);
+        umma_commit(smem_u32(&bars.d2_full[st]));
+        // D1: the products of terms that reach 24 bits, the smallest first
+        auto wg = [&](int w, int g, bool first) {
+#pragma unroll
+          for (int ks = 0; ks < NSLAB; ++ks)
+            umma_bf16(tst + SM::TM_D1, dAW + off((w + 2 * ks) * 128), dB1 + off((g + 2 * ks) * 128), id32, !first || ks > 0);
+        };
+        wg(AW_W3, SM::B1_G1, true);
+        wg(AW_W1, SM::B1_G3, false);
+        wg(AW_W2, SM::B1_G2, false);
+        wg(AW_W2, SM::B1_G1, false);
+        wg(AW_W1, SM::B1_G2, false);
+        wg(AW_W1, SM::B1_G1, false);
+        // (the accumulators of a tile that the exact path takes are junk and are never read)
         if (!mbar_wait(smem_u32(&bars.h_ready), it & 1)) timeout();
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < NS / 16; ++k) {
-          umma_bf16(tst + SM::TM_D1, dAH + off((SM::AH_H1 + 2 * k) * 128), dB1 + off((SM::B1_C + 2 * k) * 128), id32, 1u);
-          umma_bf16(tst + SM::TM_D1, dAH + off((SM::AH_H2 + 2 * k) * 128), dB1 + off((SM::B1_C + 2 * k) * 128), id32, 1u);
-        }
+        for (int term = 2; term >= 0; --term)
+#pragma unroll
+          for (int k = 0; k < NS / 16; ++k)
+            umma_bf16(tst + SM::TM_D1, dAH + off((term * SM::NC + 2 * k) * 128), dB1 + off((SM::B1_C + 2 * k) * 128), id32, 1u);
         umma_commit(smem_u32(&bars.d1_full[st]));
       }
     }
@@ -324,12 +336,13 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
     auto write_h_row = [&]() {
 #pragma unroll
       for (int k = 0; k < NSH / 8; ++k) {
-        uint32_t hi[4], lo[4];
+        uint32_t h1[4], h2[4], h3[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) split_pair(make_float2(hc[8 * k + 2 * j], hc[8 * k + 2 * j + 1]), hi[j], lo[j]);
+        for (int j = 0; j < 4; ++j) split3(make_float2(hc[8 * k + 2 * j], hc[8 * k + 2 * j + 1]), h1[j], h2[j], h3[j]);
         const int ch = half * (NSH / 8) + k;
-        *reinterpret_cast<uint4*>(h_row + (SM::AH_H1 + ch) * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(h_row + (SM::AH_H2 + ch) * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(h_row + (SM::AH_H1 + ch) * 128) = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+        *reinterpret_cast<uint4*>(h_row + (SM::AH_H2 + ch) * 128) = make_uint4(h2[0], h2[1], h2[2], h2[3]);
+        *reinterpret_cast<uint4*>(h_row + (SM::AH_H3 + ch) * 128) = make_uint4(h3[0], h3[1], h3[2], h3[3]);
       }
       fence_async_smem();
       tc_fence_before();
@@ -377,45 +390,49 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
           float hw[NSH], Pw = Pc;
 #pragma unroll
           for (int n = 0; n < NSH; ++n) hw[n] = hc[n];
-          exact_tile<TA, TG, NSH>(p, at, q, half, reinterpret_cast<float*>(smem + SM::off_deep), hw, Pw);
+          if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();   // the operand rows are scratch now
+          exact_tile<TA, TG, NSH>(p, at, q, half, reinterpret_cast<float*>(smem + SM::off_AW + st * AW_BYTES), hw, Pw);
 #pragma unroll
           for (int n = 0; n < NSH; ++n) hc[n] = hw[n];
           Pc = Pw;
         } else {
-          const float P = __frcp_rn(Rend);
+          const float P = __frcp_rn(Rend), Pl = P * fmaf(-P, Rend, 1.f);   // (P + Pl = 1 / Rend)
 #pragma unroll
-          for (int k = 0; k < NSH / 16; ++k) {
-            uint32_t sr[16];
-            tmem_ld16_async(tmem + st * SM::TM_STAGE + lane_off + SM::TM_D2 + n0 + 16 * k, sr);
-            tmem_ld_wait16(sr);
+          for (int k = 0; k < NSH / 8; ++k) {
+            uint32_t sr[8], ss[8];
+            tmem_ld8_async(tmem + st * SM::TM_STAGE + lane_off + SM::TM_D2 + n0 + 8 * k, sr);
+            tmem_ld8_async(tmem + st * SM::TM_STAGE + lane_off + SM::TM_D2S + n0 + 8 * k, ss);
+            tmem_ld_wait8(sr, ss);
 #pragma unroll
-            for (int n = 0; n < 16; ++n) hc[16 * k + n] = P * (hc[16 * k + n] + __uint_as_float(sr[n]));
+            for (int n = 0; n < 8; ++n)
+              hc[8 * k + n] = fmaf(P, __uint_as_float(sr[n]), fmaf(P, __uint_as_float(ss[n]), fmaf(Pl, __uint_as_float(sr[n]), P * hc[8 * k + n])));
           }
           Pc *= P;
         }
         tc_fence_before();
         mbar_arrive_warp(smem_u32(&bars.acc_free[st]));
+        // this tile's MMAs have read the carry-in row: the next tile's, which they wait for, before anything else
+        if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();
+        if (c + 1 < nchunks) write_h_row();
         // the chunk-end state: checkpoint, the last chunk's also the final state
         const int64_t slot = (static_cast<int64_t>(c) * ctiles + x) * kDT + q;
         float4* dstS = reinterpret_cast<float4*>(p.ckS + slot * NS + n0);
 #pragma unroll
         for (int k = 0; k < NSH / 4; ++k) dstS[k] = make_float4(hc[4 * k], hc[4 * k + 1], hc[4 * k + 2], hc[4 * k + 3]);
         if (half == 0) p.ckP[slot] = Pc;
-        if (c == nchunks - 1 && tcd.d_ok) {
-          const int64_t ch = static_cast<int64_t>(tcd.b) * p.D + tcd.d;
-          if (p.hT != nullptr)
-#pragma unroll
-            for (int n = 0; n < NSH; ++n)
-              if (n0 + n < p.N) p.hT[ch * p.N + n0 + n] = hc[n];
-          if (p.pT != nullptr && half == 0) p.pT[ch] = Pc;
-        }
-        if (!mbar_wait(smem_u32(&bars.d1_full[st]), par)) timeout();
-        // this tile's MMAs have read the carry-in row: the next tile's
         if (c + 1 == nchunks) {
+          if (tcd.d_ok) {
+            const int64_t ch = static_cast<int64_t>(tcd.b) * p.D + tcd.d;
+            if (p.hT != nullptr)
+#pragma unroll
+              for (int n = 0; n < NSH; ++n)
+                if (n0 + n < p.N) p.hT[ch * p.N + n0 + n] = hc[n];
+            if (p.pT != nullptr && half == 0) p.pT[ch] = Pc;
+          }
           if (x + x_step >= ctiles) continue;
           load_h0(x + x_step);
+          write_h_row();
         }
-        write_h_row();
       }
     }
   } else if (warp < W_CARRY) {
@@ -488,10 +505,12 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
           const float2 opb = add2(make_float2(fast_ex2(il2.x), fast_ex2(il2.y)), one2);   // 1 / i_t
           uv[j2] = UTM ? ld_pair_as_f32(s_ut + 2 * j2) : make_float2(ld_as_f32(s_u, (2 * j2) * kDT), ld_as_f32(s_u, (2 * j2 + 1) * kDT));
           const float2 R = mul2(Rs2, L[j2]);
-          const float2 x2 = mul2(R, opb);
-          const float2 r = make_float2(fast_rcp(x2.x), fast_rcp(x2.y));
-          Pv[j2] = mul2(opb, r);                                        // P_t = 1 / R_t
-          split3(mul2(uv[j2], mul2(mul2(R, r), R)), w1[jj], w2[jj], w3[jj]);   // u_t i_t R_t
+          Pv[j2] = make_float2(fast_rcp(R.x), fast_rcp(R.y));           // P_t = 1 / R_t
+          // (u_t i_t R_t; the reciprocal's last bit goes into the product: the final state's error against 64 bits stays the recurrent
+          // kernel's with it)
+          const float2 ig = make_float2(fast_rcp(opb.x), fast_rcp(opb.y)), iR = mul2(ig, R);
+          const float2 w = mul2(uv[j2], fma2(iR, fma2(make_float2(-opb.x, -opb.y), ig, one2), iR));
+          split3(w, w1[jj], w2[jj], w3[jj]);
         }
         const int ch = 2 * g + j8;
         *reinterpret_cast<uint4*>(a_row + (AW_W1 + ch) * 128) = make_uint4(w1[0], w1[1], w1[2], w1[3]);

@@ -60,3 +60,52 @@ def test_wide_state_kernels_match_the_oracle(case):
         assert oracle.rel_l2(t[src].grad.float().cpu().numpy(), ref) < 2e-3, k
     assert oracle.rel_l2(t["Dskip"].grad.cpu().numpy(), g["dD"]) < 1e-6
     assert oracle.rel_l2(t["h0"].grad.cpu().numpy(), g["dh0"]) < 1e-6
+
+
+def _inputs(B, T, D, N, f_shift, utm=False, seed=11, **kw):
+    d = oracle.make_inputs(B, T, D, N, seed=seed, f_shift=f_shift, **kw)
+    cast = {"u": BF, "Bm": BF, "Cm": BF, "dy": BF, "fl": BF, "il": BF}
+    q = {k: (_round(d[k], cast[k]) if k in cast else d[k]) for k in d}
+    t = {k: torch.tensor(q[k], device="cuda").to(cast.get(k, F32)) for k in q}
+    if utm:
+        t["u"] = t["u"].transpose(1, 2).contiguous().transpose(1, 2)
+    return q, t
+
+
+ORDER = ("u", "fl", "il", "Bm", "Cm", "Dskip")
+
+
+def _run(t, dhT=True):
+    """y, hT and the gradients of ORDER and h0, with the kernel forms that made them."""
+    from naju_b200 import naju_scan
+    from naju_b200.scan import last_kernel_forms
+    x = {k: t[k].detach().requires_grad_(True) for k in ORDER + ("h0",)}
+    y, hT = naju_scan(*(x[k] for k in ORDER), h0=x["h0"], return_final_state=True)
+    torch.autograd.backward([y, hT], [t["dy"], t["dhT"] if dhT else torch.zeros_like(hT)])
+    torch.cuda.synchronize()
+    return y.detach(), hT.detach(), {k: x[k].grad for k in x}, last_kernel_forms()
+
+
+# B, T, D, N, f_shift, time-contiguous u
+@pytest.mark.parametrize("case", [(6, 200, 2560, 64, 2.0, False), (6, 200, 2560, 64, 5.0, True), (7, 199, 2568, 32, 2.0, False)])
+def test_wide_state_kernels_compute_in_fp32(case, monkeypatch):
+    """What is rounded to 16 bits at the end is fp32 until then.  Three bf16 terms hold 24 bits, and some 60 accumulating MMAs that
+    truncate leave about 1e-6; where two values 1e-6 apart are rounded to bf16 (steps of 2^-8) one pair in 2000 lands a step apart,
+    6e-5 in the 2-norm.  (Operands of two terms, 16 bits: 4e-4.)  The fp32 results are no further off than the recurrent
+    kernels' (up to what a different order of the sums makes of 2560 x 64 roundings, 2 %)."""
+    B, T, D, N, fs, utm = case
+    q, t = _inputs(B, T, D, N, fs, utm, d_skip_scale=0.05, with_h0=True)
+    y, hT, g, forms = _run(t)
+    assert forms == {"fwd": WALK, "bwd": WALK}
+    a = tuple(q[k] for k in ORDER)
+    yo, hTo = oracle.oracle_fwd(*a, h0=q["h0"], return_final_state=True)
+    go = oracle.oracle_bwd(*a, q["dy"], h0=q["h0"], dhT=q["dhT"])
+    assert oracle.rel_l2(y.float().cpu().numpy(), _round(yo, BF)) < 1e-4
+    for k, src in (("du", "u"), ("dfl", "fl"), ("dil", "il"), ("dB", "Bm"), ("dC", "Cm")):
+        assert oracle.rel_l2(g[src].float().cpu().numpy(), _round(go[k], BF)) < 1e-4, k
+    monkeypatch.setenv("NAJU_B200_FORM", "recurrent")
+    _, hT_r, g_r, forms = _run(t)
+    assert forms == {"fwd": RECURRENT, "bwd": RECURRENT}
+    for name, ours, theirs, want in (("hT", hT, hT_r, hTo), ("dh0", g["h0"], g_r["h0"], go["dh0"])):
+        err, err_r = (oracle.rel_l2(v.cpu().numpy(), want) for v in (ours, theirs))
+        assert err <= 1.02 * err_r, (name, err, err_r)
