@@ -596,7 +596,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         uint32_t dyp[H];
 #pragma unroll
         for (int j2 = 0; j2 < H; ++j2) {
-          const float2 il2 = mul2(make_float2(fmaxf(ld_as_f32(s_il, (2 * j2) * kDT), -30.f), fmaxf(ld_as_f32(s_il, (2 * j2 + 1) * kDT), -30.f)), kk);
+          const float2 il2 = mul2(make_float2(fmaxf(ld_as_f32(s_il, (2 * j2) * kDT), -80.f), fmaxf(ld_as_f32(s_il, (2 * j2 + 1) * kDT), -80.f)), kk);
           const float2 bq = make_float2(fast_ex2(il2.x), fast_ex2(il2.y));
           const float2 opb = add2(bq, one2);                      // 1 / i_t
           const float2 u2 = UTM ? ld_pair_as_f32(s_ut + 2 * j2) : make_float2(ld_as_f32(s_u, (2 * j2) * kDT), ld_as_f32(s_u, (2 * j2 + 1) * kDT));

@@ -501,7 +501,8 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
           const int j2 = 4 * j8 + jj;
-          const float2 il2 = mul2(make_float2(fmaxf(ld_as_f32(s_il, (2 * j2) * kDT), -30.f), fmaxf(ld_as_f32(s_il, (2 * j2 + 1) * kDT), -30.f)), kk);
+          // (the floor of the exact kernels' gate: e^80 is finite, and so is its reciprocal's product with R)
+          const float2 il2 = mul2(make_float2(fmaxf(ld_as_f32(s_il, (2 * j2) * kDT), -80.f), fmaxf(ld_as_f32(s_il, (2 * j2 + 1) * kDT), -80.f)), kk);
           const float2 opb = add2(make_float2(fast_ex2(il2.x), fast_ex2(il2.y)), one2);   // 1 / i_t
           uv[j2] = UTM ? ld_pair_as_f32(s_ut + 2 * j2) : make_float2(ld_as_f32(s_u, (2 * j2) * kDT), ld_as_f32(s_u, (2 * j2 + 1) * kDT));
           const float2 R = mul2(Rs2, L[j2]);

@@ -109,3 +109,24 @@ def test_wide_state_kernels_compute_in_fp32(case, monkeypatch):
     for name, ours, theirs, want in (("hT", hT, hT_r, hTo), ("dh0", g["h0"], g_r["h0"], go["dh0"])):
         err, err_r = (oracle.rel_l2(v.cpu().numpy(), want) for v in (ours, theirs))
         assert err <= 1.02 * err_r, (name, err, err_r)
+
+
+@pytest.mark.parametrize("utm", [False, True])
+def test_wide_state_write_gates_near_zero(utm):
+    """sigmoid(-40) is 4e-18 and sigmoid(-70) 4e-31, also next to gates of ordinary size and in the gradients.  (1e-3: as above, but
+    the outputs of a third of the channels at a time.)"""
+    B, T, D, N = 6, 96, 2560, 64
+    q, t = _inputs(B, T, D, N, 2.0, utm, with_h0=True)
+    low = torch.zeros(D, device="cuda")
+    low[::3], low[1::3] = -40.0, -70.0
+    t["il"] = (t["il"].float() + low).to(BF)
+    t["h0"], t["dhT"] = torch.zeros_like(t["h0"]), torch.zeros_like(t["dhT"])
+    q["il"], q["h0"], q["dhT"] = t["il"].float().cpu().numpy(), t["h0"].cpu().numpy(), t["dhT"].cpu().numpy()
+    y, _, g, forms = _run(t, dhT=False)
+    assert forms == {"fwd": WALK, "bwd": WALK}
+    a = tuple(q[k] for k in ORDER)
+    yo = oracle.oracle_fwd(*a, h0=q["h0"])
+    go = oracle.oracle_bwd(*a, q["dy"], h0=q["h0"], dhT=q["dhT"])
+    for name, ours, want in (("y", y, yo), ("du", g["u"], go["du"]), ("dfl", g["fl"], go["dfl"]), ("dil", g["il"], go["dil"])):
+        for k in range(3):
+            assert oracle.rel_l2(ours[..., k::3].double().cpu().numpy() * 1e15, _round(want[..., k::3], BF).astype("f8") * 1e15) < 1e-3, (name, k)
