@@ -32,6 +32,11 @@ using namespace simt;
 // accuracy (it matches the f_logit >= -5 envelope of naju/chunk_triton.py:200).
 constexpr float kDeepGate = 0.0078125f;
 
+// (called behind pdl_wait(): the tensor-core backward, if there was one, has completed)
+__device__ __forceinline__ bool tc_did_it(const BwdParams& p) {
+  return p.tc_launched && (*p.fwd_form & 3) == 1 && *reinterpret_cast<volatile int*>(&p.hdr->redo) == 0;
+}
+
 template <int NS>
 struct BwdShape : Shape<NS> {
   // steps between two cross-warp flushes of the dB / dC partial sums
@@ -57,8 +62,8 @@ bwd_simt_kernel(const BwdParams p) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();
-  // the tensor-core backward was launched for this call and is doing the work
-  if (p.tc_launched && (*p.fwd_form & 3) == 1) return;
+  // the tensor-core backward was launched for this call and has done the work
+  if (tc_did_it(p)) return;
   if (blockIdx.x == 0 && tid == 0) p.hdr->form = NAJU_FORM_RECURRENT;
 
   const int q = lane % L, g = lane / L, chan0 = (warp * GW + g) * kC, my_ch = chan0 + chan_of<L>(q);
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* 
     return;
   }
   // the tensor-core backward writes four partial rows per rank and batch row, the recurrent one per chunk
-  const int rows = (dd_rows_tc > 0 && (form & 3) == 1) ? dd_rows_tc : dd_rows;
+  const int rows = tc_did_it(p) ? dd_rows_tc : dd_rows;
   const int dl = threadIdx.x & 31, rl = threadIdx.x >> 5, d = (blk - 2 * nbc) * 32 + dl, ld = p.ndt * kDT;
   float s = 0.f;
   if (d < p.D)

@@ -86,8 +86,8 @@ struct Bars {
   unsigned long long acc_free[2];      // carry warps have read D2 and s_Rend and written the deep flag
 };
 
-// Exact recurrence of one tile straight from global memory (deep-gate tiles only), by the carry threads, each with its
-// NSH states from n0 on; the second half's share of y goes through shared memory.
+// Exact recurrence of one tile straight from global memory (deep gates, or something that is not finite), by the carry
+// threads, each with its NSH states from n0 on; the second half's share of y goes through shared memory.
 template <typename TA, typename TG, int NSH>
 __device__ __noinline__ void exact_tile(const FwdParams& p, const TileCoord& tc, int q, int half, float* s_deep, float (&hw)[NSH], float& Pw) {
   const TA* gu = reinterpret_cast<const TA*>(p.u) + tc.b * p.u_sb + static_cast<int64_t>(tc.t0) * p.u_st + tc.d * p.u_sd;
@@ -130,6 +130,8 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ Bars bars;
   __shared__ int s_stage_deep[2];
+  __shared__ int s_bad[2];           // some w of the stage's tile is too large for the factorised form, or not finite
+  __shared__ int s_bad_bc[4];        // some B or C of tile `it & 3` is
   __shared__ unsigned int s_tmem;
   __shared__ float s_L[2][kDT];      // retention product of a tile's first 16 steps (as 1 / prod f)
   __shared__ float s_Rend[2][kDT];   // 1 / (retention product of the whole chunk)
@@ -140,6 +142,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   const int x_first = static_cast<int>(blockIdx.x), x_step = static_cast<int>(gridDim.x);
   const int ntotal = (x_first < ctiles ? (ctiles - x_first + x_step - 1) / x_step : 0) * nchunks;
 
+  if (tid < 2) s_bad[tid] = 0;
   if (tid == 0) {
     for (int i = 0; i < SM::RING; ++i) {
       mbar_init(smem_u32(&bars.full[i]), 1);
@@ -220,13 +223,18 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       unsigned char* s_BB = smem + SM::off_BB + st * SM::BB_BYTES;
       const unsigned char* raw = smem + SM::off_bc + st * 2 * SM::BC_BYTES;
       // 16-byte pieces: eight lanes take a row's neighbours in turn (the raw rows are read without bank conflicts)
+      uint32_t bad = 0;
 #pragma unroll 4
       for (int i = lane; i < Q * SM::NC; i += 32) {
         const int r = i / SM::NC, k = i % SM::NC;
-        *reinterpret_cast<uint4*>(s_BB + op_off16(r, k * 8, SM::SBO_BB)) = *reinterpret_cast<const uint4*>(raw + i * 16);
-        *reinterpret_cast<uint4*>(s_B1 + op_off16(r, (SM::B1_C + k) * 8, SM::SBO_B1)) =
-            *reinterpret_cast<const uint4*>(raw + SM::BC_BYTES + i * 16);
+        const uint4 bv = *reinterpret_cast<const uint4*>(raw + i * 16), cv = *reinterpret_cast<const uint4*>(raw + SM::BC_BYTES + i * 16);
+        *reinterpret_cast<uint4*>(s_BB + op_off16(r, k * 8, SM::SBO_BB)) = bv;
+        *reinterpret_cast<uint4*>(s_B1 + op_off16(r, (SM::B1_C + k) * 8, SM::SBO_B1)) = cv;
+        bad |= too_large_bf16x8(bv) | too_large_bf16x8(cv);
       }
+      // (four slots: the carry warps are at most two tiles behind)
+      const bool bad_bc = __any_sync(0xffffffffu, bad != 0);
+      if (lane == 0) s_bad_bc[it & 3] = bad_bc ? 1 : 0;
       fence_async_smem();
       tc_fence_before();
       __syncwarp();
@@ -355,9 +363,20 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         hc[n] = (p.h0 != nullptr && d < p.D && n0 + n < p.N) ? p.h0[(static_cast<int64_t>(b) * p.D + d) * p.N + n0 + n] : 0.f;
       Pc = 1.f;
     };
+    // Not 0 if a state entering the current chunk is too large or not finite.  Looked at where states come in and behind the exact
+    // path only: what the factorised path takes leaves them finite, and here they are on the chain from tile to tile (0.15 ms of
+    // 2.4 at B=8, T=8192, D=4096, N=64).
+    float hz = 0.f;
+    auto check_states = [&]() {
+      float2 z = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int n = 0; n < NSH; n += 2) z = watch(z, make_float2(hc[n], hc[n + 1]), kOverState);
+      hz = z.x + z.y;
+    };
     if (x_first < ctiles) {
       load_h0(x_first);
       write_h_row();
+      check_states();
     }
     int it = 0;
     for (int x = x_first; x < ctiles; x += x_step) {
@@ -374,10 +393,18 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         const int st = it & 1;
         const uint32_t par = (it >> 1) & 1;
         if (!mbar_wait(smem_u32(&bars.d2_full[st]), par)) timeout();
-        if (!mbar_wait(smem_u32(&bars.part[st][1]), par)) timeout();   // (the writers of s_Rend arrived here)
+        // (the writers of s_Rend and s_bad arrived on `part`, the writer of s_bad_bc on `ops_full`)
+        if (!mbar_wait(smem_u32(&bars.part[st][0]), par)) timeout();
+        if (!mbar_wait(smem_u32(&bars.part[st][1]), par)) timeout();
+        if (!mbar_wait(smem_u32(&bars.ops_full[st]), par)) timeout();
         const float Rend = s_Rend[st][q];
-        const bool deep = bar_or<2, NCARRY>(!(Rend < kRMax));
-        if (tid == W_CARRY * 32) s_stage_deep[st] = deep ? 1 : 0;
+        // The exact path takes a tile with deep gates, and one with a value that is not finite: every step of a channel meets
+        // the others' in an MMA, masked by zeros.
+        const bool deep = bar_or<2, NCARRY>(!(Rend < kRMax) || !(hz == 0.f) || (s_bad[st] | s_bad_bc[it & 3]) != 0);
+        if (tid == W_CARRY * 32) {
+          s_stage_deep[st] = deep ? 1 : 0;
+          s_bad[st] = 0;
+        }
         tc_fence_after();
         if (deep) {
           if (tid == W_CARRY * 32) atomicOr(p.fwd_form, 2);
@@ -395,6 +422,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
 #pragma unroll
           for (int n = 0; n < NSH; ++n) hc[n] = hw[n];
           Pc = Pw;
+          check_states();
         } else {
           const float P = __frcp_rn(Rend), Pl = P * fmaf(-P, Rend, 1.f);   // (P + Pl = 1 / Rend)
 #pragma unroll
@@ -432,6 +460,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
           if (x + x_step >= ctiles) continue;
           load_h0(x + x_step);
           write_h_row();
+          check_states();
         }
       }
     }
@@ -495,6 +524,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
       const float2 Rs2 = make_float2(Rstart, Rstart);
       float2 Pv[SLAB / 2];
       float2 uv[SLAB / 2];
+      float2 wz = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j8 = 0; j8 < SLAB / 8; ++j8) {
         uint32_t w1[4], w2[4], w3[4];
@@ -511,6 +541,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
           // kernel's with it)
           const float2 ig = make_float2(fast_rcp(opb.x), fast_rcp(opb.y)), iR = mul2(ig, R);
           const float2 w = mul2(uv[j2], fma2(iR, fma2(make_float2(-opb.x, -opb.y), ig, one2), iR));
+          wz = watch(wz, w, kOverW);
           split3(w, w1[jj], w2[jj], w3[jj]);
         }
         const int ch = 2 * g + j8;
@@ -518,6 +549,7 @@ fwd_wide_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         *reinterpret_cast<uint4*>(a_row + (AW_W2 + ch) * 128) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
         *reinterpret_cast<uint4*>(a_row + (AW_W3 + ch) * 128) = make_uint4(w3[0], w3[1], w3[2], w3[3]);
       }
+      if (!(wz.x + wz.y == 0.f)) s_bad[st] = 1;
       mbar_arrive_warp(smem_u32(&bars.empty[slot]));   // the slab has been read
       fence_async_smem();
       tc_fence_before();

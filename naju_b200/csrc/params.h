@@ -67,6 +67,7 @@ struct ScratchHeader {
   unsigned int ticket;   // dynamic tile counter
   int form;              // NAJU_FORM_* of the kernel that did the work (written by that kernel)
   unsigned int done;     // CTAs that have finished
+  int redo;              // the tensor-core backward met something it cannot take: the recurrent one does the work
 };
 
 // Forward scratch: header | flags[ntiles] | aggP[ntiles][128] | aggS[ntiles][128][NS]

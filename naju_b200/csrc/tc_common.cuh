@@ -348,6 +348,21 @@ __device__ __forceinline__ void split3(float2 v, uint32_t& hi, uint32_t& mid, ui
   split_pair(fma2(h, make_float2(-1.f, -1.f), v), mid, lo);
 }
 
+// ---- what the factorised form with masks takes
+// A mask's zero times an infinity is a NaN, so a tile may hold nothing that is not finite, and nothing so large that a sum over a
+// tile of it could overflow: w (with the retention product in it, up to 2^80) below 2^88, B and C below 2^14, incoming gradients
+// below 2^30, states and adjoints below 2^100 at the places where the walks look at them.  Larger values go to the exact kernels.
+constexpr float kOverW = 0x1p40f, kOverGrad = 0x1p98f, kOverState = 0x1p28f;   // times the limit = 2^128
+// `z` becomes NaN once x * over overflows.
+__device__ __forceinline__ float2 watch(float2 z, float2 x, float over) {
+  return fma2(mul2(x, make_float2(over, over)), make_float2(0.f, 0.f), z);
+}
+// Not zero if one of eight bf16 is not below 2^14 (the sum carries into the sign's place from that exponent on).
+__device__ __forceinline__ uint32_t too_large_bf16x8(uint4 v) {
+  const uint32_t m = 0x7F807F80u, up = (0x8000u - ((127u + 14u) << 7)) * 0x10001u;
+  return (((v.x & m) + up) | ((v.y & m) + up) | ((v.z & m) + up) | ((v.w & m) + up)) & 0x80008000u;
+}
+
 // ---- bf16 helpers
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {  // lo -> bits [0,16)
   uint32_t r;

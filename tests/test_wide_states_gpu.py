@@ -130,3 +130,35 @@ def test_wide_state_write_gates_near_zero(utm):
     for name, ours, want in (("y", y, yo), ("du", g["u"], go["du"]), ("dfl", g["fl"], go["dfl"]), ("dil", g["il"], go["dil"])):
         for k in range(3):
             assert oracle.rel_l2(ours[..., k::3].double().cpu().numpy() * 1e15, _round(want[..., k::3], BF).astype("f8") * 1e15) < 1e-3, (name, k)
+
+
+@pytest.mark.parametrize("where", ["u", "Bm", "Cm", "h0", "fl", "dy", "dhT", "huge u", "huge B", "huge dy"])
+def test_wide_state_kernels_keep_what_is_not_finite_where_it_belongs(where, monkeypatch):
+    """An infinity or NaN reaches the steps after it (or, in the backward, before it) and the state, channel and batch row it
+    belongs to, exactly as in the recurrent kernels; everything else is as finite as there and the same up to a rounding."""
+    B, T, D, N = 6, 104, 2560, 64
+    _, t = _inputs(B, T, D, N, 2.0, with_h0=True)
+    inf = float("inf")
+    if where in ("u", "dy"):
+        t[where][1, 41, 7], t[where][2, 70, 300] = inf, float("nan")
+    elif where == "huge u":
+        t["u"][1, 41, 7] = 1e37
+    elif where == "huge B":
+        t["Bm"][1, 41, 7], t["Cm"][2, 41, 7] = 1e30, -1e30
+    elif where == "huge dy":
+        t["dy"][1, 41, 7] = -1e30
+    elif where in ("Bm", "Cm"):
+        t[where][1, 41, 7] = -inf
+    elif where == "fl":
+        t[where][1, 41, 7], t[where][2, 41, 9] = float("nan"), -inf
+    else:
+        t[where][1, 300, 7] = inf
+    y, hT, g, forms = _run(t)
+    assert forms["bwd"] == RECURRENT   # (by the forward's mark, or because the tensor-core backward hands the work on)
+    monkeypatch.setenv("NAJU_B200_FORM", "recurrent")
+    y_r, hT_r, g_r, _ = _run(t)
+    for name, a, b in [("y", y, y_r), ("hT", hT, hT_r)] + [(k, g[k], g_r[k]) for k in g]:
+        assert torch.equal(torch.isnan(a), torch.isnan(b)), name
+        assert torch.equal(torch.isinf(a), torch.isinf(b)), name
+        both = torch.isfinite(a) & torch.isfinite(b)
+        assert bool(both.any()) and oracle.rel_l2(a[both].double().cpu().numpy(), b[both].double().cpu().numpy()) < 4e-3, name
