@@ -549,7 +549,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
       const int b = x / p.ndt, dt = x - b * p.ndt, d0 = dt * kDT, d = d0 + cid;
       const bool d_ok = d < p.D;
       const float Dv = d_ok ? __ldg(p.Dskip + d) : 0.f;
-      float dDsum = 0.f;
+      float dDsum = 0.f, dDlow = 0.f;   // (the sum over the chunks and what its additions dropped)
 #pragma unroll 1
       for (int ci = 0; ci < nchunks; ++ci, ++it) {
         const int t0 = (nchunks - 1 - ci) * Q, nvalid = p.T - t0 - SLAB * grp;   // real steps among this thread's
@@ -602,6 +602,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         const float2 Rs2 = make_float2(Rstart, Rstart);
         float2 alr[H], wtr[H], cf[H], cm[H], cu[H];
         uint32_t dyp[H];
+        float dDc = 0.f;
 #pragma unroll
         for (int j2 = 0; j2 < H; ++j2) {
           const float2 il2 = mul2(make_float2(fmaxf(ld_as_f32(s_il, (2 * j2) * kDT), -80.f), fmaxf(ld_as_f32(s_il, (2 * j2 + 1) * kDT), -80.f)), kk);
@@ -618,10 +619,15 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
           alr[j2] = mul2(dy2, P);
           cf[j2] = mul2(mul2(av[j2], Rprev), P);                  // 1 - f_t
           cm[j2] = mul2(bq, ig);                                  // 1 - i_t
-          dDsum = fmaf(dy2.x, u2.x, fmaf(dy2.y, u2.y, dDsum));
+          dDc = fmaf(dy2.x, u2.x, fmaf(dy2.y, u2.y, dDc));
           dyp[j2] = __byte_perm(__float_as_uint(dy2.x), __float_as_uint(dy2.y), 0x7632);
         }
         mbar_arrive_warp(smem_u32(&bars.empty[slot]));   // the slab has been read
+        {
+          const float s = dDsum + dDc, v = s - dDsum;
+          dDlow += (dDsum - (s - v)) + (dDc - v);
+          dDsum = s;
+        }
         // the channel rows are free once every MMA of the previous tile that reads them is complete
         if (it >= 1 && !mbar_wait(smem_u32(&bars.d4_full), par ^ 1)) timeout();
         {
@@ -721,7 +727,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
         }
       }
       // channel tile done: D_skip partials (one row per group and batch row)
-      p.dDpart[static_cast<int64_t>(grp * p.B + b) * (p.ndt * kDT) + d] = dDsum;
+      p.dDpart[static_cast<int64_t>(grp * p.B + b) * (p.ndt * kDT) + d] = dDsum + dDlow;
     }
   }
   __syncthreads();

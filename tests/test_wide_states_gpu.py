@@ -162,3 +162,20 @@ def test_wide_state_kernels_keep_what_is_not_finite_where_it_belongs(where, monk
         assert torch.equal(torch.isinf(a), torch.isinf(b)), name
         both = torch.isfinite(a) & torch.isfinite(b)
         assert bool(both.any()) and oracle.rel_l2(a[both].double().cpu().numpy(), b[both].double().cpu().numpy()) < 4e-3, name
+
+
+def test_wide_state_d_skip_gradient_over_a_long_sequence():
+    """dD = sum dy u over 8192 steps of equal products: one running sum of every fourth octet loses 2e-5 to one-sided roundings; sums
+    per chunk, added up with what the additions drop, stay at fp32's own 6e-8 a value."""
+    from naju_b200 import naju_scan
+    from naju_b200.scan import last_kernel_forms
+    B, T, D, N = 1, 8192, 6400, 24
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    u, dy = ((torch.rand(D, device="cuda", generator=gen) + 0.5).to(BF).expand(B, T, D).contiguous() for _ in range(2))
+    skip = r(D).requires_grad_(True)
+    y = naju_scan(u, (r(B, T, D) + 2).to(BF), r(B, T, D).to(BF), r(B, T, N).to(BF), r(B, T, N).to(BF), skip)
+    dD, = torch.autograd.grad(y, [skip], [dy])
+    assert last_kernel_forms()["bwd"] == WALK
+    want = (dy.double() * u.double()).sum((0, 1))
+    assert ((dD.double() - want).norm() / want.norm()).item() < 2e-7
