@@ -240,7 +240,8 @@ int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit
     if (rc2 == 0) p.tc_launched = cs;
     else if (rc2 != -1000) return rc2;
   }
-  rc = launch_bwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
+  rc = launch_bwd_chan(p, g, desc->act_dtype, desc->gate_dtype, stream);
+  if (rc == -1000) rc = launch_bwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
   if (rc != 0) return rc;
   return launch_bwd_finalize(p, g, desc->act_dtype, desc->gate_dtype, dB, dC, dD,
                              (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0, stream);

@@ -28,15 +28,6 @@ namespace naju {
 
 using namespace simt;
 
-// Below this retention the difference form of d f_logit loses more than ~3e-5 relative
-// accuracy (it matches the f_logit >= -5 envelope of naju/chunk_triton.py:200).
-constexpr float kDeepGate = 0.0078125f;
-
-// (called behind pdl_wait(): the tensor-core backward, if there was one, has completed)
-__device__ __forceinline__ bool tc_did_it(const BwdParams& p) {
-  return p.tc_launched && (*p.fwd_form & 3) == 1 && *reinterpret_cast<volatile int*>(&p.hdr->redo) == 0;
-}
-
 template <int NS>
 struct BwdShape : Shape<NS> {
   // steps between two cross-warp flushes of the dB / dC partial sums

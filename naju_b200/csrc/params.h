@@ -177,6 +177,8 @@ int launch_fwd_chan(const FwdParams& p, const Geometry& g, int act_dtype, int ga
 int launch_fwd_wide(const FwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
 int launch_bwd_wide(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, int bc_dtype, void* stream);
 int launch_bwd_simt(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);
+// exact recurrent backward of 16 states, 16-bit inputs and logits and 64-step chunks; returns -1000 when it cannot take the problem
+int launch_bwd_chan(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* stream);
 // dB, dC and dD from the partial sums; overwrites every output with NaN if the call (or its forward) failed
 int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act_dtype, int gate_dtype, void* dB, void* dC, float* dD,
                         bool inject, void* stream);
