@@ -1031,29 +1031,20 @@ int launch_bwd_tc_t(const BwdParams& p, const Geometry& g, const tcb::Maps& maps
   auto walk = tcb::bwd_tc_kernel<TA, TG, UTM, false>;
   auto shared = tcb::bwd_tc_kernel<TA, TG, UTM, true>;
   static std::atomic<unsigned long long> ok1{0}, okc{0};
-  static std::atomic<int> fit[2][64];
+  static std::atomic<int> fit[64];
   int rc = allow_smem(walk, smem, ok1);
   if (rc == 0) rc = allow_smem(shared, smem, okc);
   if (rc != 0) return rc;
-  // The cluster size with the shortest busiest CTA, in units of 0.1 us: a tile takes 6.0 us in a cluster of one, 10.0 us in
-  // one of two and 10.5 us in one of four, whose ranks wait for each other's adjoint.
+  // The cluster size with the shortest busiest CTA, in units of 0.1 us: a tile takes 6.0 us in a cluster of one and 10.0 us in one
+  // of two, whose ranks wait for each other's adjoint.  (10.5 us in one of four; at least 37 channel tiles come here and at most
+  // 36 clusters of four fit.)
   int best = 1;
-  int64_t clusters, n, cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 60;
-  for (int k = 0, cs = 2; cs <= 4 && cs <= g.nchunks; ++k, cs *= 2) {
-    const int64_t fits = tmah::max_clusters(shared, tcb::NTHREADS, smem, cs, fit[k]);
-    const int64_t c = tmah::cluster_trips(g, cs, fits, n) * (cs == 2 ? 100 : 105);
-    if (c < cost) {
-      cost = c;
-      best = cs;
-      clusters = n;
-    }
+  int64_t clusters, n;
+  const int64_t cost = tmah::cluster_trips(g, 1, tmah::sm_count(), clusters) * 60;
+  if (tmah::cluster_trips(g, 2, tmah::max_clusters(shared, tcb::NTHREADS, smem, 2, fit), n) * 100 < cost) {
+    best = 2;
+    clusters = n;
   }
-  // The exact recurrent backward spreads over time too: 15 us, and 0.3 to 0.39 us per tile of 64 steps x 128 channels on a full
-  // GPU or 1.5 us per chunk where the look-back sets the pace.  (Every tile here has its own carry to wait for, 10 us in all.)
-  if (cost + 100 > 150 + std::max<int64_t>(7 * g.ntiles / 2, 15 * static_cast<int64_t>(g.nchunks))) return -1000;
-  // The gradients of fp32 logits, and dh0, are fp32, and the two-term operands here are not (6e-5 and 1e-5 against the
-  // recurrent kernel's 2e-6 and 2e-7): with so few channel tiles that the walk alone would not be taken they stay there.
-  if (static_cast<int64_t>(g.B) * g.ndt * 4 < tmah::sm_count() && (std::is_same<TG, float>::value || p.dh0 != nullptr)) return -1000;
   cs_used = best;
   const dim3 grid(static_cast<unsigned>(clusters * best)), block(tcb::NTHREADS);
   return best == 1 ? launch_pdl(walk, grid, block, smem, st, p, maps, fwd_form)
@@ -1066,6 +1057,12 @@ int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act, int gate, int 
   if (!(g.N == tcb::NS && g.TC == tcb::Q && act == NAJU_BF16 && (gate == NAJU_BF16 || gate == NAJU_F32) &&
         bc == NAJU_BF16))
     return -1000;
+  // The operands here have two bf16 terms, 16 bits: gradients of fp32 logits come out at 6e-5 and dh0 at 1e-5, where the recurrent
+  // kernel has 5e-7 and 4e-7, and 16-bit gradients are 1e-4 of their rounding error further off.  Where one CTA per channel tile would leave
+  // three quarters of the SMs idle, or a sequence is shorter than four chunks, the recurrent kernel does the work; clusters (every rank
+  // has a chunk of every channel tile) take channel tiles above that line only.  There the walk is the faster one for any length: 37
+  // channel tiles take 5 us per chunk in clusters of two, the recurrent kernel 0.22 us per tile.
+  if (!(static_cast<int64_t>(g.B) * g.ndt * 4 >= tmah::sm_count() && g.nchunks >= 4)) return -1000;
   tcb::Maps maps = {};
   const bool ok =
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, tcb::SLAB, kDT)

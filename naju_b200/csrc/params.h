@@ -98,8 +98,8 @@ inline BwdScratchLayout bwd_scratch_layout(const Geometry& g) {
   const size_t sP = align_up(static_cast<size_t>(g.ntiles) * 128 * 4, 256);
   const size_t sS = align_up(static_cast<size_t>(g.ntiles) * 128 * g.NS * 4, 256);
   const size_t sBC = align_up(static_cast<size_t>(g.B) * g.T * g.ndt * g.NS * 4, 256);
-  // dD partial rows: one per chunk and batch row, or one per group and rank (up to 4 x 4) of the tensor-core backward
-  const size_t sD = align_up(static_cast<size_t>(g.nchunks < 16 ? 16 : g.nchunks) * g.B * g.ndt * 128 * 4, 256);
+  // dD partial rows: one per chunk and batch row, or one per group and rank (up to 4 x 2) of the tensor-core backward
+  const size_t sD = align_up(static_cast<size_t>(g.nchunks < 8 ? 8 : g.nchunks) * g.B * g.ndt * 128 * 4, 256);
   l.off_aggL = l.off_aggP + sP;
   l.off_inclL = l.off_aggL + sS;
   l.off_dBpart = l.off_inclL + sS;
