@@ -922,9 +922,10 @@ int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int
     return -1000;
   if (g.ntiles >= (1LL << 31)) return -1000;
   const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt, sms = tmah::sm_count();
-  // A time-contiguous u of a problem with fewer tiles than SMs stays with the recurrent kernel.
-  if (p.u_sd > 1 && g.ntiles < sms) return -1000;
   const int form = (ctiles * 4 >= sms && g.nchunks >= 4) ? NAJU_FORM_TC_WALK : NAJU_FORM_TC_TICKET;
+  // A time-contiguous u (which the ticket kernel cannot take) with few channel tiles or chunks stays with the recurrent kernel: its final
+  // state is fp32 throughout (4.7e-7 at B=1, T=1024, D=2048, f_mean 5), the two-term operands here are not (9.8e-6).
+  if (p.u_sd > 1 && !(ctiles * 4 >= sms && g.nchunks >= 4)) return -1000;
   tc3::Maps maps;
   const bool ok =
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, tc3::SLAB, kDT)

@@ -69,3 +69,15 @@ def test_gradients_of_few_channel_tiles_or_chunks_are_fp32_inside(case):
     assert forms["bwd"] == RECURRENT
     for k in g:
         assert _err(g[k], go[k]) < (2.5e-4 if g[k].dtype == BF else 1e-5 if k == "dfl" else 2e-6), k
+
+
+# B, T, D, f_shift, logits
+@pytest.mark.parametrize("case", [(1, 1024, 2048, 5.0, F32), (2, 520, 1024, 2.0, BF), (8, 192, 2048, 2.0, F32)])
+def test_time_contiguous_u_with_few_channel_tiles_keeps_an_fp32_state(case):
+    """The recurrent kernel: final state to 2e-6 (1e-5 with the tensor-core kernel's operands of 16 bits), y a step apart in one place
+    of 2000 at most (sqrt(1e-6 2^-7.5) = 7e-5)."""
+    B, T, D, fs, gdt = case
+    (y, hT, _, forms), (yo, hTo, _) = _run(B, T, D, fs, gdt, True)
+    assert forms["fwd"] == RECURRENT
+    assert _err(hT, hTo) < 2e-6
+    assert _err(y, yo) < 7e-5
