@@ -75,7 +75,8 @@ enum {
   NAJU_FORM_RECURRENT = 1, /* exact recurrent kernels */
   NAJU_FORM_TC_TICKET = 2, /* tensor-core chunked forward, tiles by ticket with look-back carry */
   NAJU_FORM_TC_WALK = 3    /* tensor-core chunked form walking each channel tile along time
-                              (forward) or in reverse time (backward) */
+                              (forward) or in reverse time (backward), by one CTA or by the
+                              CTAs of a thread-block cluster */
 };
 
 /* Problem description shared by forward and backward.

@@ -188,7 +188,7 @@ __device__ __noinline__ void exact_tile_from_global(const FwdParams& p, const Ti
 //   rank sending its aggregate to all others and folding theirs 4.9 us; this form 4.1 us on twice the SMs.)
 template <typename TA, typename TG, bool UTM, bool CLUSTER>
 __global__ void __launch_bounds__(kThreadsOf<CLUSTER>, 1)
-fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int form) {
+fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
   using SM = Smem<TG, CLUSTER>;
   constexpr int NTHREADS = kThreadsOf<CLUSTER>;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -264,7 +264,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
   pdl_wait();   // nothing above touches global memory
   if (blockIdx.x == 0 && tid == 0) {
     atomicOr(p.fwd_form, 1);  // tell the backward how the forward ran
-    p.hdr->form = form;
+    p.hdr->form = NAJU_FORM_TC_WALK;
   }
   auto timeout = [&]() { atomicOr(&p.hdr->status, NAJU_ST_MMA_TIMEOUT); };
   // u is time-contiguous: its slabs sit in shared memory as [channel][step].  (A compile-time
@@ -881,7 +881,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int f
 namespace {
 
 template <typename TA, typename TG, bool UTM>
-int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, int form, cudaStream_t st) {
+int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, cudaStream_t st) {
   auto walk = tc3::fwd_tc3_kernel<TA, TG, UTM, false>;
   auto shared = tc3::fwd_tc3_kernel<TA, TG, UTM, true>;
   constexpr size_t smem1 = tc3::Smem<TG, false>::total, smemc = tc3::Smem<TG, true>::total;
@@ -908,8 +908,8 @@ int launch_tc3_t(const FwdParams& p, const Geometry& g, const tc3::Maps& maps, i
   rc = launch_init(p.hdr, 256, p.fwd_form, st);
   if (rc != 0) return rc;
   const dim3 grid(static_cast<unsigned>(clusters * best)), block(best > 1 ? tc3::kThreadsOf<true> : tc3::kThreadsOf<false>);
-  return best == 1 ? launch_pdl(walk, grid, block, smem1, st, p, maps, form)
-                   : launch_cluster(shared, grid, block, smemc, best, st, p, maps, form);
+  return best == 1 ? launch_pdl(walk, grid, block, smem1, st, p, maps)
+                   : launch_cluster(shared, grid, block, smemc, best, st, p, maps);
 }
 
 }  // namespace
@@ -922,7 +922,6 @@ int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int
     return -1000;
   if (g.ntiles >= (1LL << 31)) return -1000;
   const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt, sms = tmah::sm_count();
-  const int form = (ctiles * 4 >= sms && g.nchunks >= 4) ? NAJU_FORM_TC_WALK : NAJU_FORM_TC_TICKET;
   // A time-contiguous u (which the ticket kernel cannot take) with few channel tiles or chunks stays with the recurrent kernel: its final
   // state is fp32 throughout (4.7e-7 at B=1, T=1024, D=2048, f_mean 5), the two-term operands here are not (9.8e-6).
   if (p.u_sd > 1 && !(ctiles * 4 >= sms && g.nchunks >= 4)) return -1000;
@@ -940,15 +939,15 @@ int launch_fwd_tc3(const FwdParams& p, const Geometry& g, int act, int gate, int
   const bool utm = p.u_sd > 1;
   int rc;
   if (act == NAJU_BF16 && gate == NAJU_BF16)
-    rc = utm ? launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, form, st)
-             : launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, form, st);
+    rc = utm ? launch_tc3_t<__nv_bfloat16, __nv_bfloat16, true>(p, g, maps, st)
+             : launch_tc3_t<__nv_bfloat16, __nv_bfloat16, false>(p, g, maps, st);
   else if (act == NAJU_BF16)
-    rc = utm ? launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, form, st)
-             : launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, form, st);
+    rc = utm ? launch_tc3_t<__nv_bfloat16, float, true>(p, g, maps, st)
+             : launch_tc3_t<__nv_bfloat16, float, false>(p, g, maps, st);
   else if (gate == NAJU_F16)
-    rc = utm ? launch_tc3_t<__half, __half, true>(p, g, maps, form, st) : launch_tc3_t<__half, __half, false>(p, g, maps, form, st);
+    rc = utm ? launch_tc3_t<__half, __half, true>(p, g, maps, st) : launch_tc3_t<__half, __half, false>(p, g, maps, st);
   else
-    rc = utm ? launch_tc3_t<__half, float, true>(p, g, maps, form, st) : launch_tc3_t<__half, float, false>(p, g, maps, form, st);
+    rc = utm ? launch_tc3_t<__half, float, true>(p, g, maps, st) : launch_tc3_t<__half, float, false>(p, g, maps, st);
   return rc == -1001 ? launch_fwd_tc2(p, g, act, gate, bc, stream) : rc;
 }
 

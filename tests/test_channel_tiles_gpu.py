@@ -81,3 +81,50 @@ def test_time_contiguous_u_with_few_channel_tiles_keeps_an_fp32_state(case):
     assert forms["fwd"] == RECURRENT
     assert _err(hT, hTo) < 2e-6
     assert _err(y, yo) < 7e-5
+
+
+def _deep(chunks, channels):
+    """Retention gates of some chunks and channels so deep that the chunk's product leaves fp32."""
+    def change(fl):
+        for c in chunks:
+            fl[:, 64 * c + 5: 64 * c + 60, channels] = -9.0
+    return change
+
+
+# B, T, D, f_shift, logits, time-contiguous u, initial state, chunks with deep gates
+@pytest.mark.parametrize("case", [
+    # clusters of two: 38 and 40 channel tiles (the last of 8 channels), nine chunks (the last of 8 steps)
+    (2, 520, 2432, 2.0, BF, False, True, ()),
+    (2, 520, 2440, 2.0, F32, False, True, ()),
+    (2, 520, 2440, 4.0, BF, True, True, ()),
+    (2, 520, 2432, 2.0, F32, True, False, ()),
+    (2, 520, 2432, 2.0, BF, False, True, (3,)),          # a deep tile between two mails
+    (2, 520, 2440, 2.0, F32, True, True, (0, 1, 8)),     # ... the first two and the last
+    # clusters of four (forward): 24 and 27 channel tiles, seven chunks; three, so that one rank has none
+    (3, 400, 1024, 2.0, BF, False, True, ()),
+    (3, 400, 1032, 4.0, F32, False, False, ()),
+    (3, 400, 1032, 2.0, BF, False, True, (2, 3, 6)),
+    (3, 130, 1032, 2.0, BF, False, True, ())])
+def test_clusters_share_a_channel_tile(case):
+    """Carry and adjoint from rank to rank: final state and dh0 to the 1e-5 of two-term operands, outputs in 16 bits as close as
+    elsewhere in the tensor-core form.  The form word names the walk."""
+    B, T, D, fs, gdt, utm, states, deep = case
+    (y, hT, g, forms), (yo, hTo, go) = _run(B, T, D, fs, gdt, utm, states, f_logit=_deep(deep, slice(100, 140)) if deep else None)
+    few = B * ((D + 127) // 128) * 4 < 148
+    assert forms == {"fwd": WALK, "bwd": RECURRENT if deep or few else WALK}
+    assert _err(hT, hTo) < 2e-5
+    assert _err(y, yo) < 1e-3
+    for k in g:
+        assert _err(g[k], go[k]) < (2e-5 if k == "dh0" else 2e-3), k
+
+
+@pytest.mark.parametrize("case", [(2, 64, 256, TICKET), (2, 1000, 384, TICKET), (1, 4096, 2048, WALK), (8, 128, 2048, WALK), (1, 130, 4736, WALK)])
+def test_the_form_word_names_the_kernel_that_ran(case):
+    """The ticket kernel where few channel tiles make a chain of chunks, a walk (by single CTAs, or by clusters) everywhere else."""
+    from naju_b200 import naju_scan
+    from naju_b200.scan import last_kernel_forms
+    B, T, D, form = case
+    r = lambda *s: torch.randn(*s, device="cuda", dtype=F32).to(BF)  # noqa: E731
+    with torch.no_grad():
+        naju_scan(r(B, T, D), r(B, T, D) + 2, r(B, T, D), r(B, T, 16), r(B, T, 16), torch.zeros(D, device="cuda"))
+    assert last_kernel_forms()["fwd"] == form
