@@ -566,7 +566,7 @@ bwd_tc_kernel(const BwdParams p, const __grid_constant__ Maps maps, const int* _
       auto clear_to_send = [&]() {   // this CTA's lt rows may be overwritten by the next mail
         if (!alive) return;
         if (cid == 0) mbar_arrive_expect_tx(smem_u32(&bars.mail_full), NCARRY * NS * 4);
-        mbar_arrive_cluster_relaxed_warp(out_cts);
+        mbar_arrive_cluster_warp(out_cts, false);   // (the mail before went into the lt rows that have been written since)
       };
       auto post_h = [&]() {
         write_split_rows(hv, R_H1, R_H2);

@@ -590,7 +590,7 @@ fwd_tc3_kernel(const FwdParams p, const __grid_constant__ Maps maps) {
         if (t.c > 0 && alive) {   // the mail has been used: the next one may come
           ++got;
           if (q == 0) mbar_arrive_expect_tx(smem_u32(&bars.mail_full), SM::mail_bytes);
-          mbar_arrive_cluster_relaxed_warp(out_empty);
+          mbar_arrive_cluster_warp(out_empty, t.c + 1 == nchunks);   // (the last chunk has sent nothing on)
         }
         // this tile's carry-in row, once the previous tile's MMAs have read theirs
         if (it > 0 && !mbar_wait(smem_u32(&bars.d1_full[st ^ 1]), ((it - 1) >> 1) & 1)) timeout();

@@ -243,12 +243,15 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, flo
 __device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t mbar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v), "r"(mbar) : "memory");
 }
-// One arrival for the whole warp on a barrier of another CTA of the cluster, ordered after nothing: it says that
-// values this warp has read into registers, and used, may be overwritten.
-__device__ __forceinline__ void mbar_arrive_cluster_relaxed_warp(uint32_t addr) {
+// One arrival for the whole warp on a barrier of another CTA of the cluster: it says that values this warp has read into
+// registers may be overwritten.  Relaxed where they have been used by now, in stores that could not have been issued before the
+// loads had returned; `release` where nothing has used them yet (3.5 us instead of 1, as it waits for the thread's global stores).
+__device__ __forceinline__ void mbar_arrive_cluster_warp(uint32_t addr, bool release) {
   __syncwarp();
-  if ((threadIdx.x & 31) == 0)
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+  if ((threadIdx.x & 31) == 0) {
+    if (release) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+    else asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+  }
 }
 // every thread of every CTA of the cluster
 __device__ __forceinline__ void cluster_sync() {
