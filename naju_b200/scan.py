@@ -121,7 +121,7 @@ def _ckpt_bytes_formula(B, T, D, N, act, bdt):
     """Size of the checkpoint buffer (naju_b200_ckpt_bytes) as arithmetic that also works on the
     symbolic sizes of fake tensors."""
     NS = 16 if N <= 16 else 32 if N <= 32 else 64 if N <= 64 else 128
-    TC = 64 if (N == 16 and act in (torch.bfloat16, torch.float16) and bdt == torch.bfloat16) else 32
+    TC = 64 if (N == 16 and act in (torch.bfloat16, torch.float16) and bdt == torch.bfloat16 and D % 8 == 0) else 32
     ntiles = ((T + TC - 1) // TC) * B * ((D + 127) // 128)
     a256 = lambda x: (x + 255) // 256 * 256
     return a256(ntiles * 128 * NS * 4) + a256(ntiles * 128 * 4) + 256
