@@ -1064,7 +1064,8 @@ int launch_bwd_tc(const BwdParams& p, const Geometry& g, int act, int gate, int 
   // channel tiles take 5 us per chunk in clusters of two, the recurrent kernel 0.22 us per tile.
   if (!(static_cast<int64_t>(g.B) * g.ndt * 4 >= tmah::sm_count() && g.nchunks >= 4)) return -1000;
   tcb::Maps maps = {};
-  const bool ok =
+  // (du, in u's layout, leaves in 16-byte pieces where that is time-contiguous)
+  const bool ok = (p.u_sd == 1 || (reinterpret_cast<uintptr_t>(p.du) & 15) == 0) &&
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, tcb::SLAB, kDT)
                   : tmah::make_map(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_st, kDT, tcb::SLAB)) &&
       tmah::make_map(&maps.fl, p.fl, gate, g.B, g.T, g.D, p.fl_sb, p.fl_st, kDT, tcb::SLAB) &&

@@ -755,7 +755,8 @@ int launch_bwd_wide(const BwdParams& p, const Geometry& g, int act, int gate, in
   if (!(g.N > 16 && g.NS <= 64 && g.TC == wideb::Q && act == NAJU_BF16 && gate == NAJU_BF16 && bc == NAJU_BF16)) return -1000;
   if (!wide_walk_pays(g, tmah::sm_count())) return -1000;
   wideb::Maps maps;
-  const bool ok =
+  // (du, in u's layout, leaves in 16-byte pieces where that is time-contiguous)
+  const bool ok = (p.u_sd == 1 || (reinterpret_cast<uintptr_t>(p.du) & 15) == 0) &&
       (p.u_sd > 1 ? tmah::make_map_tmajor(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_sd, wideb::SLAB, kDT)
                   : tmah::make_map(&maps.u, p.u, act, g.B, g.T, g.D, p.u_sb, p.u_st, kDT, wideb::SLAB)) &&
       tmah::make_map(&maps.fl, p.fl, gate, g.B, g.T, g.D, p.fl_sb, p.fl_st, kDT, wideb::SLAB) &&

@@ -79,16 +79,24 @@ __device__ __forceinline__ bool vec4_ok(const T* base, int64_t row_stride) {
   return (reinterpret_cast<uintptr_t>(base) % (4 * sizeof(T))) == 0 && row_stride % 4 == 0;
 }
 
+// Whether 16 bytes of consecutive steps can be moved at once in a time-contiguous tensor.
+template <typename T>
+__device__ __forceinline__ bool vec_steps_ok(const T* base, int64_t sd) {
+  return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sd * static_cast<int64_t>(sizeof(T)) % 16 == 0;
+}
+
 // A time-contiguous source (element (step r, channel c) at src[c * sd + r]) into a [kSB][128] fp32 tile:
-// thread = channel, 16 bytes of its steps at a time.  `len` steps are real; the rest become zero.
+// thread = channel, 16 bytes of its steps at a time (element by element where the layout does not allow that).  `len` steps are
+// real; the rest become zero.
 template <typename T, int NT>
 __device__ __forceinline__ void load_tmajor(float* __restrict__ dst, const T* __restrict__ src, int64_t sd, int len,
                                             int cols, int tid) {
   constexpr int E = 16 / sizeof(T);
+  const bool vec = vec_steps_ok(src, sd);
   for (int i = tid; i < kDT * (kSB / E); i += NT) {
     const int c = i % kDT, r0 = (i / kDT) * E;
     T e[E];
-    if (c < cols && r0 + E <= len) {
+    if (vec && c < cols && r0 + E <= len) {
       *reinterpret_cast<uint4*>(e) = __ldg(reinterpret_cast<const uint4*>(src + c * sd + r0));
     } else {
 #pragma unroll
@@ -102,13 +110,14 @@ template <typename T, int NT>
 __device__ __forceinline__ void store_tmajor(T* __restrict__ dst, const float* __restrict__ src, int64_t sd, int len,
                                              int cols, int tid) {
   constexpr int E = 16 / sizeof(T);
+  const bool vec = vec_steps_ok(dst, sd);
   for (int i = tid; i < kDT * (kSB / E); i += NT) {
     const int c = i % kDT, r0 = (i / kDT) * E;
     if (c >= cols || r0 >= len) continue;
     T e[E];
 #pragma unroll
     for (int k = 0; k < E; ++k) e[k] = from_f32<T>(src[(r0 + k) * kDT + c]);
-    if (r0 + E <= len) {
+    if (vec && r0 + E <= len) {
       *reinterpret_cast<uint4*>(dst + c * sd + r0) = *reinterpret_cast<const uint4*>(e);
     } else {
       for (int k = 0; k < E; ++k)
