@@ -111,7 +111,7 @@ Args prepare(const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& 
   TORCH_CHECK(dtype_code(u.scalar_type()) >= 0, "unsupported dtype ", u.scalar_type());
   const auto gdt = gate_type(u, fl, il), bdt = bc_type(Bm, Cm);
   return {time_contig(u) ? u : inner_contig(u), inner_contig(as_type(fl, gdt)), inner_contig(as_type(il, gdt)),
-          inner_contig(as_type(Bm, bdt)), inner_contig(as_type(Cm, bdt)), as_type(D.detach(), at::kFloat).contiguous()};
+          inner_contig(as_type(Bm, bdt)), inner_contig(as_type(Cm, bdt)), as_type(D, at::kFloat).contiguous()};
 }
 
 naju_scan_desc describe(const Args& a, int flags) {
@@ -141,7 +141,7 @@ naju_scan_desc describe(const Args& a, int flags) {
 Tensor state_arg(const Tensor& h, int64_t B, int64_t D, int64_t N, const char* name) {
   if (!h.defined()) return h;
   TORCH_CHECK_VALUE(h.dim() == 3 && h.size(0) == B && h.size(1) == D && h.size(2) == N, name, " must be [B, D, N]");
-  return as_type(h.detach(), at::kFloat).contiguous();
+  return as_type(h, at::kFloat).contiguous();
 }
 
 // ------------------------------------------------------------------------------ fewer than 16 states
@@ -315,7 +315,9 @@ std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor&
   Args a;
   Tensor ph0;
   {
-    at::AutoDispatchBelowADInplaceOrView below;  // nothing in here is recorded: the node is
+    // Nothing in here is recorded: the node is.  (A tensor that needs no conversion is the caller's own, with its version counter,
+    // so that the node notices a change in place before its backward.  A detach() in here would not share the counter.)
+    at::AutoDispatchBelowADInplaceOrView below;
     a = prepare(u, fl, il, Bm, Cm, D);
     ph0 = state_arg(h0, a.u.size(0), a.u.size(2), a.Bm.size(2), "h0");
     o = forward(a, ph0, want_final, false, call_flags());
@@ -433,7 +435,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("version", []() { return naju_b200_version(); });
   m.def("time_contig", &time_contig);
   m.def("prepare", [](const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm, const Tensor& D) {
-    const Args a = prepare(u, fl, il, Bm, Cm, D);
+    const Args a = prepare(u, fl, il, Bm, Cm, D.detach());
     return std::make_tuple(a.u, a.fl, a.il, a.Bm, a.Cm, a.D);
   });
   m.def("describe", [](const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm) {
@@ -441,7 +443,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return desc_bytes(d);
   });
   m.def("state_arg", [](const OptTensor& h, int64_t B, int64_t D, int64_t N, const std::string& name) {
-    return ret(state_arg(opt(h), B, D, N, name.c_str()));
+    const Tensor t = opt(h);
+    return ret(state_arg(t.defined() ? t.detach() : t, B, D, N, name.c_str()));
   });
   m.def("forward", [](const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm, const Tensor& D,
                       const OptTensor& h0, bool want_final, bool want_decay) {
