@@ -245,6 +245,10 @@ BwdOut backward(const Args& in, const Tensor& h0_in, const Tensor& dy_in, const 
   }
   const int64_t Np = a.Bm.size(2);
   const naju_scan_desc d = describe(a, flags);
+  // (the padding of fewer than 16 states, and with it the checkpoints' layout, depends on NAJU_B200_FORM)
+  const int64_t want = std::max<int64_t>(static_cast<int64_t>(naju_b200_ckpt_bytes(&d)), 256);
+  TORCH_CHECK(ckpt.numel() == want, "checkpoint buffer of ", ckpt.numel(), " bytes where this call's layout has ", want,
+              ": NAJU_B200_FORM has changed since the forward, or the buffer belongs to another call");
   c10::cuda::CUDAGuard guard(a.u.device());
   const auto f32 = a.u.options().dtype(at::kFloat);
   BwdOut o;
@@ -279,6 +283,7 @@ struct ScanBackward : public torch::autograd::Node {
   SavedVariable u, fl, il, Bm, Cm, D, h0, ckpt;
   at::ScalarType in_types[7];
   bool want_final = false;
+  int flags = 0;   // the forward's: they decide how the checkpoints are laid out
 
   std::string name() const override { return "NajuScanBackward"; }
 
@@ -296,7 +301,7 @@ struct ScanBackward : public torch::autograd::Node {
     if (want_final && grads.size() > 1 && grads[1].defined())
       dhT = state_arg(grads[1], a.u.size(0), a.u.size(2), a.Bm.size(2), "dhT");
     const bool want_dh0 = h.defined() && task_should_compute_output(6);
-    const BwdOut o = backward(a, h, dy, dhT, ckpt.unpack(), want_dh0, call_flags());
+    const BwdOut o = backward(a, h, dy, dhT, ckpt.unpack(), want_dh0, flags);
     variable_list out(7);
     const Tensor* g[7] = {&o.du, &o.dfl, &o.dil, &o.dB, &o.dC, &o.dD, &o.dh0};
     for (size_t i = 0; i < 7; ++i)
@@ -314,19 +319,21 @@ std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor&
   FwdOut o;
   Args a;
   Tensor ph0;
+  const int flags = call_flags();
   {
     // Nothing in here is recorded: the node is.  (A tensor that needs no conversion is the caller's own, with its version counter,
     // so that the node notices a change in place before its backward.  A detach() in here would not share the counter.)
     at::AutoDispatchBelowADInplaceOrView below;
     a = prepare(u, fl, il, Bm, Cm, D);
     ph0 = state_arg(h0, a.u.size(0), a.u.size(2), a.Bm.size(2), "h0");
-    o = forward(a, ph0, want_final, false, call_flags());
+    o = forward(a, ph0, want_final, false, flags);
   }
   if (grad) {
     auto node = std::shared_ptr<ScanBackward>(new ScanBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(u, fl, il, Bm, Cm, D, h0));
     for (int i = 0; i < 7; ++i) node->in_types[i] = in[i]->defined() ? in[i]->scalar_type() : at::kFloat;
     node->want_final = want_final;
+    node->flags = flags;
     node->u = SavedVariable(a.u, false);
     node->fl = SavedVariable(a.fl, false);
     node->il = SavedVariable(a.il, false);

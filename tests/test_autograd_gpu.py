@@ -28,3 +28,24 @@ def test_a_change_in_place_before_the_backward_is_noticed(which):
         t[which].add_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.sum().backward()
+
+
+def test_the_backward_keeps_the_forward_s_form(monkeypatch):
+    """Fewer than 16 states are padded or not by NAJU_B200_FORM; the checkpoints of one layout are not read as the other's."""
+    from naju_b200.scan import _desc, _prepare, scan_backward, scan_forward
+    t = [x.requires_grad_(True) for x in _inputs(2, 512, 2048, 8, BF)]
+    dy = torch.ones_like(t[0])
+    want = torch.autograd.grad(_scan(t), t, dy)
+    for first, then in (("auto", "recurrent"), ("recurrent", "auto")):
+        monkeypatch.setenv("NAJU_B200_FORM", first)
+        y = _scan(t)
+        monkeypatch.setenv("NAJU_B200_FORM", then)
+        for a, b in zip(torch.autograd.grad(y, t, dy), want):   # (two kernels apart: 16-bit operands, 2e-3 of bf16 gradients)
+            assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 2e-3
+        # the raw calls name the mistake
+        monkeypatch.setenv("NAJU_B200_FORM", first)
+        p = _prepare(*[x.detach() for x in t[:6]])
+        ckpt = scan_forward(*p)[3]
+        monkeypatch.setenv("NAJU_B200_FORM", then)
+        with pytest.raises(RuntimeError, match="NAJU_B200_FORM has changed"):
+            scan_backward(_desc(*p[:5]), *p, None, dy, None, ckpt)
