@@ -14,6 +14,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/core/AutogradState.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -313,6 +314,10 @@ struct ScanBackward : public torch::autograd::Node {
 std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm,
                                 const Tensor& D, const Tensor& h0, bool want_final) {
   const Tensor* in[7] = {&u, &fl, &il, &Bm, &Cm, &D, &h0};
+  if (c10::AutogradState::get_tls_state().get_fw_grad_mode())
+    for (const Tensor* t : in)
+      TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                  "the scan has no forward-mode derivative (jvp): use reverse mode");
   bool grad = false;
   if (at::GradMode::is_enabled())
     for (const Tensor* t : in) grad = grad || (t->defined() && t->requires_grad());

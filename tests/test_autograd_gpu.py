@@ -49,3 +49,23 @@ def test_the_backward_keeps_the_forward_s_form(monkeypatch):
         monkeypatch.setenv("NAJU_B200_FORM", then)
         with pytest.raises(RuntimeError, match="NAJU_B200_FORM has changed"):
             scan_backward(_desc(*p[:5]), *p, None, dy, None, ckpt)
+
+
+@pytest.mark.parametrize("which", range(7))
+@pytest.mark.parametrize("grad", [True, False])
+def test_forward_mode_is_refused(which, grad):
+    """A dual input raises, as any autograd function without a jvp does; its tangent is not dropped."""
+    import torch.autograd.forward_ad as fwAD
+    t = _inputs()
+    with fwAD.dual_level(), torch.set_grad_enabled(grad):
+        t[which] = fwAD.make_dual(t[which], torch.ones_like(t[which]))
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            _scan(t)
+
+
+def test_function_transforms_are_refused():
+    t = _inputs()
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda u: _scan([u] + t[1:]).sum())(t[0])
+    with pytest.raises((RuntimeError, ValueError)):
+        torch.func.vmap(lambda u: _scan([u] + t[1:]))(torch.stack([t[0], t[0]]))
