@@ -16,10 +16,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/core/AutogradState.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
-#include <torch/csrc/autograd/saved_variable.h>
 
 #include <cctype>
 #include <cstdlib>
@@ -34,7 +32,6 @@
 namespace {
 
 using at::Tensor;
-using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
 // ------------------------------------------------------------------------------ switches
@@ -205,7 +202,7 @@ struct FwdOut {
   naju_scan_desc desc;   // of the call as it was made (states padded where the rule says so)
 };
 
-FwdOut forward(const Args& in, const Tensor& h0_in, bool want_final, bool want_decay, int flags) {
+FwdOut naju_forward(const Args& in, const Tensor& h0_in, bool want_final, bool want_decay, int flags) {
   Args a = in;
   Tensor h0 = h0_in;
   const int64_t B = a.u.size(0), T = a.u.size(1), D = a.u.size(2), N = a.Bm.size(2);
@@ -236,7 +233,7 @@ struct BwdOut {
   Tensor du, dfl, dil, dB, dC, dD, dh0;
 };
 
-BwdOut backward(const Args& in, const Tensor& h0_in, const Tensor& dy_in, const Tensor& dhT_in, const Tensor& ckpt,
+BwdOut naju_backward(const Args& in, const Tensor& h0_in, const Tensor& dy_in, const Tensor& dhT_in, const Tensor& ckpt,
                 bool want_dh0, int flags) {
   Args a = in;
   Tensor h0 = h0_in, dhT = dhT_in;
@@ -278,36 +275,61 @@ BwdOut backward(const Args& in, const Tensor& h0_in, const Tensor& dy_in, const 
 }
 
 // ------------------------------------------------------------------------------ autograd
-// Counterpart of _NajuCudaFn (naju/cuda/__init__.py:38-63) as a native node: the prepared inputs and
+// Counterpart of _NajuCudaFn (naju/cuda/__init__.py:38-63) as a native autograd function: the prepared inputs and
 // the forward's checkpoints are saved, the gradients come back in each input's own type.
-struct ScanBackward : public torch::autograd::Node {
-  SavedVariable u, fl, il, Bm, Cm, D, h0, ckpt;
-  at::ScalarType in_types[7];
-  bool want_final = false;
-  int flags = 0;   // the forward's: they decide how the checkpoints are laid out
+static_assert(static_cast<int>(at::ScalarType::NumOptions) <= 64, "a type fits six bits");
 
-  std::string name() const override { return "NajuScanBackward"; }
-
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&u, &fl, &il, &Bm, &Cm, &D, &h0, &ckpt}) s->reset_data();
+struct NajuScan : public torch::autograd::Function<NajuScan> {
+  static variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& u, const Tensor& fl, const Tensor& il,
+                               const Tensor& Bm, const Tensor& Cm, const Tensor& D, const std::optional<Tensor>& h0_in,
+                               bool want_final) {
+    const Tensor h0 = h0_in.has_value() ? *h0_in : Tensor();
+    const Tensor* in[7] = {&u, &fl, &il, &Bm, &Cm, &D, &h0};
+    const int flags = call_flags();
+    Args a;
+    Tensor ph0;
+    const FwdOut o = run(u, fl, il, Bm, Cm, D, h0, want_final, flags, a, ph0);
+    ctx->save_for_backward({a.u, a.fl, a.il, a.Bm, a.Cm, a.D, ph0, o.ckpt});
+    ctx->set_materialize_grads(false);
+    // One number for what is not a tensor: the forward's flags (they decide how the checkpoints are laid out), whether the final state was
+    // asked for, the inputs' types (six bits each).
+    int64_t meta = flags | (want_final ? 1 << 8 : 0);
+    for (int i = 0; i < 7; ++i)
+      if (in[i]->defined()) meta |= static_cast<int64_t>(in[i]->scalar_type()) << (16 + 6 * i);
+    ctx->saved_data["meta"] = meta;
+    return want_final ? variable_list{o.y, o.hT} : variable_list{o.y};
   }
 
-  variable_list apply(variable_list&& grads) override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    const Args a{u.unpack(), fl.unpack(), il.unpack(), Bm.unpack(), Cm.unpack(), D.unpack()};
-    const Tensor h = h0.unpack();
+  static variable_list backward(torch::autograd::AutogradContext* ctx, const variable_list& grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const int64_t meta = ctx->saved_data["meta"].toInt();
+    const Args a{s[0], s[1], s[2], s[3], s[4], s[5]};
+    const Tensor& h = s[6];
     const Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(a.u);
     Tensor dhT;
-    if (want_final && grads.size() > 1 && grads[1].defined())
+    if ((meta & (1 << 8)) != 0 && grads.size() > 1 && grads[1].defined())
       dhT = state_arg(grads[1], a.u.size(0), a.u.size(2), a.Bm.size(2), "dhT");
-    const bool want_dh0 = h.defined() && task_should_compute_output(6);
-    const BwdOut o = backward(a, h, dy, dhT, ckpt.unpack(), want_dh0, flags);
-    variable_list out(7);
+    const bool want_dh0 = h.defined() && ctx->needs_input_grad(6);
+    BwdOut o;
+    {
+      at::AutoDispatchBelowADInplaceOrView below;
+      o = naju_backward(a, h, dy, dhT, s[7], want_dh0, static_cast<int>(meta & 0xFF));
+    }
+    variable_list out(8);
     const Tensor* g[7] = {&o.du, &o.dfl, &o.dil, &o.dB, &o.dC, &o.dD, &o.dh0};
     for (size_t i = 0; i < 7; ++i)
-      if (g[i]->defined() && task_should_compute_output(i)) out[i] = as_type(*g[i], in_types[i]);
+      if (g[i]->defined() && ctx->needs_input_grad(i)) out[i] = as_type(*g[i], static_cast<at::ScalarType>(meta >> (16 + 6 * i) & 63));
     return out;
+  }
+
+  static FwdOut run(const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm, const Tensor& D,
+                    const Tensor& h0, bool want_final, int flags, Args& a, Tensor& ph0) {
+    // Nothing in here is recorded.  (A tensor that needs no conversion is the caller's own, with its version counter, so that a
+    // change in place before the backward is noticed.  A detach() in here would not share the counter.)
+    at::AutoDispatchBelowADInplaceOrView below;
+    a = prepare(u, fl, il, Bm, Cm, D);
+    ph0 = state_arg(h0, a.u.size(0), a.u.size(2), a.Bm.size(2), "h0");
+    return naju_forward(a, ph0, want_final, false, flags);
   }
 };
 
@@ -321,35 +343,13 @@ std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor&
   bool grad = false;
   if (at::GradMode::is_enabled())
     for (const Tensor* t : in) grad = grad || (t->defined() && t->requires_grad());
-  FwdOut o;
+  if (grad) {
+    const variable_list o = NajuScan::apply(u, fl, il, Bm, Cm, D, h0.defined() ? std::optional<Tensor>(h0) : std::nullopt, want_final);
+    return {o[0], want_final ? o[1] : Tensor()};
+  }
   Args a;
   Tensor ph0;
-  const int flags = call_flags();
-  {
-    // Nothing in here is recorded: the node is.  (A tensor that needs no conversion is the caller's own, with its version counter,
-    // so that the node notices a change in place before its backward.  A detach() in here would not share the counter.)
-    at::AutoDispatchBelowADInplaceOrView below;
-    a = prepare(u, fl, il, Bm, Cm, D);
-    ph0 = state_arg(h0, a.u.size(0), a.u.size(2), a.Bm.size(2), "h0");
-    o = forward(a, ph0, want_final, false, flags);
-  }
-  if (grad) {
-    auto node = std::shared_ptr<ScanBackward>(new ScanBackward(), torch::autograd::deleteNode);
-    node->set_next_edges(torch::autograd::collect_next_edges(u, fl, il, Bm, Cm, D, h0));
-    for (int i = 0; i < 7; ++i) node->in_types[i] = in[i]->defined() ? in[i]->scalar_type() : at::kFloat;
-    node->want_final = want_final;
-    node->flags = flags;
-    node->u = SavedVariable(a.u, false);
-    node->fl = SavedVariable(a.fl, false);
-    node->il = SavedVariable(a.il, false);
-    node->Bm = SavedVariable(a.Bm, false);
-    node->Cm = SavedVariable(a.Cm, false);
-    node->D = SavedVariable(a.D, false);
-    node->h0 = SavedVariable(ph0, false);
-    node->ckpt = SavedVariable(o.ckpt, false);
-    torch::autograd::set_history(o.y, node);
-    if (want_final) torch::autograd::set_history(o.hT, node);
-  }
+  const FwdOut o = NajuScan::run(u, fl, il, Bm, Cm, D, h0, want_final, call_flags(), a, ph0);
   return {o.y, o.hT};
 }
 
@@ -461,14 +461,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("forward", [](const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm, const Tensor& D,
                       const OptTensor& h0, bool want_final, bool want_decay) {
     at::NoGradGuard ng;
-    const FwdOut o = forward({u, fl, il, Bm, Cm, D}, opt(h0), want_final, want_decay, call_flags());
+    const FwdOut o = naju_forward({u, fl, il, Bm, Cm, D}, opt(h0), want_final, want_decay, call_flags());
     return std::make_tuple(o.y, ret(o.hT), ret(o.pT), o.ckpt, desc_bytes(o.desc));
   });
   m.def("backward", [](int flags, const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm,
                        const Tensor& D, const OptTensor& h0, const Tensor& dy, const OptTensor& dhT, const Tensor& ckpt,
                        bool want_dh0) {
     at::NoGradGuard ng;
-    const BwdOut o = backward({u, fl, il, Bm, Cm, D}, opt(h0), dy, opt(dhT), ckpt, want_dh0, flags);
+    const BwdOut o = naju_backward({u, fl, il, Bm, Cm, D}, opt(h0), dy, opt(dhT), ckpt, want_dh0, flags);
     return std::make_tuple(o.du, o.dfl, o.dil, o.dB, o.dC, o.dD, ret(o.dh0));
   });
   m.def("forms", []() { return std::make_pair(g_form_fwd.load(), g_form_bwd.load()); });

@@ -69,3 +69,39 @@ def test_function_transforms_are_refused():
         torch.func.grad(lambda u: _scan([u] + t[1:]).sum())(t[0])
     with pytest.raises((RuntimeError, ValueError)):
         torch.func.vmap(lambda u: _scan([u] + t[1:]))(torch.stack([t[0], t[0]]))
+
+
+@pytest.mark.parametrize("want_final", [False, True])
+def test_compiled_autograd_around_an_eager_call(want_final):
+    """The backward of an eager call under compiled autograd gives the eager backward's gradients."""
+    t = [x.requires_grad_(True) for x in _inputs()]
+
+    def loss():
+        if not want_final:
+            return _scan(t).square().mean()
+        y, hT = _scan(t, return_final_state=True)
+        return y.square().mean() + hT.square().mean()
+
+    loss().backward()
+    want = [x.grad.clone() for x in t]
+    for x in t:
+        x.grad = None
+    with torch._dynamo.compiled_autograd._enable(torch.compile(backend="eager")):
+        loss().backward()
+    for x, w in zip(t, want):
+        assert torch.allclose(x.grad, w, rtol=1e-5, atol=1e-8)
+
+
+def test_saved_tensors_and_a_second_backward():
+    """Saved-tensor hooks see what the node saves; a second backward without retain_graph is refused, with it repeats itself."""
+    t = [x.requires_grad_(True) for x in _inputs()]
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda x: seen.append(x) or x.cpu(), lambda x: x.cuda()):
+        y = _scan(t)
+    assert len(seen) == 8
+    a = torch.autograd.grad(y.sum(), t, retain_graph=True)
+    b = torch.autograd.grad(y.sum(), t)
+    for p, q in zip(a, b):
+        assert torch.allclose(p, q, rtol=1e-5, atol=1e-7)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(y.sum(), t)
