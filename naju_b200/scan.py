@@ -216,8 +216,16 @@ def _scan_via_custom_op(u, f_logit, i_logit, B, C, D_skip, h0, want_final):
     return (y, hT) if want_final else y
 
 
+def _by_custom_op():
+    """Whether a compiler or a tracer is looking: it then has to find one op (what the native function does inside would be
+    recorded as the allocation of its outputs and nothing else)."""
+    return torch.compiler.is_compiling() or torch.jit.is_tracing()
+
+
 def naju_b200_scan(u, f_logit, i_logit, B, C, D_skip):
     """Backend callable with the reference's 6-tensor signature (naju/scan.py:3-5)."""
+    if _by_custom_op():
+        return _scan_via_custom_op(u, f_logit, i_logit, B, C, D_skip, None, False)
     return _native().scan(u, f_logit, i_logit, B, C, D_skip, None, False)
 
 
@@ -230,7 +238,7 @@ def naju_scan(u, f_logit, i_logit, B, C, D_skip, backend=None, *, h0=None,
     (y, hT) where hT [B,D,N] fp32 is the state after the last step.
     """
     resolve_backend(backend)
-    if torch.compiler.is_compiling():
+    if _by_custom_op():
         return _scan_via_custom_op(u, f_logit, i_logit, B, C, D_skip, h0, bool(return_final_state))
     return _native().scan(u, f_logit, i_logit, B, C, D_skip, h0, return_final_state)
 

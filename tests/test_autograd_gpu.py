@@ -105,3 +105,31 @@ def test_saved_tensors_and_a_second_backward():
         assert torch.allclose(p, q, rtol=1e-5, atol=1e-7)
     with pytest.raises(RuntimeError, match="second time"):
         torch.autograd.grad(y.sum(), t)
+
+
+@pytest.mark.parametrize("state", [False, True])
+def test_a_traced_scan_computes(state):
+    """torch.jit.trace records the scan, not the allocation of its outputs: on other inputs the traced function gives the eager
+    results, and their gradients."""
+    import warnings
+    from naju_b200 import naju_scan
+    from naju_b200.scan import naju_b200_scan
+
+    def fn(u, fl, il, B, C, D, h0):
+        if state:
+            y, hT = naju_scan(u * 2.0, fl, il, B, C, D, h0=h0, return_final_state=True)
+            return y, hT
+        return naju_scan(u * 2.0, fl, il, B, C, D) + naju_b200_scan(u, fl, il, B, C, D)
+
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        traced = torch.jit.trace(fn, tuple(_inputs(seed=1)), check_trace=False)
+    a, b = ([x.requires_grad_(True) for x in _inputs(seed=2)] for _ in range(2))
+    out, want = traced(*a), fn(*b)
+    out, want = (out, want) if state else ((out,), (want,))
+    for x, y in zip(out, want):
+        assert torch.allclose(x, y, rtol=1e-5, atol=1e-5)
+    sum(x.square().mean() for x in out).backward()
+    sum(x.square().mean() for x in want).backward()
+    for x, y in zip(a[:6 + state], b):
+        assert torch.allclose(x.grad, y.grad, rtol=1e-4, atol=1e-7)
