@@ -354,6 +354,14 @@ std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor&
 }
 
 // ------------------------------------------------------------------------------ decode step
+// A row operand of the step as the kernel takes it: inner stride 1, rows at least a row apart.  Rows that overlap or repeat (an operand
+// broadcast over the batch) are copied; with one row only the stride means nothing.
+Tensor step_rows(const Tensor& t) {
+  const Tensor r = inner_contig(t);
+  return r.size(0) > 1 && r.stride(0) < r.size(1) ? r.contiguous() : r;
+}
+int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
+
 // state [B,D,N] fp32 is updated in place; u, f_logit, i_logit [B,D]; B, C [B,N].
 Tensor step(const Tensor& state, const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm,
             const Tensor& D) {
@@ -372,16 +380,16 @@ Tensor step(const Tensor& state, const Tensor& u, const Tensor& fl, const Tensor
   at::AutoDispatchBelowADInplaceOrView below;
   c10::cuda::CUDAGuard guard(state.device());
   const auto gdt = gate_type(u, fl, il), bdt = bc_type(Bm, Cm);
-  const Tensor pu = inner_contig(u), pf = inner_contig(as_type(fl, gdt)), pi = inner_contig(as_type(il, gdt)),
-               pB = inner_contig(as_type(Bm, bdt)), pC = inner_contig(as_type(Cm, bdt)),
+  const Tensor pu = step_rows(u), pf = step_rows(as_type(fl, gdt)), pi = step_rows(as_type(il, gdt)), pB = step_rows(as_type(Bm, bdt)),
+               pC = step_rows(as_type(Cm, bdt)),
                pD = as_type(D, at::kFloat).contiguous();
   naju_scan_desc d{};
   d.B = static_cast<int32_t>(B); d.T = 1; d.D = static_cast<int32_t>(Dc); d.N = static_cast<int32_t>(N);
   d.act_dtype = dtype_code(pu.scalar_type());
   d.gate_dtype = dtype_code(gdt);
   d.bc_dtype = dtype_code(bdt);
-  d.u_sb = std::max(pu.stride(0), Dc); d.fl_sb = std::max(pf.stride(0), Dc); d.il_sb = std::max(pi.stride(0), Dc);
-  d.bm_sb = std::max(pB.stride(0), N); d.cm_sb = std::max(pC.stride(0), N);
+  d.u_sb = row_stride(pu); d.fl_sb = row_stride(pf); d.il_sb = row_stride(pi);
+  d.bm_sb = row_stride(pB); d.cm_sb = row_stride(pC);
   Tensor y = at::empty({B, Dc}, pu.options());
   check(naju_b200_step(&d, static_cast<float*>(state.data_ptr()), ptr(pu), ptr(pf), ptr(pi), ptr(pB), ptr(pC), fptr(pD),
                        mptr(y), stream_of(state)),
