@@ -82,6 +82,54 @@ int naju::launch_init(ScratchHeader* hdr, size_t bytes, int* trailer, cudaStream
                     reinterpret_cast<uint4*>(hdr), n16, trailer);
 }
 
+int naju::forward_with_geometry(const naju_scan_desc* desc, const Geometry& g, const void* u, const void* f_logit,
+                                const void* i_logit, const void* Bm, const void* Cm, const float* D_skip, const float* h0, void* y,
+                                float* hT, float* pT, void* ckpt, void* scratch, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int64_t nstate = static_cast<int64_t>(desc->B) * desc->D * desc->N;
+  const int64_t nchan = static_cast<int64_t>(desc->B) * desc->D;
+  if (desc->B == 0 || desc->D == 0) return NAJU_OK;
+  if (desc->T == 0) {  // empty time axis: the state passes through unchanged
+    if (hT) copy_state_kernel<<<static_cast<unsigned>((nstate + 255) / 256), 256, 0, st>>>(h0, hT, nstate, 0.f);
+    if (pT) copy_state_kernel<<<static_cast<unsigned>((nchan + 255) / 256), 256, 0, st>>>(nullptr, pT, nchan, 1.f);
+    return static_cast<int>(cudaGetLastError());
+  }
+  if (!u || !f_logit || !i_logit || !Bm || !Cm || !D_skip || !y) return NAJU_E_NULL;
+  if (!ckpt || !scratch || !aligned(ckpt, 256) || !aligned(scratch, 256)) return NAJU_E_WORKSPACE;
+  if (const int rc = check_strides(desc); rc != NAJU_OK) return rc;
+  if (!aligned(u, dtype_size(desc->act_dtype)) || !aligned(y, dtype_size(desc->act_dtype)) ||
+      !aligned(f_logit, dtype_size(desc->gate_dtype)) || !aligned(i_logit, dtype_size(desc->gate_dtype)) ||
+      !aligned(Bm, dtype_size(desc->bc_dtype)) || !aligned(Cm, dtype_size(desc->bc_dtype)))
+    return NAJU_E_ALIGN;
+
+  const CkptLayout cl = ckpt_layout(g);
+  const FwdScratchLayout sl = fwd_scratch_layout(g);
+  char* ck = static_cast<char*>(ckpt);
+  char* sc = static_cast<char*>(scratch);
+
+  FwdParams p;
+  fill_common(p, desc, g);
+  p.inject = (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0;
+  p.u = u; p.fl = f_logit; p.il = i_logit; p.Bm = Bm; p.Cm = Cm; p.Dskip = D_skip; p.h0 = h0;
+  p.y = y; p.hT = hT; p.pT = pT;
+  p.ckS = reinterpret_cast<float*>(ck + cl.off_S);
+  p.ckP = reinterpret_cast<float*>(ck + cl.off_P);
+  p.fwd_form = reinterpret_cast<int*>(ck + cl.off_trailer);
+  p.hdr = reinterpret_cast<ScratchHeader*>(sc);
+  p.flags = reinterpret_cast<int*>(sc + sl.off_flags);
+  p.aggP = reinterpret_cast<float*>(sc + sl.off_aggP);
+  p.aggS = reinterpret_cast<float*>(sc + sl.off_aggS);
+  int rck = -1000;
+  if (!(desc->flags & NAJU_FLAG_RECURRENT_ONLY)) {
+    rck = launch_fwd_tc3(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
+    if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;   // (the flag asks for the 16-state form)
+    if (rck == -1000) rck = launch_fwd_wide(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
+  }
+  if (rck == -1000) rck = launch_fwd_chan(p, g, desc->act_dtype, desc->gate_dtype, stream);
+  if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
+  return rck;
+}
+
 extern "C" {
 
 int naju_b200_version(void) { return NAJU_B200_ABI_VERSION; }
@@ -134,52 +182,9 @@ int naju_b200_fwd(const naju_scan_desc* desc, const void* u, const void* f_logit
                   const void* i_logit, const void* Bm, const void* Cm, const float* D_skip,
                   const float* h0, void* y, float* hT, float* pT, void* ckpt, void* scratch,
                   void* stream) {
-  int rc = check_desc(desc, true);
+  const int rc = check_desc(desc, true);
   if (rc != NAJU_OK) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t nstate = static_cast<int64_t>(desc->B) * desc->D * desc->N;
-  const int64_t nchan = static_cast<int64_t>(desc->B) * desc->D;
-  if (desc->B == 0 || desc->D == 0) return NAJU_OK;
-  if (desc->T == 0) {  // empty time axis: the state passes through unchanged
-    if (hT) copy_state_kernel<<<static_cast<unsigned>((nstate + 255) / 256), 256, 0, st>>>(h0, hT, nstate, 0.f);
-    if (pT) copy_state_kernel<<<static_cast<unsigned>((nchan + 255) / 256), 256, 0, st>>>(nullptr, pT, nchan, 1.f);
-    return static_cast<int>(cudaGetLastError());
-  }
-  if (!u || !f_logit || !i_logit || !Bm || !Cm || !D_skip || !y) return NAJU_E_NULL;
-  if (!ckpt || !scratch || !aligned(ckpt, 256) || !aligned(scratch, 256)) return NAJU_E_WORKSPACE;
-  if ((rc = check_strides(desc)) != NAJU_OK) return rc;
-  if (!aligned(u, dtype_size(desc->act_dtype)) || !aligned(y, dtype_size(desc->act_dtype)) ||
-      !aligned(f_logit, dtype_size(desc->gate_dtype)) || !aligned(i_logit, dtype_size(desc->gate_dtype)) ||
-      !aligned(Bm, dtype_size(desc->bc_dtype)) || !aligned(Cm, dtype_size(desc->bc_dtype)))
-    return NAJU_E_ALIGN;
-
-  const Geometry g = make_geometry(*desc);
-  const CkptLayout cl = ckpt_layout(g);
-  const FwdScratchLayout sl = fwd_scratch_layout(g);
-  char* ck = static_cast<char*>(ckpt);
-  char* sc = static_cast<char*>(scratch);
-
-  FwdParams p;
-  fill_common(p, desc, g);
-  p.inject = (desc->flags & NAJU_FLAG_INJECT_TIMEOUT) != 0;
-  p.u = u; p.fl = f_logit; p.il = i_logit; p.Bm = Bm; p.Cm = Cm; p.Dskip = D_skip; p.h0 = h0;
-  p.y = y; p.hT = hT; p.pT = pT;
-  p.ckS = reinterpret_cast<float*>(ck + cl.off_S);
-  p.ckP = reinterpret_cast<float*>(ck + cl.off_P);
-  p.fwd_form = reinterpret_cast<int*>(ck + cl.off_trailer);
-  p.hdr = reinterpret_cast<ScratchHeader*>(sc);
-  p.flags = reinterpret_cast<int*>(sc + sl.off_flags);
-  p.aggP = reinterpret_cast<float*>(sc + sl.off_aggP);
-  p.aggS = reinterpret_cast<float*>(sc + sl.off_aggS);
-  int rck = -1000;
-  if (!(desc->flags & NAJU_FLAG_RECURRENT_ONLY)) {
-    rck = launch_fwd_tc3(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
-    if (rck == -1000 && (desc->flags & NAJU_FLAG_CHUNKED_ONLY)) return NAJU_E_UNSUPPORTED;   // (the flag asks for the 16-state form)
-    if (rck == -1000) rck = launch_fwd_wide(p, g, desc->act_dtype, desc->gate_dtype, desc->bc_dtype, stream);
-  }
-  if (rck == -1000) rck = launch_fwd_chan(p, g, desc->act_dtype, desc->gate_dtype, stream);
-  if (rck == -1000) rck = launch_fwd_simt(p, g, desc->act_dtype, desc->gate_dtype, stream);
-  return rck;
+  return forward_with_geometry(desc, make_geometry(*desc), u, f_logit, i_logit, Bm, Cm, D_skip, h0, y, hT, pT, ckpt, scratch, stream);
 }
 
 int naju_b200_bwd(const naju_scan_desc* desc, const void* u, const void* f_logit,

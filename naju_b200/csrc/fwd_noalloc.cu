@@ -26,6 +26,7 @@
 #include <mutex>
 
 #include "naju_b200.h"
+#include "params.h"
 
 namespace {
 
@@ -67,15 +68,26 @@ extern "C" int naju_b200_fwd_noalloc(const naju_scan_desc* desc, const void* u, 
   if (desc == nullptr) return NAJU_E_NULL;
   if (desc->N < 1 || desc->N > 128 || desc->B < 0 || desc->T < 0 || desc->D < 0) return NAJU_E_SHAPE;
   const size_t ck = naju_b200_ckpt_bytes(desc);
-  const size_t sc = align256(naju_b200_fwd_scratch_bytes(desc));
-  if (ck + sc > static_cast<size_t>(NAJU_B200_NOALLOC_BYTES)) return NAJU_E_TOO_LARGE;
+  size_t sc = align256(naju_b200_fwd_scratch_bytes(desc));
+  int chunk_len = 0;   // the descriptor's own
+  if (ck + sc > static_cast<size_t>(NAJU_B200_NOALLOC_BYTES)) {
+    // Up to 32 states chunks of 64 steps will do where 32 are the faster choice, in half the memory.
+    if (desc->N > 32) return NAJU_E_TOO_LARGE;
+    chunk_len = 64;
+    const naju::Geometry g = naju::make_geometry(*desc, chunk_len);
+    sc = align256(naju::fwd_scratch_layout(g).bytes);
+    if (naju::ckpt_layout(g).bytes + sc > static_cast<size_t>(NAJU_B200_NOALLOC_BYTES)) return NAJU_E_TOO_LARGE;
+  }
   void* base = nullptr;
   const int rc = workspace_for_current_device(&base);
   if (rc != NAJU_OK) return rc;
   unsigned char* ws = static_cast<unsigned char*>(base);
-  // naju_b200_fwd() clears the part of the scratch that must start at zero (status word, tile
-  // ticket, chunk flags) with cudaMemsetAsync on `stream`; everything else is written before it
+  // The forward clears the part of the scratch that must start at zero (status word, tile
+  // ticket, chunk flags) by a kernel on `stream`; everything else is written before it
   // is read, so what the previous call left behind is harmless.
+  if (chunk_len > 0)
+    return naju::forward_with_geometry(desc, naju::make_geometry(*desc, chunk_len), u, f_logit, i_logit, Bm, Cm, D_skip, h0, y, hT,
+                                       nullptr, ws + sc, ws, stream);
   return naju_b200_fwd(desc, u, f_logit, i_logit, Bm, Cm, D_skip, h0, y, hT, nullptr, ws + sc, ws,
                        stream);
 }

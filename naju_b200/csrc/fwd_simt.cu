@@ -206,12 +206,11 @@ static int launch_tc(const FwdParams& p, const Geometry& g, cudaStream_t st) {
 template <typename TA, typename TG>
 static int launch_types(const FwdParams& p, const Geometry& g, cudaStream_t st) {
   if (g.NS == 16) {
-    // (64-step chunks belong to the types that the tensor-core kernels take: geometry of params.h)
-    if constexpr (sizeof(TA) == 2)
-      if (g.TC == 64) return launch_tc<TA, TG, 16, 64>(p, g, st);
-    return launch_tc<TA, TG, 16, 32>(p, g, st);
+    // (64-step chunks belong to the types that the tensor-core kernels take, see params.h, and to problems too large for
+    // naju_b200_fwd_noalloc()'s workspace with 32)
+    return g.TC == 64 ? launch_tc<TA, TG, 16, 64>(p, g, st) : launch_tc<TA, TG, 16, 32>(p, g, st);
   }
-  if (g.NS == 32) return launch_tc<TA, TG, 32, 32>(p, g, st);
+  if (g.NS == 32) return g.TC == 64 ? launch_tc<TA, TG, 32, 64>(p, g, st) : launch_tc<TA, TG, 32, 32>(p, g, st);
   if (g.NS == 64) return launch_tc<TA, TG, 64, 32>(p, g, st);
   return launch_tc<TA, TG, 128, 32>(p, g, st);
 }

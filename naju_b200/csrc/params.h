@@ -26,11 +26,11 @@ struct Geometry {
   int64_t ntiles;  // nchunks * B * ndt
 };
 
-inline Geometry make_geometry(const naju_scan_desc& d) {
+inline Geometry make_geometry(const naju_scan_desc& d, int chunk_len = 0) {
   Geometry g;
   g.B = d.B; g.T = d.T; g.D = d.D; g.N = d.N;
   g.NS = padded_states(d.N);
-  g.TC = chunk_len_for(d);
+  g.TC = chunk_len > 0 ? chunk_len : chunk_len_for(d);
   g.nchunks = (d.T + g.TC - 1) / g.TC;
   g.ndt = (d.D + 127) / 128;
   g.ntiles = static_cast<int64_t>(g.nchunks) * d.B * g.ndt;
@@ -159,6 +159,12 @@ struct BwdParams {
   int64_t u_sb, u_st, fl_sb, fl_st, il_sb, il_st, bm_sb, bm_st, cm_sb, cm_st;
   int64_t u_sd;  // element stride between channels of u: 1, or > 1 for a time-contiguous u (then u_st == 1)
 };
+
+// naju_b200_fwd() with workspaces laid out for `g` (chunks of 64 steps where the descriptor's own are 32 are taken for up to 32
+// states, by the recurrent kernels).
+int forward_with_geometry(const naju_scan_desc* desc, const Geometry& g, const void* u, const void* f_logit, const void* i_logit,
+                          const void* Bm, const void* Cm, const float* D_skip, const float* h0, void* y, float* hT, float* pT,
+                          void* ckpt, void* scratch, void* stream);
 
 // launchers implemented in the .cu files; return a CUDA runtime error code (0 = ok)
 

@@ -78,3 +78,28 @@ def test_time_contiguous_u_of_any_alignment(dtypes, T, pad, u_off, du_off):
     mask = torch.ones(size, dtype=torch.bool, device="cuda")
     strided(mask, du_off).fill_(False)
     assert bool(torch.isnan(du_buf[mask]).all())
+
+
+@pytest.mark.parametrize("case", [(2, 6000, 1000, 16, F32, F32), (3, 4100, 1001, 16, BF, BF), (1, 9000, 700, 24, F32, F32), (1, 9100, 700, 24, BF, F32)])
+def test_noalloc_forward_of_problems_that_need_long_chunks(case):
+    """Above half of the built-in array the recurrent kernels take chunks of 64 steps: the results of the caller-workspace call with
+    its 32, up to the order of fp32 sums."""
+    from naju_b200 import _lib
+    from naju_b200.scan import _desc, scan_forward
+    lib = _lib.load()
+    B, T, D, N, act, gate = case
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    t = [r(B, T, D).to(act), (r(B, T, D) + 4).to(gate), r(B, T, D).to(gate), (r(B, T, N) / 4).to(act), (r(B, T, N) / 4).to(act), r(D)]
+    h0 = r(B, D, N)
+    d = _desc(*t[:5])
+    assert lib.naju_b200_ckpt_bytes(d) + lib.naju_b200_fwd_scratch_bytes(d) > _lib.NOALLOC_BYTES
+    stream = torch.cuda.current_stream().cuda_stream
+    y, hT = torch.full_like(t[0], float("nan")), torch.full_like(h0, float("nan"))
+    rc = lib.naju_b200_fwd_noalloc(d, *map(_p, t), _p(h0), _p(y), _p(hT), stream)
+    assert rc == 0, _lib.strerror(rc)
+    torch.cuda.synchronize()
+    assert lib.naju_b200_noalloc_read_status(stream) == 0 and lib.naju_b200_noalloc_read_form(stream) == _lib.FORM_RECURRENT
+    y_ref, hT_ref, *_ = scan_forward(*t, h0, want_final=True)
+    assert oracle.rel_l2(hT.cpu().numpy(), hT_ref.cpu().numpy()) < 2e-6
+    assert oracle.rel_l2(y.float().cpu().numpy(), y_ref.float().cpu().numpy()) < (2e-6 if act == F32 else 7e-5)
