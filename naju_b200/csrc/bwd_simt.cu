@@ -362,7 +362,7 @@ bwd_simt_kernel(const BwdParams p) {
 
 // ------------------------------------------------------------------------------ finalize
 // dB[row][n] = sum_k part[row][k][n] for n < N (and dC), written in the caller's dtype; dD[d] = the sum over its
-// partial rows.  One launch: blocks [0, nbc) take dB, [nbc, 2 nbc) dC, the rest 32 channels of dD each, in a
+// partial rows.  One launch: blocks [0, ndd) take 32 channels of dD each (the longest chains first), then nbc take dB and nbc dC, in a
 // fixed order throughout.  If a bounded wait of this call or of its forward ran out (or `inject` asks for it),
 // every output is overwritten with all-ones bytes (NaN) instead.
 struct PoisonList {
@@ -371,39 +371,39 @@ struct PoisonList {
 };
 
 __global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* __restrict__ dB, void* __restrict__ dC,
-                                                       float* __restrict__ dD, int NS, int nbc, int dd_rows, int dd_rows_tc,
+                                                       float* __restrict__ dD, int NS, int nbc, int ndd, int dd_rows, int dd_rows_tc,
                                                        int inject, const PoisonList list) {
   __shared__ float red[8][33];
   pdl_wait();
+  const int blk = static_cast<int>(blockIdx.x) - ndd;
+  float sum = 0.f;
+  const int64_t i = static_cast<int64_t>(blk < nbc ? blk : blk - nbc) * 256 + threadIdx.x;
+  const bool mine = blk >= 0 && i < static_cast<int64_t>(p.B) * p.T * p.N;
+  if (mine) {   // (before the status is looked at: the loads need not wait for it)
+    const int64_t row = i < (1ll << 32) ? static_cast<uint32_t>(i) / static_cast<uint32_t>(p.N) : i / p.N;
+    const float* src = (blk < nbc ? p.dBpart : p.dCpart) + row * p.ndt * NS + (i - row * p.N);
+#pragma unroll 8
+    for (int k = 0; k < p.ndt; ++k) sum += __ldg(src + static_cast<int64_t>(k) * NS);
+  }
   if (inject && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
-  const int form = *p.fwd_form;
-  const bool bad = inject || *reinterpret_cast<volatile int*>(&p.hdr->status) != 0 || (form & 4) != 0;
-  const int blk = blockIdx.x;
+  const bool bad = inject || *reinterpret_cast<volatile int*>(&p.hdr->status) != 0 || (*p.fwd_form & 4) != 0;
   const float nan = __int_as_float(-1);
   if (bad) {
     for (int k = 0; k < 4; ++k)
-      for (unsigned long long i = static_cast<unsigned long long>(blk) * 256 + threadIdx.x; i < list.bytes[k];
-           i += static_cast<unsigned long long>(gridDim.x) * 256)
-        static_cast<unsigned char*>(list.ptr[k])[i] = 0xFF;
+      for (unsigned long long e = static_cast<unsigned long long>(blockIdx.x) * 256 + threadIdx.x; e < list.bytes[k];
+           e += static_cast<unsigned long long>(gridDim.x) * 256)
+        static_cast<unsigned char*>(list.ptr[k])[e] = 0xFF;
   }
-  if (blk < 2 * nbc) {
-    const float* part = blk < nbc ? p.dBpart : p.dCpart;
-    void* out = blk < nbc ? dB : dC;
-    const int64_t i = static_cast<int64_t>(blk < nbc ? blk : blk - nbc) * 256 + threadIdx.x;
-    if (i >= static_cast<int64_t>(p.B) * p.T * p.N) return;
-    const int64_t row = i / p.N;
-    const float* src = part + row * p.ndt * NS + (i - row * p.N);
-    float s = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < p.ndt; ++k) s += src[static_cast<int64_t>(k) * NS];
-    store_dyn(out, p.bc_dtype, i, bad ? nan : s);
+  if (blk >= 0) {
+    if (mine) store_dyn(blk < nbc ? dB : dC, p.bc_dtype, i, bad ? nan : sum);
     return;
   }
   // the tensor-core backward writes four partial rows per rank and batch row, the recurrent one per chunk
   const int rows = tc_did_it(p) ? dd_rows_tc : dd_rows;
-  const int dl = threadIdx.x & 31, rl = threadIdx.x >> 5, d = (blk - 2 * nbc) * 32 + dl, ld = p.ndt * kDT;
+  const int dl = threadIdx.x & 31, rl = threadIdx.x >> 5, d = static_cast<int>(blockIdx.x) * 32 + dl, ld = p.ndt * kDT;
   float s = 0.f;
   if (d < p.D)
+#pragma unroll 4
     for (int r = rl; r < rows; r += 8) s += p.dDpart[static_cast<int64_t>(r) * ld + d];
   red[rl][dl] = s;
   __syncthreads();
@@ -418,14 +418,15 @@ __global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* 
 int launch_bwd_finalize(const BwdParams& p, const Geometry& g, int act, int gate, void* dB, void* dC, float* dD, bool inject,
                         void* stream) {
   const int64_t ntd = static_cast<int64_t>(g.B) * g.T * g.D, nbc = (static_cast<int64_t>(g.B) * g.T * g.N + 255) / 256;
-  const int64_t blocks = 2 * nbc + (g.D + 31) / 32;
+  const int ndd = (g.D + 31) / 32;
+  const int64_t blocks = 2 * nbc + ndd;
   if (blocks > 0x7fffffff) return NAJU_E_SHAPE;
   PoisonList list = {{p.du, p.dfl, p.dil, p.dh0},
                      {static_cast<unsigned long long>(ntd) * dtype_size(act), static_cast<unsigned long long>(ntd) * dtype_size(gate),
                       static_cast<unsigned long long>(ntd) * dtype_size(gate),
                       p.dh0 ? static_cast<unsigned long long>(g.B) * g.D * g.N * 4 : 0ull}};
   return launch_pdl(finalize_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), p, dB,
-                    dC, dD, g.NS, static_cast<int>(nbc), g.nchunks * g.B, 4 * p.tc_launched * g.B, inject ? 1 : 0, list);
+                    dC, dD, g.NS, static_cast<int>(nbc), ndd, g.nchunks * g.B, 4 * p.tc_launched * g.B, inject ? 1 : 0, list);
 }
 
 template <typename TA, typename TG, int NS, int NH>
