@@ -16,6 +16,10 @@
  *    status word ends non-zero overwrites its own outputs with NaN before it
  *    completes (on the device, no host synchronisation), and a backward given the
  *    checkpoints of such a forward does the same.
+ *  - What is not finite: with 17 to 64 states, and in every recurrent kernel, an infinity or NaN in
+ *    an input reaches the steps after it (in the backward, before it) of the channel, state and
+ *    batch row it belongs to, and nothing else.  The tensor-core kernels of 16 states let one in u
+ *    (in dy) reach the other steps of its chunk of 64 steps, too.
  *  - Shapes follow naju/scan.py:3-12: u, f_logit, i_logit, y [B,T,D];
  *    Bm, Cm [B,T,N]; D_skip [D]; states [B,D,N] fp32.  The sigmoid of both gate
  *    logits is applied inside (naju/scan.py:81-82).
@@ -51,7 +55,7 @@ enum {
 /* device-side status bits, OR-ed into the workspace status word */
 enum {
   NAJU_ST_LOOKBACK_TIMEOUT = 1, /* a bounded wait on a neighbouring chunk's carry ran out */
-  NAJU_ST_BAD_TILE = 2,         /* internal tile index out of range (never expected) */
+  NAJU_ST_BAD_TILE = 2,         /* reserved; never set */
   NAJU_ST_MMA_TIMEOUT = 4,      /* a bounded wait on a tensor-core completion barrier ran out */
   NAJU_ST_DEEP_TILE = 8         /* the tensor-core backward met a deep-gate tile (never expected:
                                    the forward routes such problems to the recurrent backward) */

@@ -64,7 +64,7 @@ int read_header_word(const void* scratch, size_t offset, void* stream) {
   return word;
 }
 
-// (16-byte stores: the scratch is 256-byte aligned and `words` counts 256-byte rounded regions)
+// (16-byte stores: the scratch is 256-byte aligned, and its regions are rounded up to that)
 __global__ void init_kernel(uint4* __restrict__ scratch, int64_t n16, int* __restrict__ trailer) {
   pdl_launch_dependents();
   pdl_wait();

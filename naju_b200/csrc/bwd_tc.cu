@@ -154,7 +154,7 @@ struct Bars {
 //                    consecutive ranks, so that fewer channel tiles than SMs still fill the GPU.  The states come
 //                    from the checkpoints; only the adjoint goes from rank to rank, as soon as the chunk's dL is complete,
 //                    by asynchronous stores straight into the receiver's lt rows (which the receiver rescales in
-//                    place: no shared memory is left for a mailbox), once the receiver has said that the MMAs reading
+//                    place), once the receiver has said that the MMAs reading
 //                    its previous rows are done.
 template <typename TA, typename TG, bool UTM, bool CLUSTER>
 __global__ void __launch_bounds__(NTHREADS, 1)

@@ -63,33 +63,6 @@ constexpr uint32_t BC_BYTES = Q * NS * 2;                      // one raw B (or 
 // TMEM columns of a stage: D1 [0,64), D2 [64,80), P_t [96,160)
 constexpr uint32_t TM_D1 = 0, TM_D2 = 64, TM_P = 96, TM_STAGE = 160, TMEM_COLS = 512;
 
-// Two-term bf16 split of a pair of floats: v ~= hi + lo with 16 mantissa bits kept.  Both terms
-// are truncations (the first one's error is exactly what the second term carries), so the split
-// costs only integer and FMA-pipe operations: the conversion instructions share the SFU pipe with
-// ex2/rcp, which is the busiest pipe of the gate warps.  Residual <= 2^-16 relative.
-__device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
-  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-  const uint32_t ha = ua & 0xFFFF0000u, hb = ub & 0xFFFF0000u;
-  hi = __byte_perm(ha, hb, 0x7632);  // {hb[31:16], ha[31:16]}
-  const uint32_t la = __float_as_uint(a - __uint_as_float(ha)), lb = __float_as_uint(b - __uint_as_float(hb));
-  lo = __byte_perm(la, lb, 0x7632);
-}
-
-// shared-memory element -> fp32 without the conversion unit where the format allows it
-__device__ __forceinline__ float ld_as_f32(const __nv_bfloat16* p, int i) {
-  return __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const unsigned short*>(p)[i]) << 16);
-}
-__device__ __forceinline__ float ld_as_f32(const __half* p, int i) { return __half2float(p[i]); }
-__device__ __forceinline__ float ld_as_f32(const float* p, int i) { return p[i]; }
-// two adjacent 16-bit elements (4-byte aligned) as floats, one 32-bit load
-__device__ __forceinline__ float2 ld_pair_as_f32(const __nv_bfloat16* p) {
-  const uint32_t pk = *reinterpret_cast<const uint32_t*>(p);
-  return make_float2(bf16lo_f32(pk), bf16hi_f32(pk));
-}
-__device__ __forceinline__ float2 ld_pair_as_f32(const __half* p) {
-  return __half22float2(*reinterpret_cast<const __half2*>(p));
-}
-
 // D(16x8, fp32) += A(16x16, bf16, row) . B(16x8, bf16, col)
 __device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                  uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -326,10 +299,10 @@ fwd_tc2_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int n
           mma_bf16_16x8x16(c, a0, a1, a2, a3, b0, b1);
           const int s0 = 8 * nt + 2 * t4;
           uint32_t hi, lo;
-          split_bf16x2(s0 <= r0 ? c[0] : 0.f, s0 + 1 <= r0 ? c[1] : 0.f, hi, lo);
+          split_pair(make_float2(s0 <= r0 ? c[0] : 0.f, s0 + 1 <= r0 ? c[1] : 0.f), hi, lo);
           *reinterpret_cast<uint32_t*>(s_B1 + op_off16(r0, B1_G1 * 8 + s0, SBO_B1)) = hi;
           *reinterpret_cast<uint32_t*>(s_B1 + op_off16(r0, B1_G2 * 8 + s0, SBO_B1)) = lo;
-          split_bf16x2(s0 <= r1 ? c[2] : 0.f, s0 + 1 <= r1 ? c[3] : 0.f, hi, lo);
+          split_pair(make_float2(s0 <= r1 ? c[2] : 0.f, s0 + 1 <= r1 ? c[3] : 0.f), hi, lo);
           *reinterpret_cast<uint32_t*>(s_B1 + op_off16(r1, B1_G1 * 8 + s0, SBO_B1)) = hi;
           *reinterpret_cast<uint32_t*>(s_B1 + op_off16(r1, B1_G2 * 8 + s0, SBO_B1)) = lo;
         }
@@ -447,10 +420,10 @@ fwd_tc2_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int n
             pv[j] = __float_as_uint(P);
           }
           uint32_t h0, h1, h2, h3, l0, l1, l2, l3;
-          split_bf16x2(wv[0], wv[1], h0, l0);
-          split_bf16x2(wv[2], wv[3], h1, l1);
-          split_bf16x2(wv[4], wv[5], h2, l2);
-          split_bf16x2(wv[6], wv[7], h3, l3);
+          split_pair(make_float2(wv[0], wv[1]), h0, l0);
+          split_pair(make_float2(wv[2], wv[3]), h1, l1);
+          split_pair(make_float2(wv[4], wv[5]), h2, l2);
+          split_pair(make_float2(wv[6], wv[7]), h3, l3);
           const int ch = k * (SLAB / 8) + j8;
           *reinterpret_cast<uint4*>(a_row + (AW_W1 + ch) * 128) = make_uint4(h0, h1, h2, h3);
           *reinterpret_cast<uint4*>(a_row + (AW_W2 + ch) * 128) = make_uint4(l0, l1, l2, l3);
@@ -481,7 +454,7 @@ fwd_tc2_kernel(const FwdParams p, const __grid_constant__ Maps maps, const int n
     auto write_h_row = [&](const float (&hv)[NS]) {
       uint32_t hi[8], lo[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) split_bf16x2(hv[2 * k], hv[2 * k + 1], hi[k], lo[k]);
+      for (int k = 0; k < 8; ++k) split_pair(make_float2(hv[2 * k], hv[2 * k + 1]), hi[k], lo[k]);
       *reinterpret_cast<uint4*>(h_row + (AH_H1 + 0) * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
       *reinterpret_cast<uint4*>(h_row + (AH_H1 + 1) * 128) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
       *reinterpret_cast<uint4*>(h_row + (AH_H2 + 0) * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);

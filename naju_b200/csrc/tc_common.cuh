@@ -169,21 +169,6 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
   return ok != 0;
 }
 
-// One try that parks for at most about `ns` nanoseconds.
-__device__ __forceinline__ bool mbar_try_for(uint32_t mbar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(mbar), "r"(parity), "r"(ns)
-      : "memory");
-  return ok != 0;
-}
-
 // (kept out of line: the retry loop is cold code, and the kernels' hot loops must stay small
 // enough for the instruction caches)
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity) {

@@ -31,10 +31,10 @@ def resolve_backend(backend=None):
 
 # Switches read by every call (naju_b200/csrc/torch_host.cpp):
 #   NAJU_B200_FORM selects the kernel family: "auto" (default) takes the tcgen05 tensor-core chunked form
-#   where it applies (16-bit activations, bf16 B/C, N == 16 -- or fewer, padded with zero columns by the
-#   host when the problem is large enough --, TMA-legal strides) and the exact recurrent kernels elsewhere;
-#   "recurrent" forces the recurrent ones; "chunked" insists on the tensor-core form and raises where it
-#   does not apply.
+#   where it applies (16-bit activations, bf16 B/C, TMA-legal strides, N == 16 -- or fewer, padded with zero
+#   columns by the host when the problem is large enough --; bf16 activations and 17 to 64 states where there are
+#   channel tiles enough) and the exact recurrent kernels elsewhere; "recurrent" forces the recurrent ones;
+#   "chunked" insists on the 16-state tensor-core form and raises where it does not apply.
 #   NAJU_B200_CHECK_STATUS=1 reads the device-side status word after every call (synchronises the stream).
 #   NAJU_B200_INJECT_TIMEOUT=1 is the fault injection for tests, NAJU_B200_GUARD=1 the canary bands below.
 
@@ -92,10 +92,9 @@ def _state_arg(h, B, D, N, name):
 
 # (N < 16 on a large 16-bit problem is padded with zero columns to the 16 states of the tcgen05 kernels.
 # The same argument splits N > 16 into groups of 16 states whose y / du / d f_logit / d i_logit are added
-# up; that was built and measured -- 2.2x (N=64) and 3.1x (N=32) faster than the recurrent kernels at B=8,
-# T=8192, D=4096 -- but every group's output is rounded to the 16-bit activation type before the sum,
-# which put y and the gradients at 2.7e-3 of the reference, outside the 1e-3 / 2e-3 bounds, so N > 16
-# stays with the exact recurrent kernels.)
+# up; that was built and measured, but every group's output is rounded to the 16-bit activation type before
+# the sum, which put y and the gradients at 2.7e-3 of the reference, outside the 1e-3 / 2e-3 bounds: 17 to 64
+# states have kernels of their own.)
 _GROUP = 16
 
 
