@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(const BwdParams p, void* 
     const int64_t row = i < (1ll << 32) ? static_cast<uint32_t>(i) / static_cast<uint32_t>(p.N) : i / p.N;
     const float* src = (blk < nbc ? p.dBpart : p.dCpart) + row * p.ndt * NS + (i - row * p.N);
 #pragma unroll 8
-    for (int k = 0; k < p.ndt; ++k) sum += __ldg(src + static_cast<int64_t>(k) * NS);
+    for (int k = 0; k < p.ndt; ++k) sum += __ldcg(src + static_cast<int64_t>(k) * NS);   // (not the read-only path: the writer may overlap this kernel's start)
   }
   if (inject && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&p.hdr->status, NAJU_ST_LOOKBACK_TIMEOUT);
   const bool bad = inject || *reinterpret_cast<volatile int*>(&p.hdr->status) != 0 || (*p.fwd_form & 4) != 0;
