@@ -357,10 +357,11 @@ std::tuple<Tensor, Tensor> scan(const Tensor& u, const Tensor& fl, const Tensor&
 // A row operand of the step as the kernel takes it: inner stride 1, rows at least a row apart.  Rows that overlap or repeat (an operand
 // broadcast over the batch) are copied; with one row only the stride means nothing.
 Tensor step_rows(const Tensor& t) {
-  const Tensor r = inner_contig(t);
-  return r.size(0) > 1 && r.stride(0) < r.size(1) ? r.contiguous() : r;
+  const auto size = t.sizes(), stride = t.strides();
+  const bool ok = stride[1] == 1 && (size[0] == 1 || stride[0] >= size[1]) &&
+                  reinterpret_cast<uintptr_t>(t.data_ptr()) % t.element_size() == 0;
+  return ok ? t : t.contiguous();
 }
-int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
 
 // state [B,D,N] fp32 is updated in place; u, f_logit, i_logit [B,D]; B, C [B,N].
 Tensor step(const Tensor& state, const Tensor& u, const Tensor& fl, const Tensor& il, const Tensor& Bm, const Tensor& Cm,
@@ -388,8 +389,12 @@ Tensor step(const Tensor& state, const Tensor& u, const Tensor& fl, const Tensor
   d.act_dtype = dtype_code(pu.scalar_type());
   d.gate_dtype = dtype_code(gdt);
   d.bc_dtype = dtype_code(bdt);
-  d.u_sb = row_stride(pu); d.fl_sb = row_stride(pf); d.il_sb = row_stride(pi);
-  d.bm_sb = row_stride(pB); d.cm_sb = row_stride(pC);
+  d.u_sb = d.fl_sb = d.il_sb = Dc;   // (one row: its stride means nothing)
+  d.bm_sb = d.cm_sb = N;
+  if (B > 1) {
+    d.u_sb = pu.stride(0); d.fl_sb = pf.stride(0); d.il_sb = pi.stride(0);
+    d.bm_sb = pB.stride(0); d.cm_sb = pC.stride(0);
+  }
   Tensor y = at::empty({B, Dc}, pu.options());
   check(naju_b200_step(&d, static_cast<float*>(state.data_ptr()), ptr(pu), ptr(pf), ptr(pi), ptr(pB), ptr(pC), fptr(pD),
                        mptr(y), stream_of(state)),
