@@ -8,7 +8,7 @@
 //   r_t = r_{t+1} + al_t Yt_t - wt_t gt_t,   d f_logit = (1-f_t) r_t,   du = i_t R_t gt_t + D_skip dy_t,   d i_logit = wt_t (1-i_t) gt_t
 //
 // What bounds it: the recurrent kernel does 14 N operations per channel and step on the CUDA cores (64 states: 13.9 ms for
-// 8 x 8192 x 4096, 32 states 11.6 ms; 4.7 and 2.9 ms here).  Here they are MMAs, and a tile is a chain of phases: gates, MMAs, sweep.
+// 8 x 8192 x 4096, 32 states 11.6 ms; 4.75 and 3.36 ms here).  Here they are MMAs, and a tile is a chain of phases: gates, MMAs, sweep.
 // Every operand is in three bf16 terms, all 24 bits of an fp32 significand, as the recurrent kernel computes in fp32 throughout; of
 // the nine products of two such operands the six that reach 24 bits are taken, the smallest first (an accumulating MMA truncates).
 // A channel's row is [al 32 | wt 32 | h NS | lt NS] three times: with 64 states 147 KB for 128 channels, so a chunk is 32 steps and
@@ -399,7 +399,7 @@ bwd_wide_kernel(const BwdParams p, const __grid_constant__ Maps maps) {
     auto post_h = [&](int xx, int c) {
       const int bb = xx / p.ndt, dd = (xx - bb * p.ndt) * kDT + cid;
       const float* src = c >= 0 ? state_row(xx, c) : nullptr;
-      // (64 states: sixteen in flight at a time, 2343 -> 2237 us at B=8, T=4096, D=4096, with the prefetch below; 32 states:
+      // (64 states: sixteen in flight at a time, 2343 -> 2237 us at B=8, T=4096, D=4096, with the prefetch below and two-term operands; 32 states:
       // eight, 1477 us against 1514)
       constexpr int PER = NS == 64 ? 2 : 1;
 #pragma unroll

@@ -11,7 +11,8 @@
 //
 // What bounds it: the recurrent kernel does N multiply-adds and N loads' worth of B and C per channel and step on the
 // CUDA cores (64 states: 6.7 ms for 8 x 8192 x 4096, 32 states 3.9 ms); here that work is MMAs, and what is left per
-// step is the gates and a tile's hand-offs: 1.95 and 1.35 ms, 3.8 and 2.6 us a tile.
+// step is the gates and a tile's hand-offs: 2.25 and 1.52 ms, 4.4 and 3.0 us a tile (with two-term
+// operands and nothing watched for 1.93 and 1.35 ms).
 // Chunks are 32 steps, half the 16-state kernel's, because the carried rows are four times as wide; two sets of
 // main warps take the even and the odd tiles, so that one set's gates run while the other waits for its MMAs.
 //   warps 0-15   main warps: set s = warp / 8 takes the tiles of its parity, its half g steps [16g, 16g+16), a thread one

@@ -110,8 +110,9 @@ inline BwdScratchLayout bwd_scratch_layout(const Geometry& g) {
 }
 
 // Whether the walk kernels of 17 to 64 states (fwd_wide.cu, bwd_wide.cu) pay: a CTA takes a tile in about 50 times what the
-// recurrent kernels, spread over the whole GPU and over time, need per tile (64 states: 3.8 us against 0.10 us forward, 9.1
-// against 0.21 us backward; 32 states: 2.6 / 0.06 and 5.7 / 0.18 us).
+// recurrent kernels, spread over the whole GPU and over time, need per tile (64 states: 4.4 us against 0.10 us forward, 9.2
+// against 0.21 us backward; 32 states: 3.0 / 0.06 and 6.6 / 0.18 us; with 50 channel tiles, B=1, T=2048, D=6400, 64 states: 273 against
+// 376 us forward, 596 against 726 us backward).
 inline bool wide_walk_pays(const Geometry& g, int64_t sms) {
   const int64_t ctiles = static_cast<int64_t>(g.B) * g.ndt;
   return (ctiles + sms - 1) / sms * 50 <= ctiles;
